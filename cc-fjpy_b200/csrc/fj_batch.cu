@@ -24,6 +24,7 @@
 
 #include "batch_plan.h"
 #include "fj_cells.cuh"
+#include "fj_expand.cuh"
 
 namespace ccfj {
 
@@ -67,23 +68,32 @@ __global__ void batch_prep_u_kernel(InDesc in, const long long* __restrict__ off
                                     const float* __restrict__ drs, const float* __restrict__ wtr,
                                     const float4* __restrict__ geo,
                                     const float* __restrict__ thr, int itype,
-                                    void* __restrict__ dst) {
-  // rows on grid x (up to 2^31 - 1 blocks), frequencies on grid y
+                                    void* __restrict__ dst, const unsigned char* __restrict__ use) {
+  // rows on grid x (a CTA takes a run of rows), frequencies on grid y
   const int fi = blockIdx.y * blockDim.x + threadIdx.x;
-  const long long i = (long long)blockIdx.x * blockDim.y + threadIdx.y;
-  if (fi >= nf || i >= total) return;
+  if (fi >= nf) return;
   const long long col = (long long)fi * in.cs;
-  const float g = in.p[(in.perm ? in.perm[i] : i) * in.ld + col];
-  if (itype == 1) {
-    const int b = set_of(off, nsets, i);
-    const bool hl = i > off[b], hr = i + 1 < off[b + 1];
-    const float gl = hl ? in.p[(in.perm ? in.perm[i - 1] : i - 1) * in.ld + col] : 0.0f;
-    const float gr = hr ? in.p[(in.perm ? in.perm[i + 1] : i + 1) * in.ld + col] : 0.0f;
-    static_cast<StationCoef<float>*>(dst)[i * nf + fi] =
-        station_coef<float>(g, gl, gr, hl, hr, rs[i], hl ? rs[i - 1] : 0.0f, drs[i],
-                            hr ? drs[i + 1] : 0.0f, geo[i].w, thr[fi]);
-  } else {
-    static_cast<float*>(dst)[i * nf + fi] = g * wtr[i] / geo[i].w;
+  const long long per = (total + gridDim.x - 1) / gridDim.x;
+  const long long end = min(total, (blockIdx.x + 1) * per);
+  int b = -1;
+  long long b_end = 0;
+  for (long long i = blockIdx.x * per + threadIdx.y; i < end; i += blockDim.y) {
+    if (i >= b_end) {
+      b = set_of(off, nsets, i);
+      b_end = off[b + 1];
+    }
+    if (use && use[(long long)b * nf + fi]) continue;
+    const float g = in.p[(in.perm ? in.perm[i] : i) * in.ld + col];
+    if (itype == 1) {
+      const bool hl = i > off[b], hr = i + 1 < off[b + 1];
+      const float gl = hl ? in.p[(in.perm ? in.perm[i - 1] : i - 1) * in.ld + col] : 0.0f;
+      const float gr = hr ? in.p[(in.perm ? in.perm[i + 1] : i + 1) * in.ld + col] : 0.0f;
+      static_cast<StationCoef<float>*>(dst)[i * nf + fi] =
+          station_coef<float>(g, gl, gr, hl, hr, rs[i], hl ? rs[i - 1] : 0.0f, drs[i],
+                              hr ? drs[i + 1] : 0.0f, geo[i].w, thr[fi]);
+    } else {
+      static_cast<float*>(dst)[i * nf + fi] = g * wtr[i] / geo[i].w;
+    }
   }
 }
 
@@ -162,6 +172,7 @@ __global__ void __launch_bounds__(256, fj_min_blocks<float>()) fj_batch_persiste
     a.gb[0] = static_cast<const char*>(bd.base.gb[0]) + o * a.nf * esz;
     if (ModeTraits<MODE>::NIN > 1) a.gb[1] = static_cast<const char*>(bd.base.gb[1]) + o * a.nf * esz;
     a.out += (long long)b * a.nc * a.nf;
+    if (a.use) a.use += (long long)b * a.nf;
     // velocity tiles fastest: the items of one frequency tile run side by
     // side and share its station coefficients in L2
     const int fi = (rem / bd.ctiles) * 32 + threadIdx.x;
@@ -172,11 +183,17 @@ __global__ void __launch_bounds__(256, fj_min_blocks<float>()) fj_batch_persiste
 
 // Per (set, frequency) column normalisation (builtin-max semantics, as
 // fj_normalize_kernel), set = blockIdx.y.
-__global__ void batch_normalize_kernel(float* __restrict__ out, int nc, int nf) {
+// Columns marked in `use` [nsets][nf] are finished elsewhere.
+__global__ void batch_normalize_kernel(float* __restrict__ out, int nc, int nf,
+                                       const unsigned char* __restrict__ use) {
   __shared__ float red[8][33];
   __shared__ float colmax[32];
   float* o = out + (long long)blockIdx.y * nc * nf;
-  const int fi = blockIdx.x * 32 + threadIdx.x;
+  int fi = blockIdx.x * 32 + threadIdx.x;
+  if (use) {
+    if (fi < nf && use[(long long)blockIdx.y * nf + fi]) fi = nf;
+    if (!__syncthreads_or(fi < nf)) return;
+  }
   // two running maxima and eight loads in flight per thread (the maximum
   // does not depend on the order)
   float m = -INFINITY, m2 = -INFINITY;
@@ -298,7 +315,10 @@ int batch_variant(const ccfj_batch_args& a, long long total) {
 
 // The device sequence of one batch (all pointers device pointers;
 // `total` = offsets[nsets], known to the caller).
-int batch_device(const ccfj_batch_args& a, long long total, cudaStream_t s) {
+// `expand`: the wave-cell expansion may take columns; total_all: the pairs of
+// the whole batch that these sets are a group of.
+int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStream_t s,
+                 long long total_all = 0) {
   Scratch sc(s);
   const int nin = nin_of_mode(a.mode);
   float* drs = sc.get_n<float>(total + 1);
@@ -330,13 +350,41 @@ int batch_device(const ccfj_batch_args& a, long long total, cudaStream_t s) {
     if (st != CCFJ_OK) return st;
     in[1] = InDesc{hb, a.nf, 1, nullptr};
   }
+  XpProblem xp{};
+  XpWork xw{};
+  bool expanded = false;
+  const unsigned char* use = nullptr;
+  if (expand) {
+    xp.rs = a.r;
+    xp.wtr = wtr;
+    xp.off = a.offsets;
+    xp.nsets = a.nsets;
+    xp.total = total;
+    xp.nf = a.nf;
+    xp.nc = a.nc;
+    xp.f = a.f;
+    xp.c = a.c;
+    xp.itype = a.itype;
+    xp.mode = a.mode;
+    xp.in[0] = in[0];
+    xp.in[1] = in[1];
+    xp.out = a.out;
+    xp.normalize = a.normalize;
+    xp.nf_all = a.nf;
+    xp.total_all = total_all > 0 ? total_all : total;
+    const int st = xp_plan(xp, sc, s, &xw, &expanded);
+    if (st != CCFJ_OK) return st;
+    if (expanded) use = xw.use;
+  }
   BatchDev bd{};
+  bd.base.use = use;
   const float tau = a.tau > 0 ? a.tau : kDefaultTau32;
   float* kb = nullptr;
   if (a.itype == 1) {
     kb = sc.get_n<float>(a.nf);
     if (!kb) return CCFJ_ERR_ALLOC;
-    fj_kbounds_kernel<float><<<div_up(a.nf, 8), dim3(32, 8), 0, s>>>(a.f, a.c, a.nf, a.nc, tau, kb);
+    fj_kbounds_kernel<float><<<div_up(a.nf, 8), dim3(32, 8), 0, s>>>(a.f, a.c, a.nf, a.nc, tau, kb,
+                                                                nullptr);
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_kbounds_kernel");
   }
@@ -344,8 +392,9 @@ int batch_device(const ccfj_batch_args& a, long long total, cudaStream_t s) {
   for (int j = 0; j < nin; ++j) {
     void* g = sc.get((size_t)total * a.nf * esz);
     if (!g) return CCFJ_ERR_ALLOC;
-    batch_prep_u_kernel<<<dim3(div_up(total, 8), div_up(a.nf, 32)), dim3(32, 8), 0, s>>>(
-        in[j], a.offsets, a.nsets, total, a.nf, a.r, drs, wtr, geo, kb, a.itype, g);
+    const unsigned rows = (unsigned)std::min<long long>(1024, div_up(total, 8));
+    batch_prep_u_kernel<<<dim3(rows, div_up(a.nf, 32)), dim3(32, 8), 0, s>>>(
+        in[j], a.offsets, a.nsets, total, a.nf, a.r, drs, wtr, geo, kb, a.itype, g, use);
     count_launch();
     CCFJ_LAUNCH_CHECK("batch_prep_u_kernel");
     bd.base.gb[j] = g;
@@ -381,11 +430,18 @@ int batch_device(const ccfj_batch_args& a, long long total, cudaStream_t s) {
   CCFJ_LAUNCH_CHECK("fj_batch_persistent_kernel");
   if (a.normalize) {
     batch_normalize_kernel<<<dim3(div_up(a.nf, 32), a.nsets), dim3(32, 8), 0, s>>>(a.out, a.nc,
-                                                                                   a.nf);
+                                                                                   a.nf, use);
     count_launch();
     CCFJ_LAUNCH_CHECK("batch_normalize_kernel");
   }
-  return CCFJ_OK;
+  return expanded ? xp_run(xp, xw, s) : CCFJ_OK;
+}
+
+// Whether the expansion may take columns of a batch: not where the caller
+// asks for a variant of the direct kernel or a switch point of its rule.
+bool batch_expands(const ccfj_batch_args& a, long long total) {
+  return a.variant == 0 && !(a.tau > 0) &&
+         xp_eligible(a.mode, a.itype, total, a.nsets, a.nf, a.nc);
 }
 
 // ---------------------------------------------------------- graph cache
@@ -461,7 +517,7 @@ void evict_oldest_graph() {
 int batch_device_graph(const ccfj_batch_args& a, long long total, cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (s) CCFJ_CUDA_TRY(cudaStreamIsCapturing(s, &cs));
-  if (cs != cudaStreamCaptureStatusNone) return batch_device(a, total, s);  // caller's capture
+  if (cs != cudaStreamCaptureStatusNone) return batch_device(a, total, batch_expands(a, total), s);  // caller's
   const std::string key = graph_key(a, total);
   std::lock_guard<std::mutex> lk(g_graph_mu);
   auto it = g_graphs.find(key);
@@ -477,7 +533,7 @@ int batch_device_graph(const ccfj_batch_args& a, long long total, cudaStream_t s
     }
     cudaGraph_t graph = nullptr;
     CCFJ_CUDA_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-    const int st = batch_device(a, total, cap);
+    const int st = batch_device(a, total, batch_expands(a, total), cap);
     const cudaError_t e = cudaStreamEndCapture(cap, &graph);
     if (st != CCFJ_OK) {
       if (graph) cudaGraphDestroy(graph);
@@ -523,7 +579,7 @@ int batch_device_graph(const ccfj_batch_args& a, long long total, cudaStream_t s
 
 int batch_run_device(const ccfj_batch_args& a, long long total, cudaStream_t s) {
   if (a.use_graph && !allocator_hooked()) return batch_device_graph(a, total, s);
-  return batch_device(a, total, s);
+  return batch_device(a, total, batch_expands(a, total), s);
 }
 
 // ------------------------------------------------- host-memory batches
@@ -606,7 +662,7 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
   d.perm = dp;
   const size_t out_bytes = sizeof(float) * a.nsets * a.nc * a.nf;
   if (ng == 0) {
-    const int st = batch_device(d, total, s);
+    const int st = batch_device(d, total, batch_expands(a, total), s);
     if (st != CCFJ_OK) return st;
     return copy_to_host(a.out, dout, out_bytes, 0, s);
   }
@@ -637,6 +693,7 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
   int st = copy_group(0);
   if (st != CCFJ_OK) return st;
   const int variant = batch_variant(a, total);  // the whole batch's choice for every group
+  const bool expand = batch_expands(a, total);
   long long slot = 0;
   for (int g = 0; g < ng; ++g) {
     const SetGroup& G = groups[g];
@@ -651,7 +708,7 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
     dg.out = dout + (size_t)G.b0 * a.nc * a.nf;
     dg.variant = variant;
     CCFJ_CUDA_TRY(cudaStreamWaitEvent(s, lane.ev[g], 0));
-    st = batch_device(dg, dg.total_pairs, s);
+    st = batch_device(dg, dg.total_pairs, expand, s, total);
     if (st != CCFJ_OK) return st;
     if (g + 1 < ng && (st = copy_group(g + 1)) != CCFJ_OK) return st;
   }
@@ -662,7 +719,7 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
 
 int normalize_sets(float* out, int nsets, int nc, int nf, cudaStream_t s) {
   CCFJ_REQUIRE(nsets <= 65535, "normalisation of %d sets (> 65535)", nsets);
-  batch_normalize_kernel<<<dim3(div_up(nf, 32), nsets), dim3(32, 8), 0, s>>>(out, nc, nf);
+  batch_normalize_kernel<<<dim3(div_up(nf, 32), nsets), dim3(32, 8), 0, s>>>(out, nc, nf, nullptr);
   count_launch();
   CCFJ_LAUNCH_CHECK("batch_normalize_kernel");
   return CCFJ_OK;
@@ -705,7 +762,7 @@ CCFJ_API int ccfj_autotune_batch_v1(const ccfj_batch_args* args, void* stream, i
     float t = 1e30f;
     for (int rep = 0; rep < 3 && st == CCFJ_OK; ++rep) {
       cudaEventRecord(e0, s);
-      st = ccfj::batch_device(d, args->total_pairs, s);
+      st = ccfj::batch_device(d, args->total_pairs, false, s);
       cudaEventRecord(e1, s);
       const cudaError_t e = cudaEventSynchronize(e1);
       if (st == CCFJ_OK && e != cudaSuccess)

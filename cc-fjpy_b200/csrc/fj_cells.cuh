@@ -232,6 +232,9 @@ struct FjDev {
   int i_lo, i_hi;
   float* part;
   int split_len;  // stations per range when a launch splits the set (grid z)
+  // Columns with a nonzero byte are computed elsewhere (fj_expand.cu): they
+  // are not stored, and a tile of 32 of them is skipped. NULL: none.
+  const unsigned char* use;
 };
 
 // ------------------------------------------------- folded interval sum
@@ -337,9 +340,10 @@ __device__ __forceinline__ StationCoef<T> station_coef(T g, T gl, T gr, bool has
 // Fold threshold per frequency (one warp per frequency).
 template <typename T>
 __global__ void fj_kbounds_kernel(const float* __restrict__ f, const float* __restrict__ c,
-                                  int nf, int nc, T tau, T* __restrict__ thr) {
+                                  int nf, int nc, T tau, T* __restrict__ thr,
+                                  const unsigned char* __restrict__ use) {
   const int fi = blockIdx.x * blockDim.y + threadIdx.y;
-  if (fi >= nf) return;
+  if (fi >= nf || (use && use[fi])) return;
   const float fl = f[fi];
   T lo = T(INFINITY), hi = T(0);
   for (int j = threadIdx.x; j < nc; j += 32) {
@@ -367,14 +371,25 @@ __device__ __forceinline__ float4 station_geometry(float r, float d_next) {
 // amplitude (sqrt(r) := 1 at r = 0).
 template <typename T>
 __global__ void fj_prep_u_kernel(InDesc in, int nr, int nf, const float* __restrict__ wtr,
-                                 const float4* __restrict__ geo, T* __restrict__ dst) {
-  // pairs on grid x (no 65535 limit), frequencies on grid y
+                                 const float4* __restrict__ geo, T* __restrict__ dst,
+                                 const unsigned char* __restrict__ use) {
+  // pairs on grid x (as many rows of CTAs as prep_rows gives), frequencies on y
   const int fi = blockIdx.y * blockDim.x + threadIdx.x;
-  const int i = blockIdx.x * blockDim.y + threadIdx.y;
-  if (fi >= nf || i >= nr) return;
-  const long long row = in.perm ? in.perm[i] : i;
-  const T g = (T)in.p[row * in.ld + (long long)fi * in.cs];
-  dst[(long long)i * nf + fi] = g * (T)wtr[i] / (T)geo[i].w;
+  if (fi >= nf || (use && use[fi])) return;
+  for (int i = blockIdx.x * blockDim.y + threadIdx.y; i < nr; i += gridDim.x * blockDim.y) {
+    const long long row = in.perm ? in.perm[i] : i;
+    const T g = (T)in.p[row * in.ld + (long long)fi * in.cs];
+    dst[(long long)i * nf + fi] = g * (T)wtr[i] / (T)geo[i].w;
+  }
+}
+
+// CTAs along the pairs of the preparation kernels, which step through the
+// pairs: with one CTA per 8 pairs, the launch of a preparation whose columns
+// are all computed elsewhere took longer than the transform itself.
+constexpr long long kPrepRows = 128;
+inline unsigned prep_rows(long long nr) {
+  const long long n = (nr + 7) / 8;
+  return (unsigned)(n < kPrepRows ? n : kPrepRows);
 }
 
 // itype 1: gathers rows perm[i-1], perm[i], perm[i+1] (or i-1, i, i+1) of
@@ -383,18 +398,20 @@ template <typename T>
 __global__ void fj_prep_coef_kernel(InDesc in, int nr, int nf, const float* __restrict__ rs,
                                     const float* __restrict__ drs,
                                     const float4* __restrict__ geo, const T* __restrict__ thr,
-                                    StationCoef<T>* __restrict__ dst) {
+                                    StationCoef<T>* __restrict__ dst,
+                                    const unsigned char* __restrict__ use) {
   const int fi = blockIdx.y * blockDim.x + threadIdx.x;
-  const int i = blockIdx.x * blockDim.y + threadIdx.y;
-  if (fi >= nf || i >= nr) return;
+  if (fi >= nf || (use && use[fi])) return;
   const long long* perm = in.perm;
   const long long col = (long long)fi * in.cs;
-  const bool hl = i > 0, hr = i + 1 < nr;
-  const T g = (T)in.p[(perm ? perm[i] : i) * in.ld + col];
-  const T gl = hl ? (T)in.p[(perm ? perm[i - 1] : i - 1) * in.ld + col] : T(0);
-  const T gr = hr ? (T)in.p[(perm ? perm[i + 1] : i + 1) * in.ld + col] : T(0);
-  dst[(long long)i * nf + fi] = station_coef<T>(g, gl, gr, hl, hr, rs[i], hl ? rs[i - 1] : 0.0f,
-                                                drs[i], drs[i + 1], geo[i].w, thr[fi]);
+  for (int i = blockIdx.x * blockDim.y + threadIdx.y; i < nr; i += gridDim.x * blockDim.y) {
+    const bool hl = i > 0, hr = i + 1 < nr;
+    const T g = (T)in.p[(perm ? perm[i] : i) * in.ld + col];
+    const T gl = hl ? (T)in.p[(perm ? perm[i - 1] : i - 1) * in.ld + col] : T(0);
+    const T gr = hr ? (T)in.p[(perm ? perm[i + 1] : i + 1) * in.ld + col] : T(0);
+    dst[(long long)i * nf + fi] = station_coef<T>(g, gl, gr, hl, hr, rs[i], hl ? rs[i - 1] : 0.0f,
+                                                  drs[i], drs[i + 1], geo[i].w, thr[fi]);
+  }
 }
 
 // ------------------------------------------------- station-amortised kernel
@@ -638,9 +655,15 @@ __device__ __forceinline__ void fj_cells(const FjDev& a, int fi, int c0) {
   const bool c_valid = c0 < a.nc;
   if (!kStaged && !c_valid) return;
   c0 = c_valid ? c0 : 0;
-  const bool f_valid = fi < a.nf;
+  bool f_valid = fi < a.nf;
   const int fbase = fi - (int)(threadIdx.x & 31);  // first frequency of the warp (and CTA)
   fi = f_valid ? fi : a.nf - 1;
+  if (a.use) {
+    // the CTA's warps have the same frequencies, so all of them leave
+    const bool elsewhere = a.use[fi] != 0;
+    if (__all_sync(0xffffffffu, elsewhere)) return;
+    f_valid = f_valid && !elsewhere;
+  }
   Cell<T> cell[CPT];
   const float fl = a.f[fi];
 #pragma unroll

@@ -1,0 +1,1279 @@
+// Wave-cell expansion of the F-J transform.
+//
+// Both forms of the transform (src/FJcpu.cpp:230-419) are linear functionals
+// of the function r -> Z0(k r), k = 2 pi f / c:
+//
+//   itype 1   out(c, f) = sum over intervals of int (g_A + b (r - r_A)) r Z0(k r) dr
+//   itype 0   out(c, f) = sum over stations of g w Z0(k r)
+//
+// and k r = 2 pi u / c depends on u = r f alone. So the axis of u is cut into
+// cells on which Z0 is a polynomial to FP32 rounding at every velocity of the
+// call: cells of 9.8 radians at the slowest velocity and 16 Chebyshev terms
+// (the series of a wave over +-5.2 radians has the coefficients 2 J_n(5.2):
+// 1e-7 at n = 16, at the slowest velocity alone). With Z0(2 pi u / c) = sum_n E[c][cell, n] T_n,
+// the transform is a matrix product
+//
+//   out[c, f] = sum_{cell, n} E[c][cell, n] W[cell, n][f]
+//
+// of a matrix E that is the same for every frequency, every set of a batch
+// and every input, and the moments W of the spectra over the cells, which
+// know nothing of the velocities:
+//
+//   W[cell, n][f] = int over the cell of g(r) r T_n dr.
+//
+// A short interval belongs to the cell of its far end, so the polynomials
+// reach 1/16 of a cell below their cell (10.4 radians in all).
+//
+// The direct kernels evaluate the special functions once per (pair, f, c);
+// here they are evaluated once per (cell node, c), the pairs are visited once
+// per f, and the rest is multiply-adds. The number of cells of a frequency,
+// f (r_max - r_min) / h, does not depend on the number of pairs.
+//
+// An interval that spans whole cells would add up as much over them as it
+// cancels again (its integral is that of a wave), in FP32. It is integrated in
+// closed form between the first and the last cell end inside it:
+//
+//   int (g_A + s (r - r_A)) r Z0(k r) dr = [g r Z1 / k + s (r Z0 / k^2 - B / k^3)]
+//
+// (B the integral of Z0): two more rows of E per cell, V their weights, and
+// nothing in the cells between.
+//
+// Where the Y basis is asked for, the first cell is cut in half again and
+// again towards u = 0 (kDyadic cells), so that the singularity of Y0 stays a
+// cell length away from every cell.
+//
+// Kernels of a call, in order:
+//   xp_columns_kernel  which columns take the expansion, cell range per tile
+//                      of 64 frequencies; checks that r ascends
+//   xp_scan_kernel     where each tile's W blocks and GEMM units begin
+//   xp_basis_kernel    E
+//   xp_moments_kernel  W, in chunks of stations; the cells that a chunk
+//                      shares with its neighbours go to head / tail parts
+//   xp_join_kernel     adds those parts in chunk order
+//   xp_gemm_kernel     the product, in units of (128 velocities x 64 columns x
+//                      a run of cells)
+//   xp_finish_kernel   adds a column's units in order, |.| and normalisation
+//
+// Measured against the direct kernels on one B200 (device-resident call):
+// 19,900 pairs x 2048 f x 1000 c 61.3 -> 1.71 ms, 200 x 512 x 300 0.215 ->
+// 0.099 ms, 128 subarrays of 50-20,000 pairs (512 f x 500 c) 188 -> 6.2 ms; the
+// error against 64-bit quadrature 1.1e-6 -> 2e-7 of the spectrum (2-norm).
+//
+// Every sum is in an order fixed by the sizes, so results do not depend on
+// scheduling, nor on which frequencies share a call.
+#include <algorithm>
+#include <cmath>
+
+#include "fj_cells.cuh"
+#include "fj_expand.cuh"
+
+namespace ccfj {
+
+namespace {
+
+constexpr int kNodes = 16;          // Chebyshev terms of a cell
+constexpr double kCellPhase = 9.8;  // radians of a cell at the slowest velocity
+// Cells of one frequency: 2048 are 3190 wavelengths of the slowest velocity.
+// Columns with more go to the direct kernels.
+constexpr int kMaxCells = 2048;
+constexpr int kDyadic = 24;         // halved cells below the first (Y basis)
+constexpr int kTileCols = 64;       // frequencies of a W tile and GEMM column tile
+constexpr int kTileRows = 128;      // velocities of a GEMM tile
+constexpr int kGroup = 4;           // tiles begin and end with groups of cells
+constexpr int kEndRows = 2;         // rows of a cell's end
+constexpr int kEndFloats = kTileCols * kEndRows;  // one (tile, cell, input) of V
+constexpr int kBlockFloats = kTileCols * kNodes;  // one (tile, cell, input) of W
+// Intervals up to this share of a cell are short: whole in the cell of their
+// far end. A cell's polynomials live on [-kShort, 1] of it; the middle of that
+// is kCentre, and t = (x - middle) kPerHalf.
+constexpr float kShort = 0.0625f;
+constexpr float kCentre = 0.46875f;
+constexpr float kPerHalf = 1.8823529f;
+constexpr int kGemmThreads = 128;
+
+struct XpTile {
+  int lo, hi;    // cells [lo, hi) of the tile's columns, whole groups
+  long long w;   // first W block (cell blocks of one input)
+  long long unit;  // first GEMM unit
+};
+
+struct XpPlan {
+  double hu, inv_hu;  // cell length in u = r f, and its inverse
+  long long units;
+  int lo, hi;         // cells of E
+};
+
+struct XpDev {
+  const float* rs;
+  const float* wtr;
+  const long long* off;
+  int nsets;
+  long long total;
+  int nf, nc, ncp;       // ncp: velocities padded to GEMM tiles
+  const float* f;
+  const float* c;
+  InDesc in[2];
+  float* out;
+  int normalize;
+  int ft;                // column tiles of a set
+  int chunk;             // stations of a moments chunk
+  int mtiles;            // velocity tiles
+  int run;               // cells of a GEMM unit
+  int nsrc, nacc;        // products of a result, results of a column
+  int has_ends;          // itype 1: V and Eend are in use
+  int cells_cap;
+  long long blocks_cap, units_cap, slots;
+  unsigned char* use;
+  XpPlan* plan;
+  XpTile* tile;
+  int* bad;              // [nsets * ft] the tile's part of r is out of order
+  float* E;              // [basis][cell][16][ncp]
+  float* Eend;           // [basis][cell][2][ncp]
+  float* W;              // [block][input][64][16]
+  float* V;              // [block][input][64][2]
+  unsigned char* ends;   // [group] some column has weights in V
+  float* part;           // [unit][128][64]
+  float* head;           // [slot][nf][input][16]
+  float* tail;
+  int2* span;            // [slot][nf] first and last cell of a chunk
+};
+
+__device__ __forceinline__ long long set_begin(const XpDev& d, int b) { return d.off ? d.off[b] : 0; }
+__device__ __forceinline__ long long set_end(const XpDev& d, int b) {
+  return d.off ? d.off[b + 1] : d.total;
+}
+
+// ------------------------------------------------------------------ cells
+// x = r f / hu as a double-float product of r and fx = f / hu.
+struct Fx {
+  float hi, lo;
+};
+__device__ __forceinline__ Fx make_fx(float f, double inv_hu) {
+  const double v = __dmul_rn((double)f, inv_hu);  // (not fused: every kernel forms the same fx)
+  Fx x;
+  x.hi = (float)v;
+  x.lo = (float)(v - (double)x.hi);
+  return x;
+}
+
+// The cell that holds x = r f / hu, and x's place in it from kCentre (so that
+// its rounding is smallest, -kCentre .. 1 - kCentre). The cell never decreases
+// with r. DY: the cells below 1 are [2^(i-24), 2^(i-23)).
+template <bool DY>
+__device__ __forceinline__ int locate(float r, Fx fx, float& v) {
+  const float p = __fmul_rn(r, fx.hi);  // (not fused into p - c: l holds its rounding)
+  const float l = fmaf(r, fx.lo, fmaf(r, fx.hi, -p));
+  float c = floorf(p);
+  if ((p - c) + l < 0.0f) c -= 1.0f;
+  if (!DY || c >= 1.0f) {
+    v = (p - (c + kCentre)) + l;
+    return (int)c + (DY ? kDyadic - 1 : 0);
+  }
+  // x < 1: [len, 2 len) with len the power of two at or below x
+  float len = __int_as_float(__float_as_int(p) & 0x7f800000);
+  if (p >= 1.0f) len = 0.5f;  // x just below 1
+  if ((p - len) + l < 0.0f) len *= 0.5f;
+  v = ((p - len * (1.0f + kCentre)) + l) / len;
+  const int e = (__float_as_int(len) >> 23) - 127;  // -24 .. -1
+  return max(e + kDyadic, 0);
+}
+template <bool DY>
+__device__ __forceinline__ float cell_len(int cell) {
+  return DY && cell < kDyadic ? __int_as_float((cell - kDyadic + 127) << 23) : 1.0f;
+}
+template <bool DY>
+__device__ __forceinline__ float cell_begin(int cell) {
+  if (!DY) return (float)cell;
+  return cell < kDyadic ? cell_len<DY>(cell) : (float)(cell - kDyadic + 1);
+}
+
+// ------------------------------------------------------------------- plan
+// One CTA of 64 threads per (set, 64 frequencies).
+template <int MODE, int ITYPE>
+__global__ void xp_columns_kernel(XpDev d) {
+  constexpr bool DY = ModeTraits<MODE>::WY;
+  __shared__ float red[2][2];
+  __shared__ int ired[2][3];
+  const int t = threadIdx.x, b = blockIdx.y;
+  float lo = INFINITY, hi = -INFINITY;
+  bool fine = true;
+  for (int j = t; j < d.nc; j += 64) {
+    const float v = d.c[j];
+    fine = fine && v > 0.0f && v < INFINITY;
+    lo = fminf(lo, v);
+    hi = fmaxf(hi, v);
+  }
+  // this tile's share of the set's distances: finite and ascending
+  const long long o = set_begin(d, b), n = set_end(d, b) - o;
+  for (long long i = blockIdx.x * 64 + t; i < n; i += (long long)d.ft * 64) {
+    const float v = d.rs[o + i];
+    fine = fine && v >= 0.0f && v < INFINITY && (i == 0 || v >= d.rs[o + i - 1]);
+  }
+  for (int s = 16; s > 0; s >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, s));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, s));
+  }
+  fine = __all_sync(0xffffffffu, fine);
+  if ((t & 31) == 0) {
+    red[0][t >> 5] = lo;
+    red[1][t >> 5] = hi;
+    ired[t >> 5][2] = fine;
+  }
+  __syncthreads();
+  lo = fminf(red[0][0], red[0][1]);
+  fine = ired[0][2] && ired[1][2];
+  const double hu = kCellPhase / fjs::kTwoPi * (double)lo, inv_hu = 1.0 / hu;
+  const int tile = b * d.ft + blockIdx.x;
+  if (t == 0) d.bad[tile] = !fine;
+  if (tile == 0 && t == 0) {
+    d.plan->hu = hu;
+    d.plan->inv_hu = inv_hu;
+  }
+  const int fi = blockIdx.x * 64 + t;
+  int first = 0, last = 0;
+  bool use = false;
+  if (fine && fi < d.nf && n > 0) {
+    const float fl = d.f[fi];
+    const float r0 = d.rs[o], r1 = d.rs[o + n - 1];
+    if (fl == 0.0f) {
+      // itype 1: the column is NaN; itype 0: Z0(0) everywhere
+      use = ITYPE == 1 || !DY;
+      last = ITYPE == 1 ? 0 : 1;
+    } else if (fl >= 1e-20f && fl < INFINITY) {
+      const double x0 = (double)r0 * fl * inv_hu, x1 = (double)r1 * fl * inv_hu;
+      if (x1 < (double)(d.cells_cap - kGroup - (DY ? kDyadic : 0)) && (!DY || x0 >= 0x1p-23)) {
+        const Fx fx = make_fx(fl, inv_hu);
+        float rel;
+        first = locate<DY>(r0, fx, rel);
+        last = locate<DY>(r1, fx, rel) + 1;
+        // multiply-adds of the expansion against those of the direct kernel
+        // (56 issue slots a term measured on short intervals, 250 where most
+        // are long against the wavelength)
+        const double cells = last - first;
+        const double grid =
+            (cells + kGroup) * kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0) + 200.0 * n;
+        const double direct = (double)n * d.nc * d.nsrc * (cells > n ? 250.0 : 56.0);
+        use = grid < direct;
+      }
+    }
+    d.use[(long long)b * d.nf + fi] = use;
+  }
+  const bool has = use && last > first;
+  int mn = has ? first : 0x7fffffff, mx = has ? last : 0;
+  for (int s = 16; s > 0; s >>= 1) {
+    mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, s));
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+  }
+  if ((t & 31) == 0) {
+    ired[t >> 5][0] = mn;
+    ired[t >> 5][1] = mx;
+  }
+  __syncthreads();
+  if (t == 0) {
+    mn = min(ired[0][0], ired[1][0]);
+    mx = max(ired[0][1], ired[1][1]);
+    if (mx <= mn) mn = mx = 0;
+    d.tile[tile].lo = mn & ~(kGroup - 1);
+    d.tile[tile].hi = (mx + kGroup - 1) & ~(kGroup - 1);
+  }
+}
+
+// One CTA: exclusive sums over the tiles; without the memory for all of them,
+// or with distances out of order anywhere, every column goes direct.
+__global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
+  __shared__ long long sw[32], su[32];
+  __shared__ int slo[32], shi[32], sbad[32];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const int ntile = d.nsets * d.ft;
+  long long bw = 0, bu = 0;
+  int lo = 0x7fffffff, hi = 0, bad = 0;
+  for (int i0 = 0; i0 < ntile; i0 += 1024) {
+    const int i = i0 + t;
+    long long w = 0, u = 0;
+    if (i < ntile) {
+      const int a = d.tile[i].lo, z = d.tile[i].hi;
+      w = z - a;
+      u = (long long)d.nacc * d.mtiles * ((z - a + d.run - 1) / d.run);
+      if (z > a) {
+        lo = min(lo, a);
+        hi = max(hi, z);
+      }
+      bad |= d.bad[i];
+    }
+    long long iw = w, iu = u;
+    for (int s = 1; s < 32; s <<= 1) {
+      const long long pw = __shfl_up_sync(0xffffffffu, iw, s), pu = __shfl_up_sync(0xffffffffu, iu, s);
+      if (lane >= s) {
+        iw += pw;
+        iu += pu;
+      }
+    }
+    if (lane == 31) {
+      sw[wid] = iw;
+      su[wid] = iu;
+    }
+    __syncthreads();
+    long long ow = bw, ou = bu;
+    for (int k = 0; k < wid; ++k) {
+      ow += sw[k];
+      ou += su[k];
+    }
+    if (i < ntile) {
+      d.tile[i].w = ow + iw - w;
+      d.tile[i].unit = ou + iu - u;
+    }
+    for (int k = 0; k < 32; ++k) {
+      bw += sw[k];
+      bu += su[k];
+    }
+    __syncthreads();
+  }
+  for (int s = 16; s > 0; s >>= 1) {
+    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, s));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, s));
+    bad |= __shfl_xor_sync(0xffffffffu, bad, s);
+  }
+  if (lane == 0) {
+    slo[wid] = lo;
+    shi[wid] = hi;
+    sbad[wid] = bad;
+  }
+  __syncthreads();
+  for (int k = 0; k < 32; ++k) {
+    lo = min(lo, slo[k]);
+    hi = max(hi, shi[k]);
+    bad |= sbad[k];
+  }
+  const bool ok = !bad && bw <= d.blocks_cap && bu <= d.units_cap;
+  if (t == 0) {
+    d.plan->units = ok ? bu : 0;
+    d.plan->lo = ok && hi > lo ? lo : 0;
+    d.plan->hi = ok && hi > lo ? hi : 0;
+  }
+  if (!ok) {
+    const long long ncol = (long long)d.nsets * d.nf;
+    for (long long i = t; i < ncol; i += 1024) d.use[i] = 0;
+  }
+}
+
+// ------------------------------------------------------------------ basis
+// E: the values of Z0 at the cell's 16 Chebyshev nodes, from the FP64
+// functions (k r reaches 1e4 rad), to coefficients. T_4..T_7 and T_12..T_15
+// carry a minus sign here and in the moments, where it saves the negation of
+// the paired recurrence. One thread per (velocity, cell).
+template <int MODE, int ITYPE>
+__global__ void __launch_bounds__(kTileRows) xp_basis_kernel(XpDev d) {
+  using MT = ModeTraits<MODE>;
+  constexpr bool DY = MT::WY;
+  __shared__ double dct[kNodes][kNodes];  // [node][term]
+  __shared__ double node[kNodes];
+  const int t = threadIdx.x;
+  for (int e = t; e < kNodes * kNodes; e += kTileRows) {
+    const int m = e / kNodes, n = e % kNodes;
+    const double v = cospi(n * (m + 0.5) / kNodes) * (n == 0 ? 1.0 : 2.0) / kNodes;
+    dct[m][n] = n & 4 ? -v : v;
+  }
+  if (t < kNodes) node[t] = kCentre + cospi((t + 0.5) / kNodes) / (double)kPerHalf;
+  __syncthreads();
+  const int lo = d.plan->lo, hi = d.plan->hi;
+  const double hu = d.plan->hu;
+  const int j = blockIdx.x * kTileRows + t;
+  const double per_c = j < d.nc ? hu / (double)d.c[j] : 0.0;  // cycles per cell
+  for (int cell = lo + blockIdx.y; cell < hi; cell += gridDim.y) {
+    double eJ[kNodes], eY[kNodes];
+#pragma unroll
+    for (int n = 0; n < kNodes; ++n) eJ[n] = eY[n] = 0.0;
+    const double x0 = cell_begin<DY>(cell), len = cell_len<DY>(cell);
+    if (j < d.nc) {
+#pragma unroll 1
+      for (int m = 0; m < kNodes; ++m) {
+        const double cyc = (x0 + len * node[m]) * per_c;
+        ZB<double> J{}, Y{};
+        fjs::eval_station_f64<MT::WJ, MT::WY, false>(fjs::kTwoPi * cyc, cyc, J, Y);
+#pragma unroll
+        for (int n = 0; n < kNodes; ++n) {
+          const double w = dct[m][n];
+          if (MT::WJ) eJ[n] = fma(w, J.z0, eJ[n]);
+          if (MT::WY) eY[n] = fma(w, Y.z0, eY[n]);
+        }
+      }
+    }
+    const long long plane = (long long)d.cells_cap * kNodes * d.ncp;
+    float* e = d.E + (long long)cell * kNodes * d.ncp + j;
+#pragma unroll
+    for (int n = 0; n < kNodes; ++n) {
+      if (MT::WJ) e[(long long)n * d.ncp] = (float)eJ[n];
+      if (MT::WY) e[(MT::WJ ? plane : 0) + (long long)n * d.ncp] = (float)eY[n];
+    }
+    if (ITYPE == 1) {
+      // the cell's end, with r in cells and k = 2 pi per_c
+      ZB<double> J{}, Y{};
+      double r1 = 0.0, r2J = 0.0, r2Y = 0.0, r1Y = 0.0;
+      if (j < d.nc) {
+        const double x = x0 + len, cyc = x * per_c, ik = 1.0 / (fjs::kTwoPi * per_c);
+        fjs::eval_station_f64<MT::WJ, MT::WY, true>(fjs::kTwoPi * cyc, cyc, J, Y);
+        r1 = x * J.z1 * ik;
+        r2J = (x * J.z0 - J.b * ik) * ik * ik;
+        r1Y = x * Y.z1 * ik;
+        r2Y = (x * Y.z0 - Y.b * ik) * ik * ik;
+      }
+      const long long eplane = (long long)d.cells_cap * kEndRows * d.ncp;
+      float* v = d.Eend + (long long)cell * kEndRows * d.ncp + j;
+      if (MT::WJ) {
+        v[0] = (float)r1;
+        v[d.ncp] = (float)r2J;
+      }
+      if (MT::WY) {
+        v[MT::WJ ? eplane : 0] = (float)r1Y;
+        v[(MT::WJ ? eplane : 0) + d.ncp] = (float)r2Y;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------- moments
+// acc[m] += a (T_2m, T_2m+1) (signed as above) at t. The pairs follow the
+// recurrence of step 2, T_{n+2} = 2 T_2 T_n - T_{n-2}; the signs turn it into
+// R_{m+1} = -+ (2 T_2) R_m + R_{m-1}. With one input the recurrence runs on
+// a R_m itself.
+template <int NIN>
+__device__ __forceinline__ void add_point(float2 (&acc)[NIN][kNodes / 2], float t,
+                                          const float (&a)[NIN]) {
+  const float dt = t + t;
+  const float t2 = fmaf(dt, t, -1.0f);
+  const float t3 = fmaf(dt, t2, -t);
+  const float2 s = fjs::psplat(t2 + t2), ns = fjs::psplat(-(t2 + t2));
+  float2 p = make_float2(1.0f, t), q = make_float2(t2, t3);
+  if (NIN == 1) {
+    p = make_float2(a[0], a[0] * t);
+    q = make_float2(a[0] * t2, a[0] * t3);
+  }
+#pragma unroll
+  for (int m = 0; m < kNodes / 2; ++m) {
+    if (NIN == 1) {
+      acc[0][m] = fjs::padd(acc[0][m], p);
+    } else {
+#pragma unroll
+      for (int k = 0; k < NIN; ++k) acc[k][m] = fjs::pfma(fjs::psplat(a[k]), p, acc[k][m]);
+    }
+    const float2 n = fjs::pfma(m & 1 ? s : ns, q, p);  // R_{m+2}
+    p = q;
+    q = n;
+  }
+}
+
+// Gauss rules of 5 and 9 points, one after the other: (x, weight).
+__constant__ float2 kRule[14] = {
+    {-0.906179846f, 0.236926885f}, {-0.538469310f, 0.478628670f}, {0.0f, 0.568888889f},
+    {0.538469310f, 0.478628670f},  {0.906179846f, 0.236926885f},
+    {-0.968160240f, 0.081274388f}, {-0.836031107f, 0.180648161f}, {-0.613371433f, 0.260610696f},
+    {-0.324253423f, 0.312347077f}, {0.0f, 0.330239355f},          {0.324253423f, 0.312347077f},
+    {0.613371433f, 0.260610696f},  {0.836031107f, 0.180648161f},  {0.968160240f, 0.081274388f}};
+
+// One point of a piece: its middle tm and half length th in the cell's t, in r
+// rm and hr; the spectrum's value gm at the middle and its rise gh over half
+// the piece.
+template <int NIN>
+__device__ __forceinline__ void piece_point(float2 (&acc)[NIN][kNodes / 2], float x, float w,
+                                            float tm, float th, float rm, float hr,
+                                            const float (&gm)[NIN], const float (&gh)[NIN]) {
+  float a[NIN];
+  const float rw = fmaf(hr, x, rm) * (hr * w);
+#pragma unroll
+  for (int k = 0; k < NIN; ++k) a[k] = fmaf(gh[k], x, gm[k]) * rw;
+  add_point<NIN>(acc, fmaf(th, x, tm), a);
+}
+
+// Slot of a set's first chunk: sets' slots do not overlap, since a set of n
+// pairs has at most n / chunk + 1 chunks.
+__device__ __forceinline__ long long slot_begin(const XpDev& d, int b) {
+  return set_begin(d, b) / d.chunk + b;
+}
+__device__ __forceinline__ int chunks_of(const XpDev& d, long long n) {
+  return max(1, (int)((n - 1 + d.chunk - 1) / d.chunk));
+}
+__device__ __forceinline__ int set_of_slot(const XpDev& d, long long slot) {
+  int lo = 0, hi = d.nsets;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (slot_begin(d, mid) <= slot)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
+// A CTA is one warp; it takes 32 frequencies and a chunk of stations. Chunk q
+// visits the stations after q chunk up to (q + 1) chunk (chunk 0 of itype 0 its
+// first station too), and for itype 1 the intervals that end there. Its lanes
+// keep the 16 moments of the cell they are in; a finished cell that the chunk
+// has to itself goes to W, the first one to head, the last one to tail (their
+// numbers to span).
+//
+// An interval (or the piece of it in one cell) takes the Gauss rule of 2, 3, 5
+// or 9 points by its length d in cells: each rule is at most 5e-8 of the
+// integral off where the next one begins, at 0.1, 0.6, 2.5 and 9.8 radians. A
+// short interval is not cut at a cell's end: since the lanes' cells end at
+// different stations, cutting each one ran two pieces in nearly every step.
+//
+// Bound by issue: 15 paired multiply-adds and about as many other instructions
+// a point, 2 or 3 points for most intervals. The spectra come in by cp.async,
+// 32 stations ahead; unrolling the stations instead (loads into registers)
+// left the warps waiting for instructions as long as they issued.
+template <int NIN>
+struct MomStage {
+  float g[NIN][32][32];  // [station][frequency]
+  float4 st[32];         // r, the interval's length, 1 / max(length, 0.1), trapezoid weight
+};
+
+template <int NIN, int ITYPE, bool DY>
+__global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
+  __shared__ __align__(16) MomStage<NIN> stage[2];
+  __shared__ float2 rule[14];
+  const int lane = threadIdx.x;
+  const long long slot = blockIdx.x / ftiles;
+  const int fi = (int)(blockIdx.x % ftiles) * 32 + lane;
+  const int b = set_of_slot(d, slot);
+  const long long o = set_begin(d, b);
+  const int n = (int)(set_end(d, b) - o);
+  const int q = (int)(slot - slot_begin(d, b));
+  if (q >= chunks_of(d, n)) return;
+  const bool mine = fi < d.nf && d.use[(long long)b * d.nf + fi] != 0 &&
+                    !(ITYPE == 1 && d.f[fi] == 0.0f);
+  if (__all_sync(0xffffffffu, !mine)) return;
+  if (lane < 14) rule[lane] = kRule[lane];
+  const int fc = min(fi, d.nf - 1);
+  const float fl = mine ? d.f[fc] : 0.0f;
+  const Fx fx = make_fx(fl, d.plan->inv_hu);
+  const float huf = ITYPE == 1 ? (float)(d.plan->hu / (double)(mine ? fl : 1.0f)) : 0.0f;
+  const XpTile tile = d.tile[b * d.ft + fc / kTileCols];
+  const int s0 = q * d.chunk, s1 = min(s0 + d.chunk, n - 1);
+  const float* const rs = d.rs + o;
+  float2 acc[NIN][kNodes / 2], tot[NIN][kNodes / 2];
+#pragma unroll
+  for (int k = 0; k < NIN; ++k)
+#pragma unroll
+    for (int m = 0; m < kNodes / 2; ++m) acc[k][m] = tot[k][m] = make_float2(0.f, 0.f);
+  bool more = false;  // tot holds part of the cell's sums
+  float vA;
+  int cell = locate<DY>(rs[s0], fx, vA);
+  const int cell0 = cell;
+  float base_x = cell_begin<DY>(cell);
+  const long long edge = ((slot * d.nf + fc) * NIN) * kNodes;
+  float* W = d.W + (tile.w + cell - tile.lo) * NIN * kBlockFloats + (fc & (kTileCols - 1)) * kNodes;
+  float* V = ITYPE == 1 ? d.V + (tile.w + cell - tile.lo) * NIN * kEndFloats +
+                              (fc & (kTileCols - 1)) * kEndRows
+                        : nullptr;
+  auto store = [&](float* base, long long step) {
+    if (more) {
+#pragma unroll
+      for (int k = 0; k < NIN; ++k)
+#pragma unroll
+        for (int m = 0; m < kNodes / 2; ++m) {
+          acc[k][m] = fjs::padd(acc[k][m], tot[k][m]);
+          tot[k][m] = make_float2(0.f, 0.f);
+        }
+      more = false;
+    }
+#pragma unroll
+    for (int k = 0; k < NIN; ++k) {
+      float4* p = reinterpret_cast<float4*>(base + k * step);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        p[m] = make_float4(acc[k][2 * m].x, acc[k][2 * m].y, acc[k][2 * m + 1].x,
+                           acc[k][2 * m + 1].y);
+        acc[k][2 * m] = acc[k][2 * m + 1] = make_float2(0.f, 0.f);
+      }
+    }
+  };
+  // the cell is finished; vx, vy: the weights of its end
+  auto flush = [&](const float (&vx)[NIN], const float (&vy)[NIN], bool ends) {
+    const bool first = cell == cell0;
+    store(first ? d.head + edge : W, first ? kNodes : kBlockFloats);
+    if (ITYPE == 1) {
+#pragma unroll
+      for (int k = 0; k < NIN; ++k)
+        *reinterpret_cast<float2*>(V + k * kEndFloats) = make_float2(vx[k], vy[k]);
+      if (ends) d.ends[(tile.w + cell - tile.lo) / kGroup] = 1;
+      V += NIN * kEndFloats;
+    }
+    W += NIN * kBlockFloats;
+    ++cell;
+    if (DY)
+      base_x = cell_begin<DY>(cell);
+    else
+      base_x += 1.0f;
+  };
+  const float* u[NIN];
+#pragma unroll
+  for (int k = 0; k < NIN; ++k) u[k] = d.in[k].p + (long long)fc * d.in[k].cs;
+  auto row_of = [&](int k, int i) -> long long {
+    const long long* perm = d.in[k].perm;
+    return (perm ? __ldg(perm + o + i) : o + i) * d.in[k].ld;
+  };
+  // stations base .. base + 31 (each lane one station's numbers, all lanes
+  // every station's spectrum)
+  auto load = [&](int base, int buf) {
+    const int i = min(base + lane, s1);
+    const float r = rs[i];
+    const float D = ITYPE == 1 ? r - rs[i - 1] : 0.0f;
+    stage[buf].st[lane] = make_float4(r, D, 1.0f / fmaxf(D, 0.1f), ITYPE == 0 ? d.wtr[o + i] : 0.0f);
+    long long row[NIN];
+#pragma unroll
+    for (int k = 0; k < NIN; ++k) row[k] = row_of(k, i);
+    const int cnt = min(32, s1 - base + 1);
+    for (int j = 0; j < cnt; ++j)
+#pragma unroll
+      for (int k = 0; k < NIN; ++k)
+        cp_async4(&stage[buf].g[k][j][lane], u[k] + __shfl_sync(0xffffffffu, row[k], j));
+    cp_async_commit();
+  };
+  if (s0 + 1 <= s1) load(s0 + 1, 0);
+  float gA[NIN];
+#pragma unroll
+  for (int k = 0; k < NIN; ++k) gA[k] = __ldg(u[k] + row_of(k, s0));
+  if (ITYPE == 0 && q == 0 && mine) {
+    float a[NIN];
+#pragma unroll
+    for (int k = 0; k < NIN; ++k) a[k] = gA[k] * d.wtr[o];
+    add_point<NIN>(acc, vA * kPerHalf, a);
+  }
+  int buf = 0;
+  for (int base = s0 + 1; base <= s1; base += 32, buf ^= 1) {
+    if (base + 32 <= s1)
+      load(base + 32, buf ^ 1);
+    else
+      cp_async_commit();  // one group per round keeps the count below
+    cp_async_wait<1>();
+    __syncwarp();
+    const int cnt = mine ? min(32, s1 - base + 1) : 0;
+    const int mark = cell;
+#pragma unroll 1
+    for (int j = 0; j < cnt; ++j) {
+      const float4 st = stage[buf].st[j];
+      const float rB = st.x, D = st.y;
+      // the station's cell and place, as locate() finds them, from the cell
+      // that the lane is in
+      const float p = __fmul_rn(rB, fx.hi);
+      const float l = fmaf(rB, fx.lo, fmaf(rB, fx.hi, -p));
+      int cB = cell;
+      float vB;
+      if (DY && cell < kDyadic) {
+        cB = locate<DY>(rB, fx, vB);
+      } else {
+        if ((p - (base_x + 1.0f)) + l >= 0.0f) cB = locate<DY>(rB, fx, vB);
+        vB = (p - (base_x + (float)(cB - cell) + kCentre)) + l;
+      }
+      float gB[NIN], gm[NIN], gh[NIN];
+#pragma unroll
+      for (int k = 0; k < NIN; ++k) gB[k] = stage[buf].g[k][j][lane];
+      // itype 1: a short interval whole, in the cell of its far end; a long one
+      // from its beginning to the first cell end, from the last cell end on,
+      // and between the two in closed form. (Lanes that end a cell do so before
+      // all lanes' points.)
+      const float dB = D * fx.hi * (DY ? 1.0f / cell_len<DY>(cB) : 1.0f);
+      if (ITYPE == 0 || dB <= kShort) {
+        if (cell < cB) {
+          float none[NIN];
+#pragma unroll
+          for (int k = 0; k < NIN; ++k) none[k] = 0.0f;
+#pragma unroll 1
+          do
+            flush(none, none, false);
+          while (cell < cB);
+        }
+        if (ITYPE == 0) {
+#pragma unroll
+          for (int k = 0; k < NIN; ++k) gm[k] = gB[k] * st.w;
+          add_point<NIN>(acc, vB * kPerHalf, gm);
+        } else {
+          const float hr = 0.5f * D, th = 0.5f * kPerHalf * dB;
+          const float tm = fmaf(vB, kPerHalf, -th), rm = rB - hr;
+#pragma unroll
+          for (int k = 0; k < NIN; ++k) {
+            // over the reference's floor of an interval (src/FJcpu.cpp:259)
+            gh[k] = (gB[k] - gA[k]) * (st.z * hr);
+            gm[k] = gA[k] + gh[k];
+          }
+          if (dB <= 0.01f) {
+            piece_point<NIN>(acc, -0.577350269f, 1.0f, tm, th, rm, hr, gm, gh);
+            piece_point<NIN>(acc, 0.577350269f, 1.0f, tm, th, rm, hr, gm, gh);
+          } else {
+            piece_point<NIN>(acc, -0.774596669f, 0.555555556f, tm, th, rm, hr, gm, gh);
+            piece_point<NIN>(acc, 0.0f, 0.888888889f, tm, th, rm, hr, gm, gh);
+            piece_point<NIN>(acc, 0.774596669f, 0.555555556f, tm, th, rm, hr, gm, gh);
+          }
+        }
+      } else {
+        const int span = cB - cell;
+#pragma unroll 1
+        for (int step = 0;; ++step) {
+          const bool cross = step < span;
+          float hr = 0.0f;
+          if (!cross || step == 0) {
+            const float va = step == 0 ? vA : -kCentre;
+            const float w = (cross ? 1.0f - kCentre : vB) - va;  // in cells
+            const float cl = cell_len<DY>(cell);
+            hr = span == 0 ? 0.5f * D : 0.5f * w * cl * huf;
+            const float th = 0.5f * kPerHalf * w, tm = fmaf(va, kPerHalf, th);
+            const float rm = fmaf(cl, fmaf(0.5f, w, va) + kCentre, cell_begin<DY>(cell)) * huf;
+#pragma unroll
+            for (int k = 0; k < NIN; ++k) {
+              const float sl = (gB[k] - gA[k]) * st.z;
+              gm[k] = fmaf(sl, cross || span == 0 ? hr : D - hr, gA[k]);
+              gh[k] = sl * hr;
+            }
+            const bool five = w <= 0.25f;
+#pragma unroll 1
+            for (int i = five ? 0 : 5; i < (five ? 5 : 14); ++i)
+              piece_point<NIN>(acc, rule[i].x, rule[i].y, tm, th, rm, hr, gm, gh);
+          }
+          if (!cross) break;
+          float vx[NIN], vy[NIN];
+          const bool ends = span > 1 && (step == 0 || step == span - 1);
+#pragma unroll
+          for (int k = 0; k < NIN; ++k) {
+            vx[k] = vy[k] = 0.0f;
+            if (ends) {
+              // the spectrum's line at the cell end: from A, or from B back
+              const float sl = (gB[k] - gA[k]) * st.z;
+              const float back = (vB + kCentre) * cell_len<DY>(cB) * huf;
+              const float h2 = step == 0 ? -huf * huf : huf * huf;
+              vx[k] = h2 * fmaf(sl, step == 0 ? 2.0f * hr : D - back, gA[k]);
+              vy[k] = h2 * huf * sl;
+            }
+          }
+          flush(vx, vy, ends);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < NIN; ++k) gA[k] = gB[k];
+      vA = vB;
+    }
+    // many stations to a cell (low frequencies): sums of 32 stations, added up
+    if (cell == mark) {
+#pragma unroll
+      for (int k = 0; k < NIN; ++k)
+#pragma unroll
+        for (int m = 0; m < kNodes / 2; ++m) {
+          tot[k][m] = fjs::padd(tot[k][m], acc[k][m]);
+          acc[k][m] = make_float2(0.f, 0.f);
+        }
+      more = true;
+    }
+    __syncwarp();  // the stage is filled again
+  }
+  if (!mine) return;
+  store((cell == cell0 ? d.head : d.tail) + edge, kNodes);
+  d.span[slot * d.nf + fi] = make_int2(cell0, cell);
+}
+
+// Adds the parts of the cells that lie across chunk boundaries, in chunk
+// order, and clears the cells of the tile that a column does not reach. Four
+// threads per (slot, frequency). The first chunk that begins in a cell adds
+// all that the cell got: the tail of the chunk before it, its own head, and
+// the heads of the chunks after it that begin in the same cell.
+template <int NIN, int ITYPE, bool DY>
+__global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
+  const int n4 = threadIdx.x & 3;
+  const int fi = blockIdx.y * 64 + (threadIdx.x >> 2);
+  const long long slot = blockIdx.x;
+  if (fi >= d.nf) return;
+  const int b = set_of_slot(d, slot);
+  const int n = (int)(set_end(d, b) - set_begin(d, b));
+  const int q = (int)(slot - slot_begin(d, b)), nch = chunks_of(d, n);
+  if (q >= nch || !d.use[(long long)b * d.nf + fi]) return;
+  if (ITYPE == 1 && d.f[fi] == 0.0f) return;
+  const int2* span = d.span + slot * d.nf + fi;  // of chunk q + i: span[i nf]
+  const int2 me = span[0];
+  const int before = q > 0 ? span[-(long long)d.nf].x : -1;
+  if (before == me.x && q != nch - 1) return;
+  const XpTile tile = d.tile[b * d.ft + fi / kTileCols];
+  float* const col = d.W + (fi & (kTileCols - 1)) * kNodes + n4 * 4;
+  auto put = [&](int cell, int k, float4 v) {
+    *reinterpret_cast<float4*>(col + ((tile.w + cell - tile.lo) * NIN + k) * kBlockFloats) = v;
+  };
+  const long long step = (long long)d.nf * NIN * kNodes;
+  const long long at = ((slot * d.nf + fi) * NIN) * kNodes + n4 * 4;
+  auto add = [](float4& v, const float* p) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p));
+    v = make_float4(v.x + a.x, v.y + a.y, v.z + a.z, v.w + a.w);
+  };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto clear_end = [&](int cell) {
+    if (ITYPE == 0 || n4 != 0) return;
+    float* p = d.V + (tile.w + cell - tile.lo) * NIN * kEndFloats + (fi & (kTileCols - 1)) * kEndRows;
+#pragma unroll
+    for (int k = 0; k < NIN; ++k) *reinterpret_cast<float2*>(p + k * kEndFloats) = make_float2(0.f, 0.f);
+  };
+  if (q == 0)
+    for (int c = tile.lo; c < me.x; ++c) {
+#pragma unroll
+      for (int k = 0; k < NIN; ++k) put(c, k, zero);
+      clear_end(c);
+    }
+  if (before != me.x) {
+#pragma unroll
+    for (int k = 0; k < NIN; ++k) {
+      float4 v = zero;
+      if (q > 0) add(v, d.tail + at - step + k * kNodes);
+      add(v, d.head + at + k * kNodes);
+      // eight chunks' loads at a time (many stations to a cell: low frequencies)
+      for (int c = 1; q + c < nch; c += 8) {
+        float4 h[8];
+        bool in[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int cc = min(c + i, nch - 1 - q);
+          in[i] = q + c + i < nch && span[(long long)cc * d.nf].x == me.x;
+          h[i] = __ldg(reinterpret_cast<const float4*>(d.head + at + cc * step + k * kNodes));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (in[i]) v = make_float4(v.x + h[i].x, v.y + h[i].y, v.z + h[i].z, v.w + h[i].w);
+        if (!in[7]) break;
+      }
+      put(me.x, k, v);
+    }
+  }
+  if (q == nch - 1) {
+    if (me.y != me.x) {
+#pragma unroll
+      for (int k = 0; k < NIN; ++k) {
+        float4 v = zero;
+        add(v, d.tail + at + k * kNodes);
+        put(me.y, k, v);
+      }
+    }
+    clear_end(me.y);
+    for (int c = me.y + 1; c < tile.hi; ++c) {
+#pragma unroll
+      for (int k = 0; k < NIN; ++k) put(c, k, zero);
+      clear_end(c);
+    }
+  }
+}
+
+// ------------------------------------------------------------------- GEMM
+// Units of 128 velocities x 64 columns x up to `run` cells; a thread holds
+// 8 x 8 results. Per cell (16 terms) the E rows come in by cp.async and the W
+// block, which lies column by column, through registers, transposed.
+struct GemmStage {
+  float e[kNodes][kTileRows];
+  float w[kNodes][kTileCols + 4];
+};
+
+template <int NSRC>
+__global__ void __launch_bounds__(kGemmThreads, 3) xp_gemm_kernel(XpDev d) {
+  __shared__ __align__(16) GemmStage st[2];
+  __shared__ int s_tile;
+  __shared__ unsigned s_ends;
+  const int tid = threadIdx.x;
+  const int tn = tid & 7, tm = tid >> 3;
+  const int ntile = d.nsets * d.ft;
+  const int nin = d.nacc > NSRC ? d.nacc : NSRC;
+  const long long plane = (long long)d.cells_cap * kNodes * d.ncp;
+  for (long long unit = blockIdx.x; unit < d.plan->units; unit += gridDim.x) {
+    if (tid == 0) {
+      int lo = 0, hi = ntile;  // the last tile whose first unit is not past `unit`
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (d.tile[mid].unit <= unit)
+          lo = mid;
+        else
+          hi = mid;
+      }
+      s_tile = lo;
+    }
+    __syncthreads();
+    const XpTile tile = d.tile[s_tile];
+    const int rest = (int)(unit - tile.unit);
+    const int mt = rest % d.mtiles;
+    const int q = (rest / d.mtiles) % d.nacc;
+    const int c0 = tile.lo + rest / (d.mtiles * d.nacc) * d.run;
+    const int c1 = min(c0 + d.run, tile.hi);
+    // which of the unit's groups have end rows
+    if (tid < 32) {
+      const int g = c0 + tid * kGroup;
+      const bool ends = d.has_ends && g < c1 && d.ends[(tile.w + g - tile.lo) / kGroup] != 0;
+      const unsigned m = __ballot_sync(0xffffffffu, ends);
+      if (tid == 0) s_ends = m;
+    }
+    __syncthreads();
+    const unsigned ends = s_ends;
+    // the steps: a group's four cells and, if it has them, its end rows, each
+    // for every source
+    struct Step {
+      int cell, sub, src;
+    };
+    auto next = [&](Step p) {
+      if (++p.src < NSRC) return p;
+      p.src = 0;
+      if (p.sub < kGroup) ++p.cell;
+      ++p.sub;
+      if (p.sub == kGroup && !(ends >> ((p.cell - c0) / kGroup - 1) & 1)) ++p.sub;
+      if (p.sub > kGroup) p.sub = 0;
+      return p;
+    };
+    float4 wreg[2];
+    auto load = [&](const Step& p, int buf) {
+      const int in = NSRC == 2 && p.src ? 1 - q : q;
+      if (p.sub < kGroup) {
+        const float* e = d.E + (p.src ? plane : 0) + (long long)p.cell * kNodes * d.ncp + mt * kTileRows;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int v = tid + i * kGemmThreads;  // 16 rows of 32 float4
+          cp_async16(&st[buf].e[v >> 5][(v & 31) * 4], e + (long long)(v >> 5) * d.ncp + (v & 31) * 4);
+        }
+        const float4* w = reinterpret_cast<const float4*>(
+            d.W + ((tile.w + p.cell - tile.lo) * nin + in) * kBlockFloats);
+        wreg[0] = __ldg(w + tid);
+        wreg[1] = __ldg(w + tid + kGemmThreads);
+      } else {  // p.cell is the first cell of the next group
+        const int g = p.cell - kGroup;
+        const float* e = d.Eend + (p.src ? plane / kNodes * kEndRows : 0) +
+                         (long long)g * kEndRows * d.ncp + mt * kTileRows;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int v = tid + i * kGemmThreads;  // 8 rows
+          cp_async16(&st[buf].e[v >> 5][(v & 31) * 4], e + (long long)(v >> 5) * d.ncp + (v & 31) * 4);
+        }
+        // four cells of 64 columns x 2: a thread takes two columns of a cell
+        wreg[0] = __ldg(reinterpret_cast<const float4*>(
+                            d.V + ((tile.w + g + (tid >> 5) - tile.lo) * nin + in) * kEndFloats) +
+                        (tid & 31));
+      }
+      cp_async_commit();
+    };
+    auto put = [&](const Step& p, int buf) {
+      const float sg = NSRC == 2 && p.src && q == 0 ? -1.0f : 1.0f;
+      if (p.sub == kGroup) {
+        const int k = (tid >> 5) * kEndRows, col = (tid & 31) * 2;
+        st[buf].w[k][col] = sg * wreg[0].x;
+        st[buf].w[k + 1][col] = sg * wreg[0].y;
+        st[buf].w[k][col + 1] = sg * wreg[0].z;
+        st[buf].w[k + 1][col + 1] = sg * wreg[0].w;
+        return;
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int v = tid + i * kGemmThreads, col = v >> 2, k = (v & 3) * 4;
+        st[buf].w[k][col] = sg * wreg[i].x;
+        st[buf].w[k + 1][col] = sg * wreg[i].y;
+        st[buf].w[k + 2][col] = sg * wreg[i].z;
+        st[buf].w[k + 3][col] = sg * wreg[i].w;
+      }
+    };
+    // sums of a group, added to the unit's totals: 64 terms in a row round half
+    // as much as a unit's 1024 do
+    float2 acc[8][4], tot[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = tot[i][j] = make_float2(0.f, 0.f);
+    Step cur{c0, 0, 0};
+    load(cur, 0);
+    for (int buf = 0;; buf ^= 1) {
+      put(cur, buf);
+      cp_async_wait<0>();
+      __syncthreads();
+      const Step nx = next(cur);
+      const bool more = nx.cell < c1 || nx.sub == kGroup;
+      if (more) load(nx, buf ^ 1);
+      const int rows = cur.sub < kGroup ? kNodes : kGroup * kEndRows;
+#pragma unroll 8
+      for (int k = 0; k < rows; ++k) {
+        const float4 e0 = *reinterpret_cast<const float4*>(&st[buf].e[k][tm * 4]);
+        const float4 e1 = *reinterpret_cast<const float4*>(&st[buf].e[k][64 + tm * 4]);
+        const float4 w0 = *reinterpret_cast<const float4*>(&st[buf].w[k][tn * 4]);
+        const float4 w1 = *reinterpret_cast<const float4*>(&st[buf].w[k][32 + tn * 4]);
+        const float ev[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+        const float2 wv[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w),
+                              make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fjs::pfma(fjs::psplat(ev[i]), wv[j], acc[i][j]);
+      }
+      if (nx.sub == 0 && nx.src == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            tot[i][j] = fjs::padd(tot[i][j], acc[i][j]);
+            acc[i][j] = make_float2(0.f, 0.f);
+          }
+      }
+      if (!more) break;
+      cur = nx;
+    }
+    float* o = d.part + unit * (kTileRows * kTileCols);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = (i & 4) * 16 + tm * 4 + (i & 3);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float4*>(o + row * kTileCols + h * 32 + tn * 4) = make_float4(
+            tot[i][2 * h].x, tot[i][2 * h].y, tot[i][2 * h + 1].x, tot[i][2 * h + 1].y);
+    }
+    __syncthreads();  // the stages and s_tile are used again
+  }
+}
+
+// ----------------------------------------------------------------- finish
+// The units of a result added in order, the mode's magnitude, NaN at f = 0
+// (itype 1, as the reference's 1/k), and the normalisation with Python's
+// builtin max (see fj_normalize_kernel). A CTA takes 16 columns of one set; a
+// thread keeps its velocities' values in registers up to 1024 velocities.
+constexpr int kFinRows = 32, kFinKeep = 32;
+template <int MODE, int ITYPE>
+__global__ void __launch_bounds__(16 * kFinRows) xp_finish_kernel(XpDev d) {
+  constexpr int NACC = ModeTraits<MODE>::NACC;
+  __shared__ float red[kFinRows][17];
+  const int fi = blockIdx.x * 16 + threadIdx.x, b = blockIdx.y;
+  const bool mine = fi < d.nf && d.use[(long long)b * d.nf + min(fi, d.nf - 1)] != 0;
+  if (!__syncthreads_or(mine)) return;
+  const XpTile tile = d.tile[b * d.ft + (blockIdx.x * 16) / kTileCols];
+  const int nrun = (tile.hi - tile.lo + d.run - 1) / d.run;
+  const bool nan_col = ITYPE == 1 && mine && d.f[fi] == 0.0f;
+  float* o = d.out + (long long)b * d.nc * d.nf + fi;
+  auto value = [&](int c) {
+    float v[2] = {0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < NACC; ++q) {
+      const float* p = d.part +
+                       (tile.unit + q * d.mtiles + c / kTileRows) * (kTileRows * kTileCols) +
+                       (c % kTileRows) * kTileCols + (fi & (kTileCols - 1));
+      const long long step = (long long)d.mtiles * NACC * kTileRows * kTileCols;
+#pragma unroll 4
+      for (int s = 0; s < nrun; ++s) v[q] += p[s * step];
+    }
+    if (nan_col) return __int_as_float(0x7fffffff);
+    return NACC == 1 ? v[0] : sqrtf(v[0] * v[0] + v[1] * v[1]);
+  };
+  float keep[kFinKeep];
+  const bool in_regs = d.nc <= kFinRows * kFinKeep;
+  float m = -INFINITY;
+  if (mine) {
+    if (in_regs) {
+#pragma unroll
+      for (int i = 0; i < kFinKeep; ++i) {
+        const int c = threadIdx.y + i * kFinRows;
+        if (c < d.nc) {
+          keep[i] = value(c);
+          m = fmaxf(m, fabsf(keep[i]));
+        }
+      }
+    } else {
+      for (int c = threadIdx.y; c < d.nc; c += kFinRows) {
+        const float v = value(c);
+        o[(long long)c * d.nf] = v;
+        m = fmaxf(m, fabsf(v));
+      }
+    }
+  }
+  red[threadIdx.y][threadIdx.x] = m;
+  __shared__ float first[16];
+  if (threadIdx.y == 0 && mine) first[threadIdx.x] = fabsf(in_regs ? keep[0] : o[0]);
+  __syncthreads();
+  if (!mine) return;
+  float div = 1.0f;
+  if (d.normalize) {
+    for (int y = 0; y < kFinRows; ++y) m = fmaxf(m, red[y][threadIdx.x]);
+    const float f0 = first[threadIdx.x];
+    div = isnan(f0) ? f0 : m;
+  }
+  if (in_regs) {
+#pragma unroll
+    for (int i = 0; i < kFinKeep; ++i) {
+      const int c = threadIdx.y + i * kFinRows;
+      if (c < d.nc) o[(long long)c * d.nf] = d.normalize ? keep[i] / div : keep[i];
+    }
+  } else if (d.normalize) {
+    for (int c = threadIdx.y; c < d.nc; c += kFinRows) o[(long long)c * d.nf] /= div;
+  }
+}
+
+// ------------------------------------------------------------------- host
+int nin_of(int mode) { return mode == CCFJ_MODE_J || mode == CCFJ_MODE_Y ? 1 : 2; }
+int nsrc_of(int mode) { return mode == CCFJ_MODE_J_MINUS_Y || mode == CCFJ_MODE_ABS_H ? 2 : 1; }
+int nacc_of(int mode) { return mode == CCFJ_MODE_ABS_J || mode == CCFJ_MODE_ABS_H ? 2 : 1; }
+
+size_t round256(size_t v) { return (v + 255) & ~size_t(255); }
+
+// Sizes, and places relative to `base`; returns the bytes needed.
+size_t layout(const XpProblem& p, void* base, XpDev* out) {
+  XpDev d{};
+  d.rs = p.rs;
+  d.wtr = p.wtr;
+  d.off = p.off;
+  d.nsets = p.nsets;
+  d.total = p.total;
+  d.nf = p.nf;
+  d.nc = p.nc;
+  d.f = p.f;
+  d.c = p.c;
+  d.in[0] = p.in[0];
+  d.in[1] = p.in[1];
+  d.out = p.out;
+  d.normalize = p.normalize;
+  d.ft = (int)div_up(p.nf, kTileCols);
+  d.mtiles = (int)div_up(p.nc, kTileRows);
+  d.ncp = d.mtiles * kTileRows;
+  d.nsrc = nsrc_of(p.mode);
+  d.nacc = nacc_of(p.mode);
+  d.has_ends = p.itype == 1;
+  const int nin = nin_of(p.mode);
+  const bool batch = p.off != nullptr;
+  // Stations of a moments chunk: long chunks leave fewer shared cells to
+  // join, short ones keep the SMs busy when there are few pairs.
+  if (batch)
+    d.chunk = p.total_all >= 100000 ? 128 : 32;
+  else
+    d.chunk = p.total <= 1024 ? 8 : p.total <= 2048 ? 16 : p.total <= 4096 ? 32 : p.total <= 8192 ? 64 : 128;
+  // Shorter runs of cells where the tiles alone leave SMs idle.
+  const long long mn = (long long)div_up(p.nf_all, kTileCols) * d.mtiles * d.nacc;
+  d.run = batch || mn >= 256 ? 64 : mn >= 64 ? 32 : 16;
+  // No column that is cheaper here than directly (xp_columns_kernel) has more
+  // cells than this.
+  const double most = (double)p.total * p.nc * d.nsrc * 250.0 /
+                      (kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0));
+  d.cells_cap = (int)std::min<double>(kMaxCells, 2 * kGroup + kDyadic + most) & ~(kGroup - 1);
+  const long long ntile = (long long)p.nsets * d.ft;
+  long long cells = ntile * d.cells_cap;
+  if (batch) {
+    // as much as the direct kernels' interval data, and 64 MiB
+    const long long direct = (long long)p.total * p.nf * 16 / ((long long)kBlockFloats * 4);
+    cells = std::min(cells, direct + (64ll << 20) / (kBlockFloats * 4));
+  }
+  cells &= ~(long long)(kGroup - 1);
+  d.blocks_cap = cells;
+  d.units_cap = (long long)d.nacc * d.mtiles * (cells / d.run + ntile);
+  d.slots = p.total / d.chunk + p.nsets + 1;
+  size_t at = 0;
+  auto place = [&](size_t bytes) {
+    const size_t o = at;
+    at += round256(bytes);
+    return static_cast<char*>(base) + o;
+  };
+  d.use = reinterpret_cast<unsigned char*>(place((size_t)p.nsets * p.nf));
+  d.plan = reinterpret_cast<XpPlan*>(place(sizeof(XpPlan)));
+  d.tile = reinterpret_cast<XpTile*>(place(sizeof(XpTile) * ntile));
+  d.bad = reinterpret_cast<int*>(place(sizeof(int) * ntile));
+  const int nbasis = d.nsrc;
+  d.E = reinterpret_cast<float*>(place(sizeof(float) * (size_t)nbasis * d.cells_cap * kNodes * d.ncp));
+  d.W = reinterpret_cast<float*>(place(sizeof(float) * (size_t)cells * nin * kBlockFloats));
+  if (d.has_ends) {
+    d.Eend = reinterpret_cast<float*>(
+        place(sizeof(float) * (size_t)nbasis * d.cells_cap * kEndRows * d.ncp));
+    d.V = reinterpret_cast<float*>(place(sizeof(float) * (size_t)cells * nin * kEndFloats));
+    d.ends = reinterpret_cast<unsigned char*>(place((size_t)(cells / kGroup)));
+  }
+  d.part = reinterpret_cast<float*>(
+      place(sizeof(float) * (size_t)d.units_cap * kTileRows * kTileCols));
+  const size_t edge = sizeof(float) * (size_t)d.slots * p.nf * nin * kNodes;
+  d.head = reinterpret_cast<float*>(place(edge));
+  d.tail = reinterpret_cast<float*>(place(edge));
+  d.span = reinterpret_cast<int2*>(place(sizeof(int2) * (size_t)d.slots * p.nf));
+  *out = d;
+  return at;
+}
+
+template <int MODE, int ITYPE>
+int plan_mode(const XpDev& d, cudaStream_t s) {
+  xp_columns_kernel<MODE, ITYPE><<<dim3(d.ft, d.nsets), 64, 0, s>>>(d);
+  count_launch();
+  CCFJ_LAUNCH_CHECK("xp_columns_kernel");
+  xp_scan_kernel<<<1, 1024, 0, s>>>(d);
+  count_launch();
+  CCFJ_LAUNCH_CHECK("xp_scan_kernel");
+  return CCFJ_OK;
+}
+
+template <int MODE, int ITYPE>
+int run_mode(const XpDev& d, cudaStream_t s) {
+  using MT = ModeTraits<MODE>;
+  constexpr int NIN = MT::NIN;
+  constexpr bool DY = MT::WY;
+  constexpr int NSRC = MT::WJ && MT::WY ? 2 : 1;
+  int dev = 0, sms = 148;
+  CCFJ_CUDA_TRY(cudaGetDevice(&dev));
+  CCFJ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (ITYPE == 1)
+    CCFJ_CUDA_TRY(cudaMemsetAsync(d.ends, 0, (size_t)(d.blocks_cap / kGroup), s));
+  prof_begin(s);
+  const int by = std::max(1, std::min(d.cells_cap, 16 * sms / d.mtiles));
+  xp_basis_kernel<MODE, ITYPE><<<dim3(d.mtiles, by), kTileRows, 0, s>>>(d);
+  count_launch();
+  CCFJ_LAUNCH_CHECK("xp_basis_kernel");
+  const int ftiles = (int)div_up(d.nf, 32);
+  const long long warps = d.slots * ftiles;
+  xp_moments_kernel<NIN, ITYPE, DY><<<(unsigned)warps, 32, 0, s>>>(d, ftiles);
+  count_launch();
+  CCFJ_LAUNCH_CHECK("xp_moments_kernel");
+  xp_join_kernel<NIN, ITYPE, DY>
+      <<<dim3((unsigned)d.slots, div_up(d.nf, 64)), 256, 0, s>>>(d);
+  count_launch();
+  CCFJ_LAUNCH_CHECK("xp_join_kernel");
+  const int grid = (int)std::min<long long>(d.units_cap, 3ll * sms);
+  xp_gemm_kernel<NSRC><<<grid, kGemmThreads, 0, s>>>(d);
+  count_launch();
+  CCFJ_LAUNCH_CHECK("xp_gemm_kernel");
+  prof_end(s);
+  xp_finish_kernel<MODE, ITYPE><<<dim3(div_up(d.nf, 16), d.nsets), dim3(16, kFinRows), 0, s>>>(d);
+  count_launch();
+  CCFJ_LAUNCH_CHECK("xp_finish_kernel");
+  return CCFJ_OK;
+}
+
+template <int ITYPE>
+int dispatch(const XpDev& d, int mode, bool plan, cudaStream_t s) {
+  switch (mode) {
+#define CCFJ_XP(M) \
+  case M:          \
+    return plan ? plan_mode<M, ITYPE>(d, s) : run_mode<M, ITYPE>(d, s)
+    CCFJ_XP(CCFJ_MODE_J);
+    CCFJ_XP(CCFJ_MODE_Y);
+    CCFJ_XP(CCFJ_MODE_J_MINUS_Y);
+    CCFJ_XP(CCFJ_MODE_ABS_J);
+    CCFJ_XP(CCFJ_MODE_ABS_H);
+#undef CCFJ_XP
+  }
+  return set_error(CCFJ_ERR_INVALID, "bad mode %d", mode);
+}
+
+}  // namespace
+
+bool xp_eligible(int mode, int itype, long long total, int nsets, int nf_all, int nc) {
+  (void)mode;
+  (void)itype;
+  // below this the direct kernels finish before the expansion's launches do
+  return total >= 2ll * nsets && nsets <= 65535 && nf_all <= 65535 * 16 &&
+         (double)total * nf_all * nc >= 6e6;
+}
+
+int xp_plan(const XpProblem& p, Scratch& sc, cudaStream_t s, XpWork* w, bool* ok) {
+  XpDev d;
+  *ok = false;
+  const size_t bytes = layout(p, nullptr, &d);
+  if (d.slots > 0x7fffffffll || d.slots * div_up(p.nf, 32) > 0x7fffffffll) return CCFJ_OK;
+  void* base = sc.get(bytes);
+  if (!base) {
+    clear_error();
+    return CCFJ_OK;
+  }
+  layout(p, base, &d);
+  w->base = base;
+  w->use = d.use;
+  *ok = true;
+  return p.itype == 1 ? dispatch<1>(d, p.mode, true, s) : dispatch<0>(d, p.mode, true, s);
+}
+
+int xp_run(const XpProblem& p, const XpWork& w, cudaStream_t s) {
+  XpDev d;
+  layout(p, w.base, &d);
+  return p.itype == 1 ? dispatch<1>(d, p.mode, false, s) : dispatch<0>(d, p.mode, false, s);
+}
+
+}  // namespace ccfj

@@ -1,0 +1,47 @@
+// Wave-cell expansion of the FP32 transform (fj_expand.cu): host interface.
+#pragma once
+
+#include "ccfj_core.cuh"
+#include "fj_frontend.cuh"
+
+namespace ccfj {
+
+// One transform, or a batch of sets that share f and c, as the expansion
+// reads it (every pointer is device memory).
+struct XpProblem {
+  const float* rs;       // [total] distances, ascending within each set
+  const float* wtr;      // [total] trapezoid weights (itype 0)
+  const long long* off;  // [nsets + 1], or NULL for one set of `total` pairs
+  int nsets;
+  long long total;
+  int nf, nc;
+  const float* f;
+  const float* c;
+  int itype, mode;
+  InDesc in[2];
+  float* out;  // [nsets][nc][nf]
+  int normalize;
+  // frequencies and pairs of the whole problem that this one is a window or
+  // a group of sets of
+  int nf_all;
+  long long total_all;
+};
+
+// What the host sized and where it lies in the call's scratch.
+struct XpWork {
+  unsigned char* use;  // [nsets][nf] 1: the expansion computes the column
+  void* base;
+};
+
+// Whether a problem of these sizes runs the expansion at all. Decided from
+// the sizes of the whole problem alone, so that frequency windows and blocks
+// of one problem decide alike.
+bool xp_eligible(int mode, int itype, long long total, int nsets, int nf_all, int nc);
+// Reserves the scratch and runs the plan (which columns take the expansion).
+// ok = false (and no error) where the memory cannot be had: the caller then
+// computes every column directly.
+int xp_plan(const XpProblem& p, Scratch& sc, cudaStream_t s, XpWork* w, bool* ok);
+// Computes the columns the plan chose, normalised if asked.
+int xp_run(const XpProblem& p, const XpWork& w, cudaStream_t s);
+
+}  // namespace ccfj

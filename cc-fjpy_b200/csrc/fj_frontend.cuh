@@ -24,10 +24,19 @@ bool hilbert_fft_supported(int n);
 int hilbert_rows_fft(const InDesc& in, int n, int es, int nr, int nf, int fstride, int col_begin,
                      float* dst, cudaStream_t s, Scratch& sc);
 
-// Device-resident transform (all pointers in args are device pointers);
-// cpt > 0 forces that variant of the FP32 kernel (velocities per thread),
-// nsplit > 0 that many station ranges (split launch, fixed-order sum).
-int fj_device(const ccfj_fj_args& a, cudaStream_t s, int cpt = 0, int nsplit = 0);
+// How a transform runs: cpt > 0 forces that variant of the FP32 direct
+// kernel (velocities per thread), nsplit > 0 that many station ranges (split
+// launch, fixed-order sum). path: -1 decides by sizes and settings whether
+// the wave-cell expansion may take columns (fj_expand.cu), 0 keeps it off, 1
+// allows it, with nf_all the frequencies of the whole problem that this one
+// is a block of.
+struct FjChoice {
+  int cpt = 0, nsplit = 0;
+  int path = -1;
+  int nf_all = 0;
+};
+// Device-resident transform (all pointers in args are device pointers).
+int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice = FjChoice());
 // The argument checks of ccfj_fj_v1 (status and message as it returns them).
 int fj_validate(const ccfj_fj_args* a);
 

@@ -33,6 +33,7 @@
 
 #include "ccfj_core.cuh"
 #include "fj_cells.cuh"
+#include "fj_expand.cuh"
 #include "fj_frontend.cuh"
 #include "fj_interval.cuh"
 
@@ -81,10 +82,11 @@ __global__ void __launch_bounds__(256, fj_min_blocks<T>()) fj_amortized_kernel(F
 template <int MODE>
 __global__ void fj_split_finish_kernel(const float* __restrict__ part, int nsplit,
                                        const float* __restrict__ f, const float* __restrict__ c,
-                                       int nc, int nf, float* __restrict__ out) {
+                                       int nc, int nf, float* __restrict__ out,
+                                       const unsigned char* __restrict__ use) {
   const int fi = blockIdx.x * 32 + threadIdx.x;
   const int ci = blockIdx.y * 8 + threadIdx.y;
-  if (fi >= nf || ci >= nc) return;
+  if (fi >= nf || ci >= nc || (use && use[fi])) return;
   constexpr int NACC = ModeTraits<MODE>::NACC;
   const long long plane = (long long)nc * nf, at = (long long)ci * nf + fi;
   float tot[2] = {0.f, 0.f};
@@ -183,10 +185,16 @@ __global__ void fj_gather_kernel(InDesc in, int nr, int nf, float* __restrict__ 
 // (src/ccfj-gpu.pyx:266-267): the running maximum starts at row 0 and is
 // replaced only by a strictly larger value, so a NaN in row 0 makes the
 // column NaN while NaNs in later rows are skipped.
-__global__ void fj_normalize_kernel(float* __restrict__ out, int nc, int nf) {
+// Columns marked in `use` are finished elsewhere.
+__global__ void fj_normalize_kernel(float* __restrict__ out, int nc, int nf,
+                                    const unsigned char* __restrict__ use) {
   __shared__ float red[8][33];
   __shared__ float colmax[32];
-  const int fi = blockIdx.x * 32 + threadIdx.x;
+  int fi = blockIdx.x * 32 + threadIdx.x;
+  if (use) {
+    if (fi < nf && use[fi]) fi = nf;
+    if (!__syncthreads_or(fi < nf)) return;
+  }
   float m = -INFINITY;
   if (fi < nf)
     for (int c = threadIdx.y; c < nc; c += blockDim.y) m = fmaxf(m, fabsf(out[(long long)c * nf + fi]));
@@ -361,41 +369,42 @@ size_t interval_data_bytes(const ccfj_fj_args& a) {
 // sizes above; d.rs, d.drs, d.geo (itype 1), d.nr, d.nf, d.tau must be set.
 int prep_interval_data(const ccfj_fj_args& a, FjDev& d, const InDesc* in, int nin, void* kb,
                        void* const* gbuf, const float* wtr, cudaStream_t s) {
+  const unsigned char* use = d.use;
   const bool fp32 = a.precision == CCFJ_PREC_FP32;
   if (a.itype == 1) {
     const dim3 kbb(32, 8);
     if (fp32)
       fj_kbounds_kernel<float><<<div_up(a.nf, 8), kbb, 0, s>>>(a.f, a.c, a.nf, a.nc, d.tau,
-                                                               static_cast<float*>(kb));
+                                                               static_cast<float*>(kb), use);
     else
       fj_kbounds_kernel<double><<<div_up(a.nf, 8), kbb, 0, s>>>(a.f, a.c, a.nf, a.nc,
                                                                 (double)d.tau,
-                                                                static_cast<double*>(kb));
+                                                                static_cast<double*>(kb), use);
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_kbounds_kernel");
     d.kb = kb;
   }
-  const dim3 pb(32, 8), pg(div_up(a.nr, 8), div_up(a.nf, 32));
+  const dim3 pb(32, 8), pg(prep_rows(a.nr), div_up(a.nf, 32));
   for (int j = 0; j < nin; ++j) {
     void* g = gbuf[j];
     if (a.itype == 1) {
       if (fp32)
         fj_prep_coef_kernel<float><<<pg, pb, 0, s>>>(in[j], a.nr, a.nf, d.rs, d.drs, d.geo,
                                                      static_cast<const float*>(kb),
-                                                     static_cast<StationCoef<float>*>(g));
+                                                     static_cast<StationCoef<float>*>(g), use);
       else
         fj_prep_coef_kernel<double><<<pg, pb, 0, s>>>(in[j], a.nr, a.nf, d.rs, d.drs, d.geo,
                                                       static_cast<const double*>(kb),
-                                                      static_cast<StationCoef<double>*>(g));
+                                                      static_cast<StationCoef<double>*>(g), use);
       count_launch();
       CCFJ_LAUNCH_CHECK("fj_prep_coef_kernel");
     } else {
       if (fp32)
         fj_prep_u_kernel<float><<<pg, pb, 0, s>>>(in[j], a.nr, a.nf, wtr, d.geo,
-                                                  static_cast<float*>(g));
+                                                  static_cast<float*>(g), use);
       else
         fj_prep_u_kernel<double><<<pg, pb, 0, s>>>(in[j], a.nr, a.nf, wtr, d.geo,
-                                                   static_cast<double*>(g));
+                                                   static_cast<double*>(g), use);
       count_launch();
       CCFJ_LAUNCH_CHECK("fj_prep_u_kernel");
     }
@@ -404,10 +413,22 @@ int prep_interval_data(const ccfj_fj_args& a, FjDev& d, const InDesc* in, int ni
   return CCFJ_OK;
 }
 
+// Whether the wave-cell expansion may take columns of a transform: not with
+// a forced variant, split or switch point of the direct kernels, whose
+// meaning it would take away. Decided for the whole problem (nf_total), so
+// that its frequency windows and blocks decide alike.
+static bool expansion_allowed(const ccfj_fj_args& a) {
+  return a.precision == CCFJ_PREC_FP32 && !(a.tau > 0) &&
+         g_force_cpt.load(std::memory_order_relaxed) == 0 &&
+         g_force_split.load(std::memory_order_relaxed) == 0 &&
+         xp_eligible(a.mode, a.itype, a.nr, 1, a.nf_total > 0 ? a.nf_total : a.nf, a.nc);
+}
+
 // Device-resident transform: every pointer in `a` is a device pointer.
-// cpt > 0 runs that variant (velocities per thread) of the FP32 kernel.
-int fj_device(const ccfj_fj_args& a, cudaStream_t s, int cpt_choice, int split_choice) {
+int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
   const int nin = nin_of(a.mode);
+  const int cpt_choice = choice.cpt, split_choice = choice.nsplit;
+  const bool expand = choice.path < 0 ? expansion_allowed(a) : choice.path == 1;
   Scratch sc(s);
   float* drs = sc.get_n<float>(a.nr + 1);
   float* wtr = sc.get_n<float>(a.nr);
@@ -445,6 +466,32 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, int cpt_choice, int split_c
                                 a.nf, a.fstride, a.col_begin, hb, s, sc);
     if (st != CCFJ_OK) return st;
     in[1] = InDesc{hb, a.nf, 1, nullptr};
+  }
+
+  // the expansion plans which columns it takes; the direct kernels below
+  // compute the others
+  XpProblem xp{};
+  XpWork xw{};
+  bool expanded = false;
+  if (expand) {
+    xp.rs = a.r;
+    xp.wtr = wtr;
+    xp.nsets = 1;
+    xp.total = xp.total_all = a.nr;
+    xp.nf = a.nf;
+    xp.nc = a.nc;
+    xp.f = a.f;
+    xp.c = a.c;
+    xp.itype = a.itype;
+    xp.mode = a.mode;
+    xp.in[0] = in[0];
+    xp.in[1] = in[1];
+    xp.out = a.out;
+    xp.normalize = a.normalize;
+    xp.nf_all = choice.nf_all > 0 ? choice.nf_all : a.nf_total > 0 ? a.nf_total : a.nf;
+    const int st = xp_plan(xp, sc, s, &xw, &expanded);
+    if (st != CCFJ_OK) return st;
+    if (expanded) d.use = xw.use;
   }
 
   const float* plain[2] = {nullptr, nullptr};
@@ -485,7 +532,7 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, int cpt_choice, int split_c
       }
     }
   }
-  prof_begin(s);
+  if (!expanded) prof_begin(s);
   switch (a.mode) {
     case CCFJ_MODE_J:
       launch_mode<CCFJ_MODE_J>(a.precision, a.itype, d, plain[0], plain[1], cpt, s);
@@ -503,7 +550,7 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, int cpt_choice, int split_c
       launch_mode<CCFJ_MODE_ABS_H>(a.precision, a.itype, d, plain[0], plain[1], cpt, s);
       break;
   }
-  prof_end(s);
+  if (!expanded) prof_end(s);
   count_launch();
   CCFJ_LAUNCH_CHECK("fj transform kernel");
   if (d.part) {
@@ -511,22 +558,22 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, int cpt_choice, int split_c
     const dim3 fg(div_up(a.nf, 32), div_up(a.nc, 8)), fb(32, 8);
     switch (a.mode) {
       case CCFJ_MODE_J:
-        fj_split_finish_kernel<CCFJ_MODE_J><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out);
+        fj_split_finish_kernel<CCFJ_MODE_J><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out, d.use);
         break;
       case CCFJ_MODE_Y:
-        fj_split_finish_kernel<CCFJ_MODE_Y><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out);
+        fj_split_finish_kernel<CCFJ_MODE_Y><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out, d.use);
         break;
       case CCFJ_MODE_J_MINUS_Y:
         fj_split_finish_kernel<CCFJ_MODE_J_MINUS_Y><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc,
-                                                                     a.nf, a.out);
+                                                                     a.nf, a.out, d.use);
         break;
       case CCFJ_MODE_ABS_J:
         fj_split_finish_kernel<CCFJ_MODE_ABS_J><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf,
-                                                                 a.out);
+                                                                 a.out, d.use);
         break;
       default:
         fj_split_finish_kernel<CCFJ_MODE_ABS_H><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf,
-                                                                 a.out);
+                                                                 a.out, d.use);
         break;
     }
     count_launch();
@@ -534,11 +581,11 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, int cpt_choice, int split_c
   }
 
   if (a.normalize) {
-    fj_normalize_kernel<<<div_up(a.nf, 32), dim3(32, 8), 0, s>>>(a.out, a.nc, a.nf);
+    fj_normalize_kernel<<<div_up(a.nf, 32), dim3(32, 8), 0, s>>>(a.out, a.nc, a.nf, d.use);
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_normalize_kernel");
   }
-  return CCFJ_OK;
+  return expanded ? xp_run(xp, xw, s) : CCFJ_OK;
 }
 
 static int validate(const ccfj_fj_args* a) {
@@ -667,6 +714,11 @@ static int fj_host_blocks(const ccfj_fj_args& a, cudaStream_t s, int nblk, int n
   cudaStream_t hs[2] = {hp->st[0], hp->st[1]};
   const int full_cpt = variant_for(a, 0);
   const int full_split = a.precision == CCFJ_PREC_FP32 ? split_for(a, full_cpt, 0) : 1;
+  FjChoice block;
+  block.cpt = full_cpt;
+  block.nsplit = full_split;
+  block.path = expansion_allowed(a) ? 1 : 0;
+  block.nf_all = a.nf_total > 0 ? a.nf_total : a.nf;
   Scratch sc(s);
   float* dr = sc.get_n<float>(a.nr);
   float* df = sc.get_n<float>(a.nf);
@@ -806,7 +858,7 @@ static int fj_host_blocks(const ccfj_fj_args& a, cudaStream_t s, int nblk, int n
     d.out = B.dout;
     // every block runs the whole problem's tile choice, so the blocks give
     // the device path's result bit for bit
-    st = fj_device(d, cs, full_cpt, full_split);
+    st = fj_device(d, cs, block);
     if (st != CCFJ_OK) return fail(st);
   }
   for (int p = 0; p < nblk; ++p) {
@@ -973,9 +1025,13 @@ CCFJ_API int ccfj_autotune_fj_v1(const ccfj_fj_args* args, void* stream, int* be
     for (int n : splits) {
       if (n > 1 && (n * ctas > 2 * slots || args->nr < 2 * 32 * n)) continue;
       float t = 1e30f;
+      ccfj::FjChoice cand;  // the direct kernels alone
+      cand.cpt = c;
+      cand.nsplit = n;
+      cand.path = 0;
       for (int rep = 0; rep < 3 && st == CCFJ_OK; ++rep) {
         cudaEventRecord(e0, s);
-        st = ccfj::fj_device(*args, s, c, n);
+        st = ccfj::fj_device(*args, s, cand);
         cudaEventRecord(e1, s);
         if (cudaEventSynchronize(e1) != cudaSuccess) st = CCFJ_ERR_CUDA;
         float ms = 0;
@@ -1161,7 +1217,7 @@ static int fj_noalloc(const ccfj_fj_args& a, cudaStream_t s) {
   count_launch();
   CCFJ_LAUNCH_CHECK("fj transform kernel");
   if (a.normalize) {
-    fj_normalize_kernel<<<div_up(a.nf, 32), dim3(32, 8), 0, s>>>(a.out, a.nc, a.nf);
+    fj_normalize_kernel<<<div_up(a.nf, 32), dim3(32, 8), 0, s>>>(a.out, a.nc, a.nf, nullptr);
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_normalize_kernel");
   }
