@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "ccfj_core.cuh"
+#include "fj_expand.cuh"
 #include "fj_fft.cuh"
 #include "fj_frontend.cuh"
 
@@ -213,7 +214,11 @@ CCFJ_API int ccfj_device_status(void* stream) {
   bool failed = false;
   const int st = ccfj::mw_tc_sticky_error((cudaStream_t)stream, &failed);
   if (st != CCFJ_OK) return st;
-  if (failed) return ccfj::set_error(CCFJ_ERR_TIMEOUT, "a bounded device wait ran out");
+  bool xp_failed = false;
+  const int xst = ccfj::xp_sticky_error((cudaStream_t)stream, &xp_failed);
+  if (xst != CCFJ_OK) return xst;
+  if (failed || xp_failed)
+    return ccfj::set_error(CCFJ_ERR_TIMEOUT, "a bounded device wait ran out");
   return CCFJ_OK;
 }
 

@@ -44,19 +44,19 @@
 //
 // Kernels of a call, in order:
 //   xp_columns_kernel  which columns take the expansion, cell range per tile
-//                      of 64 frequencies; checks that r ascends
+//                      of 128 frequencies; checks that r ascends
 //   xp_scan_kernel     where each tile's W blocks and GEMM units begin
 //   xp_basis_kernel    E
 //   xp_moments_kernel  W, in chunks of stations; the cells that a chunk
 //                      shares with its neighbours go to head / tail parts
 //   xp_join_kernel     adds those parts in chunk order
-//   xp_gemm_kernel     the product, in units of (128 velocities x 64 columns x
-//                      a run of cells)
+//   xp_gemm_kernel     the product on the tensor cores, in units of (128
+//                      velocities x 128 columns x a run of cells)
 //   xp_finish_kernel   adds a column's units in order, |.| and normalisation
 //
 // Measured against the direct kernels on one B200 (device-resident call):
-// 19,900 pairs x 2048 f x 1000 c 61.3 -> 1.71 ms, 200 x 512 x 300 0.215 ->
-// 0.099 ms, 128 subarrays of 50-20,000 pairs (512 f x 500 c) 188 -> 6.2 ms; the
+// 19,900 pairs x 2048 f x 1000 c 61.3 -> 1.07 ms, 200 x 512 x 300 0.215 ->
+// 0.089 ms, 128 subarrays of 50-20,000 pairs (512 f x 500 c) 196 -> 4.3 ms; the
 // error against 64-bit quadrature 1.1e-6 -> 2e-7 of the spectrum (2-norm).
 //
 // Every sum is in an order fixed by the sizes, so results do not depend on
@@ -66,6 +66,7 @@
 
 #include "fj_cells.cuh"
 #include "fj_expand.cuh"
+#include "fj_tcgen05.cuh"
 
 namespace ccfj {
 
@@ -77,11 +78,11 @@ constexpr double kCellPhase = 9.8;  // radians of a cell at the slowest velocity
 // Columns with more go to the direct kernels.
 constexpr int kMaxCells = 2048;
 constexpr int kDyadic = 24;         // halved cells below the first (Y basis)
-constexpr int kTileCols = 64;       // frequencies of a W tile and GEMM column tile
+constexpr int kTileCols = 128;      // frequencies of a W tile and GEMM column tile
 constexpr int kTileRows = 128;      // velocities of a GEMM tile
 constexpr int kGroup = 4;           // tiles begin and end with groups of cells
 constexpr int kEndRows = 2;         // rows of a cell's end
-constexpr int kEndFloats = kTileCols * kEndRows;  // one (tile, cell, input) of V
+constexpr int kEndFloats = kTileCols * kGroup * kEndRows;  // one (tile, group, input) of V
 constexpr int kBlockFloats = kTileCols * kNodes;  // one (tile, cell, input) of W
 // Intervals up to this share of a cell are short: whole in the cell of their
 // far end. A cell's polynomials live on [-kShort, 1] of it; the middle of that
@@ -89,7 +90,6 @@ constexpr int kBlockFloats = kTileCols * kNodes;  // one (tile, cell, input) of 
 constexpr float kShort = 0.0625f;
 constexpr float kCentre = 0.46875f;
 constexpr float kPerHalf = 1.8823529f;
-constexpr int kGemmThreads = 128;
 
 struct XpTile {
   int lo, hi;    // cells [lo, hi) of the tile's columns, whole groups
@@ -127,12 +127,13 @@ struct XpDev {
   XpPlan* plan;
   XpTile* tile;
   int* bad;              // [nsets * ft] the tile's part of r is out of order
-  float* E;              // [basis][cell][16][ncp]
-  float* Eend;           // [basis][cell][2][ncp]
-  float* W;              // [block][input][64][16]
-  float* V;              // [block][input][64][2]
+  float* E;              // [basis][cell][velocity tile][128][16]
+  float* Eend;           // [basis][group][velocity tile][128][cell of the group][2]
+  float* W;              // [block][input][128][16]
+  float* V;              // [group][input][128][cell of the group][2]
+  int* unit_tile;        // [unit]
   unsigned char* ends;   // [group] some column has weights in V
-  float* part;           // [unit][128][64]
+  float* part;           // [unit][128][128]
   float* head;           // [slot][nf][input][16]
   float* tail;
   int2* span;            // [slot][nf] first and last cell of a chunk
@@ -188,40 +189,38 @@ __device__ __forceinline__ float cell_begin(int cell) {
 }
 
 // ------------------------------------------------------------------- plan
-// One CTA of 64 threads per (set, 64 frequencies).
+// One CTA of 128 threads per (set, 128 frequencies).
 template <int MODE, int ITYPE>
 __global__ void xp_columns_kernel(XpDev d) {
   constexpr bool DY = ModeTraits<MODE>::WY;
-  __shared__ float red[2][2];
-  __shared__ int ired[2][3];
+  constexpr int kWarps = kTileCols / 32;
+  __shared__ float red[kWarps];
+  __shared__ int ired[kWarps][3];
   const int t = threadIdx.x, b = blockIdx.y;
-  float lo = INFINITY, hi = -INFINITY;
+  float lo = INFINITY;  // the slowest velocity
   bool fine = true;
-  for (int j = t; j < d.nc; j += 64) {
+  for (int j = t; j < d.nc; j += kTileCols) {
     const float v = d.c[j];
     fine = fine && v > 0.0f && v < INFINITY;
     lo = fminf(lo, v);
-    hi = fmaxf(hi, v);
   }
   // this tile's share of the set's distances: finite and ascending
   const long long o = set_begin(d, b), n = set_end(d, b) - o;
-  for (long long i = blockIdx.x * 64 + t; i < n; i += (long long)d.ft * 64) {
+  for (long long i = blockIdx.x * kTileCols + t; i < n; i += (long long)d.ft * kTileCols) {
     const float v = d.rs[o + i];
     fine = fine && v >= 0.0f && v < INFINITY && (i == 0 || v >= d.rs[o + i - 1]);
   }
-  for (int s = 16; s > 0; s >>= 1) {
-    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, s));
-    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, s));
-  }
+  for (int s = 16; s > 0; s >>= 1) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, s));
   fine = __all_sync(0xffffffffu, fine);
   if ((t & 31) == 0) {
-    red[0][t >> 5] = lo;
-    red[1][t >> 5] = hi;
+    red[t >> 5] = lo;
     ired[t >> 5][2] = fine;
   }
   __syncthreads();
-  lo = fminf(red[0][0], red[0][1]);
-  fine = ired[0][2] && ired[1][2];
+  for (int w = 0; w < kWarps; ++w) {
+    lo = fminf(lo, red[w]);
+    fine = fine && ired[w][2];
+  }
   const double hu = kCellPhase / fjs::kTwoPi * (double)lo, inv_hu = 1.0 / hu;
   const int tile = b * d.ft + blockIdx.x;
   if (t == 0) d.bad[tile] = !fine;
@@ -229,7 +228,7 @@ __global__ void xp_columns_kernel(XpDev d) {
     d.plan->hu = hu;
     d.plan->inv_hu = inv_hu;
   }
-  const int fi = blockIdx.x * 64 + t;
+  const int fi = blockIdx.x * kTileCols + t;
   int first = 0, last = 0;
   bool use = false;
   if (fine && fi < d.nf && n > 0) {
@@ -270,8 +269,10 @@ __global__ void xp_columns_kernel(XpDev d) {
   }
   __syncthreads();
   if (t == 0) {
-    mn = min(ired[0][0], ired[1][0]);
-    mx = max(ired[0][1], ired[1][1]);
+    for (int w = 0; w < kWarps; ++w) {
+      mn = min(mn, ired[w][0]);
+      mx = max(mx, ired[w][1]);
+    }
     if (mx <= mn) mn = mx = 0;
     d.tile[tile].lo = mn & ~(kGroup - 1);
     d.tile[tile].hi = (mx + kGroup - 1) & ~(kGroup - 1);
@@ -350,7 +351,14 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
     d.plan->lo = ok && hi > lo ? lo : 0;
     d.plan->hi = ok && hi > lo ? hi : 0;
   }
-  if (!ok) {
+  __syncthreads();
+  if (ok) {
+    for (int i = t; i < ntile; i += 1024) {
+      const int runs = (d.tile[i].hi - d.tile[i].lo + d.run - 1) / d.run;
+      int* u = d.unit_tile + d.tile[i].unit;
+      for (int k = 0; k < d.nacc * d.mtiles * runs; ++k) u[k] = i;
+    }
+  } else {
     const long long ncol = (long long)d.nsets * d.nf;
     for (long long i = t; i < ncol; i += 1024) d.use[i] = 0;
   }
@@ -399,11 +407,15 @@ __global__ void __launch_bounds__(kTileRows) xp_basis_kernel(XpDev d) {
       }
     }
     const long long plane = (long long)d.cells_cap * kNodes * d.ncp;
-    float* e = d.E + (long long)cell * kNodes * d.ncp + j;
+    float4* e = reinterpret_cast<float4*>(
+        d.E + (((long long)cell * d.mtiles + blockIdx.x) * kTileRows + t) * kNodes);
 #pragma unroll
-    for (int n = 0; n < kNodes; ++n) {
-      if (MT::WJ) e[(long long)n * d.ncp] = (float)eJ[n];
-      if (MT::WY) e[(MT::WJ ? plane : 0) + (long long)n * d.ncp] = (float)eY[n];
+    for (int n = 0; n < kNodes; n += 4) {
+      if (MT::WJ)
+        e[n / 4] = make_float4((float)eJ[n], (float)eJ[n + 1], (float)eJ[n + 2], (float)eJ[n + 3]);
+      if (MT::WY)
+        e[(MT::WJ ? plane / 4 : 0) + n / 4] =
+            make_float4((float)eY[n], (float)eY[n + 1], (float)eY[n + 2], (float)eY[n + 3]);
     }
     if (ITYPE == 1) {
       // the cell's end, with r in cells and k = 2 pi per_c
@@ -418,15 +430,13 @@ __global__ void __launch_bounds__(kTileRows) xp_basis_kernel(XpDev d) {
         r2Y = (x * Y.z0 - Y.b * ik) * ik * ik;
       }
       const long long eplane = (long long)d.cells_cap * kEndRows * d.ncp;
-      float* v = d.Eend + (long long)cell * kEndRows * d.ncp + j;
-      if (MT::WJ) {
-        v[0] = (float)r1;
-        v[d.ncp] = (float)r2J;
-      }
-      if (MT::WY) {
-        v[MT::WJ ? eplane : 0] = (float)r1Y;
-        v[(MT::WJ ? eplane : 0) + d.ncp] = (float)r2Y;
-      }
+      float* v = d.Eend +
+                 (((long long)(cell / kGroup) * d.mtiles + blockIdx.x) * kTileRows + t) *
+                     (kGroup * kEndRows) +
+                 (cell & (kGroup - 1)) * kEndRows;
+      if (MT::WJ) *reinterpret_cast<float2*>(v) = make_float2((float)r1, (float)r2J);
+      if (MT::WY)
+        *reinterpret_cast<float2*>(v + (MT::WJ ? eplane : 0)) = make_float2((float)r1Y, (float)r2Y);
     }
   }
 }
@@ -562,9 +572,7 @@ __global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
   float base_x = cell_begin<DY>(cell);
   const long long edge = ((slot * d.nf + fc) * NIN) * kNodes;
   float* W = d.W + (tile.w + cell - tile.lo) * NIN * kBlockFloats + (fc & (kTileCols - 1)) * kNodes;
-  float* V = ITYPE == 1 ? d.V + (tile.w + cell - tile.lo) * NIN * kEndFloats +
-                              (fc & (kTileCols - 1)) * kEndRows
-                        : nullptr;
+  float* const V = d.V + (tile.w / kGroup) * NIN * kEndFloats + (fc & (kTileCols - 1)) * kGroup * kEndRows;
   auto store = [&](float* base, long long step) {
     if (more) {
 #pragma unroll
@@ -592,11 +600,12 @@ __global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
     const bool first = cell == cell0;
     store(first ? d.head + edge : W, first ? kNodes : kBlockFloats);
     if (ITYPE == 1) {
+      const int at = cell - tile.lo;
+      float* v = V + (long long)(at / kGroup) * (NIN * kEndFloats) + (at & (kGroup - 1)) * kEndRows;
 #pragma unroll
       for (int k = 0; k < NIN; ++k)
-        *reinterpret_cast<float2*>(V + k * kEndFloats) = make_float2(vx[k], vy[k]);
-      if (ends) d.ends[(tile.w + cell - tile.lo) / kGroup] = 1;
-      V += NIN * kEndFloats;
+        *reinterpret_cast<float2*>(v + k * kEndFloats) = make_float2(vx[k], vy[k]);
+      if (ends) d.ends[(tile.w + at) / kGroup] = 1;
     }
     W += NIN * kBlockFloats;
     ++cell;
@@ -803,7 +812,9 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   auto clear_end = [&](int cell) {
     if (ITYPE == 0 || n4 != 0) return;
-    float* p = d.V + (tile.w + cell - tile.lo) * NIN * kEndFloats + (fi & (kTileCols - 1)) * kEndRows;
+    const long long blk = tile.w + cell - tile.lo;
+    float* p = d.V + (blk / kGroup) * NIN * kEndFloats +
+               ((fi & (kTileCols - 1)) * kGroup + (blk & (kGroup - 1))) * kEndRows;
 #pragma unroll
     for (int k = 0; k < NIN; ++k) *reinterpret_cast<float2*>(p + k * kEndFloats) = make_float2(0.f, 0.f);
   };
@@ -856,185 +867,377 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
 }
 
 // ------------------------------------------------------------------- GEMM
-// Units of 128 velocities x 64 columns x up to `run` cells; a thread holds
-// 8 x 8 results. Per cell (16 terms) the E rows come in by cp.async and the W
-// block, which lies column by column, through registers, transposed.
-struct GemmStage {
-  float e[kNodes][kTileRows];
-  float w[kNodes][kTileCols + 4];
+// Units of 128 velocities x 128 columns x up to `run` cells on the tensor
+// cores, kind::tf32. An FP32 operand x is split into hi (its 11 leading bits,
+// rounded) and lo = x - hi, which keep 22 of its 24 bits and all of its range
+// (no scales, as a split into fp16 halves would need), and the product is
+// hi hi + hi lo + lo hi with FP32 accumulation. The tensor core truncates each
+// sum, so hi hi is taken out of tensor memory after every group of four cells
+// (8 steps) and added in FP32 registers; the two small products, 2^-11 of it,
+// have an accumulator of their own that is read once, at the unit's end.
+//
+// One persistent CTA per SM, by warps: 8 that drain tensor memory (each 32
+// rows x 64 columns of the totals), 8 that bring the operands in (global to
+// registers, split, to shared memory as 8 x 16 byte core matrices), one that
+// issues the MMAs. Four stages of one step each: a cell (K = 16) or a group's
+// end rows (K = 8). Bound by shared memory: a step's MMAs read 48 KB of it and
+// the loaders store 32 KB. 19,900 pairs x 2048 f x 1000 c: 322 us, 884 us with
+// FP32 multiply-adds (128 x 64 tiles, 8 x 8 a thread, paired).
+//
+// Every wait is bounded. One that runs out sets `abort`, the other roles then
+// run out or see it, the unit's sums become NaN and g_xp_error is set.
+__device__ unsigned int g_xp_error = 0;
+constexpr int kDrainWarps = 8, kLoadWarps = 8;
+constexpr int kGemmThreads = 32 * (kDrainWarps + kLoadWarps + 1);
+constexpr int kStages = 4;
+constexpr int kLbo = kTileRows * 16 + 32;       // bytes between core matrices along K (padded)
+constexpr int kPlane = 4 * kLbo;                // one operand's hi or lo part, K = 16
+constexpr int kStageBytes = 4 * kPlane;         // A hi, A lo, B hi, B lo
+constexpr int kGemmSmem = kStages * kStageBytes + 1024;
+static_assert(kTileRows == kTileCols, "one loader serves both operands");
+
+__device__ __forceinline__ uint32_t instr_desc_tf32() {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kTileCols >> 3) << 17) |
+         ((uint32_t)(kTileRows >> 4) << 24);
+}
+__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
+                                         uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+// x rounded to 11 bits (half up; a NaN or an infinity stays one), and the rest
+__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
+  hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+  lo = x - hi;
+}
+
+// A unit: its tile, velocity tile, result and cells.
+struct Unit {
+  XpTile tile;
+  int mt, q, c0, c1;
+  unsigned ends;  // its groups that have end rows
 };
+__device__ __forceinline__ Unit unit_at(const XpDev& d, long long unit) {
+  Unit u;
+  u.tile = d.tile[d.unit_tile[unit]];
+  const int rest = (int)(unit - u.tile.unit);
+  u.mt = rest % d.mtiles;
+  u.q = (rest / d.mtiles) % d.nacc;
+  u.c0 = u.tile.lo + rest / (d.mtiles * d.nacc) * d.run;
+  u.c1 = min(u.c0 + d.run, u.tile.hi);
+  const int g = u.c0 + (threadIdx.x & 31) * kGroup;
+  u.ends = __ballot_sync(0xffffffffu, d.has_ends && g < u.c1 &&
+                                          d.ends[(u.tile.w + g - u.tile.lo) / kGroup] != 0);
+  return u;
+}
+// The steps of a unit: a group's four cells (sub 0 .. 3) and, if it has them,
+// its end rows (sub 4, cell then the first one after the group), each for
+// every source.
+struct Step {
+  int cell, sub, src;
+};
+template <int NSRC>
+__device__ __forceinline__ Step next_step(Step p, const Unit& u) {
+  if (++p.src < NSRC) return p;
+  p.src = 0;
+  if (p.sub < kGroup) ++p.cell;
+  ++p.sub;
+  if (p.sub == kGroup && !(u.ends >> ((p.cell - u.c0) / kGroup - 1) & 1)) ++p.sub;
+  if (p.sub > kGroup) p.sub = 0;
+  return p;
+}
+__device__ __forceinline__ bool in_unit(const Step& p, const Unit& u) {
+  return p.cell < u.c1 || p.sub == kGroup;
+}
 
 template <int NSRC>
-__global__ void __launch_bounds__(kGemmThreads, 3) xp_gemm_kernel(XpDev d) {
-  __shared__ __align__(16) GemmStage st[2];
-  __shared__ int s_tile;
-  __shared__ unsigned s_ends;
-  const int tid = threadIdx.x;
-  const int tn = tid & 7, tm = tid >> 3;
-  const int ntile = d.nsets * d.ft;
+__global__ void __launch_bounds__(kGemmThreads, 1) xp_gemm_kernel(XpDev d) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  // full[4] empty[4] acc_full[2] acc_empty[2] low_empty done
+  __shared__ __align__(8) uint64_t bars[2 * kStages + 6];
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int abort_flag;
+  uint64_t* const full = bars;
+  uint64_t* const empty = bars + kStages;
+  uint64_t* const acc_full = bars + 2 * kStages;
+  uint64_t* const acc_empty = acc_full + 2;
+  uint64_t* const low_empty = acc_full + 4;
+  uint64_t* const done = acc_full + 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int kMmaWarp = kDrainWarps + kLoadWarps;
+  if (tid == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      tc::mbar_init(full + i, kLoadWarps);
+      tc::mbar_init(empty + i, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(acc_full + i, 1);
+      tc::mbar_init(acc_empty + i, kDrainWarps);
+    }
+    tc::mbar_init(low_empty, kDrainWarps);
+    tc::mbar_init(done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    abort_flag = 0;
+  }
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     tc::smem_u32(&tmem_slot)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  const long long units = d.plan->units;
   const int nin = d.nacc > NSRC ? d.nacc : NSRC;
-  const long long plane = (long long)d.cells_cap * kNodes * d.ncp;
-  for (long long unit = blockIdx.x; unit < d.plan->units; unit += gridDim.x) {
-    if (tid == 0) {
-      int lo = 0, hi = ntile;  // the last tile whose first unit is not past `unit`
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (d.tile[mid].unit <= unit)
-          lo = mid;
-        else
-          hi = mid;
-      }
-      s_tile = lo;
+
+  // false (for the whole warp) once a wait has run out anywhere
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    bool ok = true;
+    if (!tc::mbar_try_wait(bar, parity)) {
+      const long long t0 = clock64();
+      while (ok && !tc::mbar_try_wait(bar, parity))
+        if (abort_flag || clock64() - t0 > tc::kWaitCycles) ok = false;
     }
-    __syncthreads();
-    const XpTile tile = d.tile[s_tile];
-    const int rest = (int)(unit - tile.unit);
-    const int mt = rest % d.mtiles;
-    const int q = (rest / d.mtiles) % d.nacc;
-    const int c0 = tile.lo + rest / (d.mtiles * d.nacc) * d.run;
-    const int c1 = min(c0 + d.run, tile.hi);
-    // which of the unit's groups have end rows
-    if (tid < 32) {
-      const int g = c0 + tid * kGroup;
-      const bool ends = d.has_ends && g < c1 && d.ends[(tile.w + g - tile.lo) / kGroup] != 0;
-      const unsigned m = __ballot_sync(0xffffffffu, ends);
-      if (tid == 0) s_ends = m;
-    }
-    __syncthreads();
-    const unsigned ends = s_ends;
-    // the steps: a group's four cells and, if it has them, its end rows, each
-    // for every source
-    struct Step {
-      int cell, sub, src;
-    };
-    auto next = [&](Step p) {
-      if (++p.src < NSRC) return p;
-      p.src = 0;
-      if (p.sub < kGroup) ++p.cell;
-      ++p.sub;
-      if (p.sub == kGroup && !(ends >> ((p.cell - c0) / kGroup - 1) & 1)) ++p.sub;
-      if (p.sub > kGroup) p.sub = 0;
-      return p;
-    };
-    float4 wreg[2];
-    auto load = [&](const Step& p, int buf) {
-      const int in = NSRC == 2 && p.src ? 1 - q : q;
-      if (p.sub < kGroup) {
-        const float* e = d.E + (p.src ? plane : 0) + (long long)p.cell * kNodes * d.ncp + mt * kTileRows;
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) abort_flag = 1;
+    return ok;
+  };
+
+  if (warp < kDrainWarps) {
+    // ---------------------------------------------------------------- drain
+    const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(half * 64);
+    uint32_t groups = 0, n = 0;
+    bool ok = true;
+    for (long long unit = blockIdx.x; unit < units; unit += gridDim.x, ++n) {
+      const Unit u = unit_at(d, unit);
+      float tot[64];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int v = tid + i * kGemmThreads;  // 16 rows of 32 float4
-          cp_async16(&st[buf].e[v >> 5][(v & 31) * 4], e + (long long)(v >> 5) * d.ncp + (v & 31) * 4);
+      for (int j = 0; j < 64; ++j) tot[j] = 0.0f;
+      auto add = [&](uint32_t column) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          float v[16];
+          tc::tmem_ld16(lane_base + column + h * 16, v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) tot[h * 16 + j] += v[j];
         }
-        const float4* w = reinterpret_cast<const float4*>(
-            d.W + ((tile.w + p.cell - tile.lo) * nin + in) * kBlockFloats);
-        wreg[0] = __ldg(w + tid);
-        wreg[1] = __ldg(w + tid + kGemmThreads);
-      } else {  // p.cell is the first cell of the next group
-        const int g = p.cell - kGroup;
-        const float* e = d.Eend + (p.src ? plane / kNodes * kEndRows : 0) +
-                         (long long)g * kEndRows * d.ncp + mt * kTileRows;
+      };
+      for (int c = u.c0; ok && c < u.c1; c += kGroup, ++groups) {
+        const uint32_t b = groups & 1;
+        ok = wait(acc_full + b, (groups >> 1) & 1);
+        if (!ok) break;
+        tc::tc_fence_after();
+        add(b * kTileCols);
+        if (c + kGroup >= u.c1) {  // the unit's last group: its commit covers the low products
+          add(2 * kTileCols);
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(low_empty);
+        }
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty + b);
+      }
+      float4* o = reinterpret_cast<float4*>(d.part + unit * (kTileRows * kTileCols) +
+                                            row * kTileCols + half * 64);
+      const float bad = __int_as_float(0x7fffffff);
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        o[j] = ok ? make_float4(tot[4 * j], tot[4 * j + 1], tot[4 * j + 2], tot[4 * j + 3])
+                  : make_float4(bad, bad, bad, bad);
+    }
+  } else if (warp < kMmaWarp) {
+    // ----------------------------------------------------------------- load
+    const int lt = tid - 32 * kDrainWarps;
+    const long long plane = (long long)d.cells_cap * kNodes * d.ncp;
+    uint32_t it = 0;
+    bool ok = true;
+    for (long long unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
+      const Unit u = unit_at(d, unit);
+      struct Raw {
+        float4 a[2], b[2];
+      };
+      auto fetch = [&](const Step& p, Raw& r) {
+        const int in = NSRC == 2 && p.src ? 1 - u.q : u.q;
+        if (p.sub < kGroup) {
+          const float4* e = reinterpret_cast<const float4*>(
+              d.E + (p.src ? plane : 0) +
+              ((long long)p.cell * d.mtiles + u.mt) * (kTileRows * kNodes));
+          const float4* w = reinterpret_cast<const float4*>(
+              d.W + ((u.tile.w + p.cell - u.tile.lo) * nin + in) * kBlockFloats);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            r.a[i] = __ldg(e + lt + i * 256);
+            r.b[i] = __ldg(w + lt + i * 256);
+          }
+        } else {
+          const int g = p.cell - kGroup;
+          r.a[0] = __ldg(reinterpret_cast<const float4*>(
+                             d.Eend + (p.src ? plane / kNodes * kEndRows : 0) +
+                             ((long long)(g / kGroup) * d.mtiles + u.mt) *
+                                 (kTileRows * kGroup * kEndRows)) + lt);
+          r.b[0] = __ldg(reinterpret_cast<const float4*>(
+                             d.V + ((u.tile.w + g - u.tile.lo) / kGroup * nin + in) * kEndFloats) + lt);
+        }
+      };
+      // splits and stores a step; false when a wait ran out
+      auto put = [&](const Step& p, const Raw& r) {
+        const uint32_t s = it % kStages;
+        if (it >= kStages && !wait(empty + s, (it / kStages - 1) & 1)) return false;
+        const float sg = NSRC == 2 && p.src && u.q == 0 ? -1.0f : 1.0f;
+        unsigned char* st = smem + s * kStageBytes;
+        const bool ends = p.sub == kGroup;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          const int v = tid + i * kGemmThreads;  // 8 rows
-          cp_async16(&st[buf].e[v >> 5][(v & 31) * 4], e + (long long)(v >> 5) * d.ncp + (v & 31) * 4);
+          if (i == 1 && ends) break;
+          const int v = lt + i * 256;
+          const int off = ends ? (v & 1) * kLbo + (v >> 1) * 16 : (v & 3) * kLbo + (v >> 2) * 16;
+          float4 h, l;
+          split_tf32(r.a[i].x, h.x, l.x);
+          split_tf32(r.a[i].y, h.y, l.y);
+          split_tf32(r.a[i].z, h.z, l.z);
+          split_tf32(r.a[i].w, h.w, l.w);
+          *reinterpret_cast<float4*>(st + off) = h;
+          *reinterpret_cast<float4*>(st + kPlane + off) = l;
+          split_tf32(sg * r.b[i].x, h.x, l.x);
+          split_tf32(sg * r.b[i].y, h.y, l.y);
+          split_tf32(sg * r.b[i].z, h.z, l.z);
+          split_tf32(sg * r.b[i].w, h.w, l.w);
+          *reinterpret_cast<float4*>(st + 2 * kPlane + off) = h;
+          *reinterpret_cast<float4*>(st + 3 * kPlane + off) = l;
         }
-        // four cells of 64 columns x 2: a thread takes two columns of a cell
-        wreg[0] = __ldg(reinterpret_cast<const float4*>(
-                            d.V + ((tile.w + g + (tid >> 5) - tile.lo) * nin + in) * kEndFloats) +
-                        (tid & 31));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + s);
+        ++it;
+        return true;
+      };
+      // the loads run three steps ahead of their use (a step's MMAs take less
+      // than the latency of L2)
+      Raw raw[3];
+      Step at[3];
+      at[0] = Step{u.c0, 0, 0};
+      bool on[3] = {true, false, false};
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        if (i > 0 && on[i - 1]) {
+          at[i] = next_step<NSRC>(at[i - 1], u);
+          on[i] = in_unit(at[i], u);
+        }
+        if (on[i]) fetch(at[i], raw[i]);
       }
-      cp_async_commit();
-    };
-    auto put = [&](const Step& p, int buf) {
-      const float sg = NSRC == 2 && p.src && q == 0 ? -1.0f : 1.0f;
-      if (p.sub == kGroup) {
-        const int k = (tid >> 5) * kEndRows, col = (tid & 31) * 2;
-        st[buf].w[k][col] = sg * wreg[0].x;
-        st[buf].w[k + 1][col] = sg * wreg[0].y;
-        st[buf].w[k][col + 1] = sg * wreg[0].z;
-        st[buf].w[k + 1][col + 1] = sg * wreg[0].w;
-        return;
-      }
+      while (ok && on[0]) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int v = tid + i * kGemmThreads, col = v >> 2, k = (v & 3) * 4;
-        st[buf].w[k][col] = sg * wreg[i].x;
-        st[buf].w[k + 1][col] = sg * wreg[i].y;
-        st[buf].w[k + 2][col] = sg * wreg[i].z;
-        st[buf].w[k + 3][col] = sg * wreg[i].w;
-      }
-    };
-    // sums of a group, added to the unit's totals: 64 terms in a row round half
-    // as much as a unit's 1024 do
-    float2 acc[8][4], tot[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = tot[i][j] = make_float2(0.f, 0.f);
-    Step cur{c0, 0, 0};
-    load(cur, 0);
-    for (int buf = 0;; buf ^= 1) {
-      put(cur, buf);
-      cp_async_wait<0>();
-      __syncthreads();
-      const Step nx = next(cur);
-      const bool more = nx.cell < c1 || nx.sub == kGroup;
-      if (more) load(nx, buf ^ 1);
-      const int rows = cur.sub < kGroup ? kNodes : kGroup * kEndRows;
-#pragma unroll 8
-      for (int k = 0; k < rows; ++k) {
-        const float4 e0 = *reinterpret_cast<const float4*>(&st[buf].e[k][tm * 4]);
-        const float4 e1 = *reinterpret_cast<const float4*>(&st[buf].e[k][64 + tm * 4]);
-        const float4 w0 = *reinterpret_cast<const float4*>(&st[buf].w[k][tn * 4]);
-        const float4 w1 = *reinterpret_cast<const float4*>(&st[buf].w[k][32 + tn * 4]);
-        const float ev[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
-        const float2 wv[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w),
-                              make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fjs::pfma(fjs::psplat(ev[i]), wv[j], acc[i][j]);
-      }
-      if (nx.sub == 0 && nx.src == 0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            tot[i][j] = fjs::padd(tot[i][j], acc[i][j]);
-            acc[i][j] = make_float2(0.f, 0.f);
+        for (int i = 0; i < 3; ++i) {
+          if (!on[i]) break;
+          if (!(ok = put(at[i], raw[i]))) break;
+          const int last = (i + 2) % 3;  // the furthest step that is fetched
+          on[i] = on[last];
+          if (on[i]) {
+            at[i] = next_step<NSRC>(at[last], u);
+            on[i] = in_unit(at[i], u);
+            if (on[i]) fetch(at[i], raw[i]);
           }
+        }
       }
-      if (!more) break;
-      cur = nx;
     }
-    float* o = d.part + unit * (kTileRows * kTileCols);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = (i & 4) * 16 + tm * 4 + (i & 3);
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        *reinterpret_cast<float4*>(o + row * kTileCols + h * 32 + tn * 4) = make_float4(
-            tot[i][2 * h].x, tot[i][2 * h].y, tot[i][2 * h + 1].x, tot[i][2 * h + 1].y);
+  } else {
+    // ------------------------------------------------------------------ MMA
+    // One thread. The descriptors differ in their address field alone, so a
+    // step's are sums of 32-bit words (formed anew for each MMA they took
+    // longer than the MMAs).
+    const uint32_t idesc = instr_desc_tf32();
+    const uint64_t desc0 = tc::smem_desc(smem, kLbo, 128);
+    const uint32_t desc_hi = (uint32_t)(desc0 >> 32);
+    const uint32_t low = tmem + 2 * kTileCols;
+    uint32_t it = 0, groups = 0, n = 0;
+    int ok = 1;
+    auto wait1 = [&](uint64_t* bar, uint32_t parity) {
+      if (tc::mbar_try_wait(bar, parity)) return true;
+      const long long t0 = clock64();
+      while (!tc::mbar_try_wait(bar, parity))
+        if (abort_flag || clock64() - t0 > tc::kWaitCycles) {
+          abort_flag = 1;
+          return false;
+        }
+      return true;
+    };
+    for (long long unit = blockIdx.x; ok && unit < units; unit += gridDim.x, ++n) {
+      const Unit u = unit_at(d, unit);
+      if (lane == 0) {
+        if (n > 0) ok = wait1(low_empty, (n - 1) & 1);
+        uint32_t low_on = 0;
+        for (int c = u.c0; ok && c < u.c1; c += kGroup, ++groups) {
+          const uint32_t top = tmem + (groups & 1) * kTileCols;
+          if (groups >= 2 && !(ok = wait1(acc_empty + (groups & 1), ((groups >> 1) - 1) & 1))) break;
+          const int cells = kGroup * NSRC;
+          const int steps = cells + ((u.ends >> ((c - u.c0) / kGroup)) & 1 ? NSRC : 0);
+          uint32_t top_on = 0;
+          for (int step = 0; step < steps; ++step, ++it) {
+            const uint32_t s = it % kStages;
+            if (!(ok = wait1(full + s, (it / kStages) & 1))) break;
+            // the loaders' stores before the tensor core's reads; here rather than
+            // in the loaders, where the fence would wait for their loads in flight
+            tc::fence_async_smem();
+            tc::tc_fence_after();
+            const uint32_t ah = (uint32_t)desc0 + s * (kStageBytes >> 4);
+            auto desc = [&](uint32_t at) { return ((uint64_t)desc_hi << 32) | at; };
+            auto mma3 = [&](uint32_t k, uint32_t on_low, uint32_t on_top) {
+              const uint64_t dah = desc(ah + k), dal = desc(ah + k + (kPlane >> 4));
+              const uint64_t dbh = desc(ah + k + 2 * (kPlane >> 4)), dbl = desc(ah + k + 3 * (kPlane >> 4));
+              mma_tf32(low, dal, dbh, idesc, on_low);
+              mma_tf32(low, dah, dbl, idesc, 1u);
+              mma_tf32(top, dah, dbh, idesc, on_top);
+            };
+            mma3(0, low_on, top_on);
+            if (step < cells) mma3(2 * kLbo >> 4, 1u, 1u);
+            tc::mma_commit(empty + s);
+            low_on = top_on = 1;
+          }
+          if (ok) tc::mma_commit(acc_full + (groups & 1));
+        }
+      }
+      ok = __shfl_sync(0xffffffffu, ok, 0);
     }
-    __syncthreads();  // the stages and s_tile are used again
+    if (!ok) {
+      // no MMA may be in flight when the tensor memory goes
+      if (lane == 0) {
+        tc::mma_commit(done);
+        tc::mbar_wait(done, 0, tc::kWaitCycles);
+      }
+      __syncwarp();
+    }
   }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (tid == 0 && abort_flag) atomicOr(&g_xp_error, 1u);
+  if (warp == kMmaWarp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
 // ----------------------------------------------------------------- finish
 // The units of a result added in order, the mode's magnitude, NaN at f = 0
 // (itype 1, as the reference's 1/k), and the normalisation with Python's
-// builtin max (see fj_normalize_kernel). A CTA takes 16 columns of one set; a
-// thread keeps its velocities' values in registers up to 1024 velocities.
-constexpr int kFinRows = 32, kFinKeep = 32;
+// builtin max (see fj_normalize_kernel). A CTA takes 8 columns (one 32-byte
+// sector of a row) of one set, so that 512 frequencies still make 64 CTAs; a
+// thread keeps its velocities' values in registers up to 2048 velocities.
+constexpr int kFinCols = 8, kFinRows = 128, kFinKeep = 16;
 template <int MODE, int ITYPE>
-__global__ void __launch_bounds__(16 * kFinRows) xp_finish_kernel(XpDev d) {
+__global__ void __launch_bounds__(kFinCols * kFinRows) xp_finish_kernel(XpDev d) {
   constexpr int NACC = ModeTraits<MODE>::NACC;
-  __shared__ float red[kFinRows][17];
-  const int fi = blockIdx.x * 16 + threadIdx.x, b = blockIdx.y;
+  __shared__ float red[kFinRows / 4][kFinCols];
+  const int fi = blockIdx.x * kFinCols + threadIdx.x, b = blockIdx.y;
   const bool mine = fi < d.nf && d.use[(long long)b * d.nf + min(fi, d.nf - 1)] != 0;
   if (!__syncthreads_or(mine)) return;
-  const XpTile tile = d.tile[b * d.ft + (blockIdx.x * 16) / kTileCols];
+  const XpTile tile = d.tile[b * d.ft + (blockIdx.x * kFinCols) / kTileCols];
   const int nrun = (tile.hi - tile.lo + d.run - 1) / d.run;
   const bool nan_col = ITYPE == 1 && mine && d.f[fi] == 0.0f;
   float* o = d.out + (long long)b * d.nc * d.nf + fi;
@@ -1073,14 +1276,17 @@ __global__ void __launch_bounds__(16 * kFinRows) xp_finish_kernel(XpDev d) {
       }
     }
   }
-  red[threadIdx.y][threadIdx.x] = m;
-  __shared__ float first[16];
+  // a warp holds 4 velocities of the 8 columns
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+  if ((threadIdx.y & 3) == 0) red[threadIdx.y >> 2][threadIdx.x] = m;
+  __shared__ float first[kFinCols];
   if (threadIdx.y == 0 && mine) first[threadIdx.x] = fabsf(in_regs ? keep[0] : o[0]);
   __syncthreads();
   if (!mine) return;
   float div = 1.0f;
   if (d.normalize) {
-    for (int y = 0; y < kFinRows; ++y) m = fmaxf(m, red[y][threadIdx.x]);
+    for (int y = 0; y < kFinRows / 4; ++y) m = fmaxf(m, red[y][threadIdx.x]);
     const float f0 = first[threadIdx.x];
     div = isnan(f0) ? f0 : m;
   }
@@ -1134,7 +1340,7 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
     d.chunk = p.total <= 1024 ? 8 : p.total <= 2048 ? 16 : p.total <= 4096 ? 32 : p.total <= 8192 ? 64 : 128;
   // Shorter runs of cells where the tiles alone leave SMs idle.
   const long long mn = (long long)div_up(p.nf_all, kTileCols) * d.mtiles * d.nacc;
-  d.run = batch || mn >= 256 ? 64 : mn >= 64 ? 32 : 16;
+  d.run = batch || mn >= 96 ? 64 : mn >= 32 ? 32 : mn >= 12 ? 16 : 8;
   // No column that is cheaper here than directly (xp_columns_kernel) has more
   // cells than this.
   const double most = (double)p.total * p.nc * d.nsrc * 250.0 /
@@ -1167,9 +1373,10 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   if (d.has_ends) {
     d.Eend = reinterpret_cast<float*>(
         place(sizeof(float) * (size_t)nbasis * d.cells_cap * kEndRows * d.ncp));
-    d.V = reinterpret_cast<float*>(place(sizeof(float) * (size_t)cells * nin * kEndFloats));
+    d.V = reinterpret_cast<float*>(place(sizeof(float) * (size_t)(cells / kGroup) * nin * kEndFloats));
     d.ends = reinterpret_cast<unsigned char*>(place((size_t)(cells / kGroup)));
   }
+  d.unit_tile = reinterpret_cast<int*>(place(sizeof(int) * (size_t)d.units_cap));
   d.part = reinterpret_cast<float*>(
       place(sizeof(float) * (size_t)d.units_cap * kTileRows * kTileCols));
   const size_t edge = sizeof(float) * (size_t)d.slots * p.nf * nin * kNodes;
@@ -1182,7 +1389,7 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
 
 template <int MODE, int ITYPE>
 int plan_mode(const XpDev& d, cudaStream_t s) {
-  xp_columns_kernel<MODE, ITYPE><<<dim3(d.ft, d.nsets), 64, 0, s>>>(d);
+  xp_columns_kernel<MODE, ITYPE><<<dim3(d.ft, d.nsets), kTileCols, 0, s>>>(d);
   count_launch();
   CCFJ_LAUNCH_CHECK("xp_columns_kernel");
   xp_scan_kernel<<<1, 1024, 0, s>>>(d);
@@ -1216,12 +1423,15 @@ int run_mode(const XpDev& d, cudaStream_t s) {
       <<<dim3((unsigned)d.slots, div_up(d.nf, 64)), 256, 0, s>>>(d);
   count_launch();
   CCFJ_LAUNCH_CHECK("xp_join_kernel");
-  const int grid = (int)std::min<long long>(d.units_cap, 3ll * sms);
-  xp_gemm_kernel<NSRC><<<grid, kGemmThreads, 0, s>>>(d);
+  const int grid = (int)std::min<long long>(d.units_cap, sms);
+  CCFJ_CUDA_TRY(cudaFuncSetAttribute(xp_gemm_kernel<NSRC>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+  xp_gemm_kernel<NSRC><<<grid, kGemmThreads, kGemmSmem, s>>>(d);
   count_launch();
   CCFJ_LAUNCH_CHECK("xp_gemm_kernel");
   prof_end(s);
-  xp_finish_kernel<MODE, ITYPE><<<dim3(div_up(d.nf, 16), d.nsets), dim3(16, kFinRows), 0, s>>>(d);
+  xp_finish_kernel<MODE, ITYPE>
+      <<<dim3(div_up(d.nf, kFinCols), d.nsets), dim3(kFinCols, kFinRows), 0, s>>>(d);
   count_launch();
   CCFJ_LAUNCH_CHECK("xp_finish_kernel");
   return CCFJ_OK;
@@ -1249,7 +1459,7 @@ bool xp_eligible(int mode, int itype, long long total, int nsets, int nf_all, in
   (void)mode;
   (void)itype;
   // below this the direct kernels finish before the expansion's launches do
-  return total >= 2ll * nsets && nsets <= 65535 && nf_all <= 65535 * 16 &&
+  return total >= 2ll * nsets && nsets <= 65535 && nf_all <= 65535 * 8 &&
          (double)total * nf_all * nc >= 6e6;
 }
 
@@ -1268,6 +1478,16 @@ int xp_plan(const XpProblem& p, Scratch& sc, cudaStream_t s, XpWork* w, bool* ok
   w->use = d.use;
   *ok = true;
   return p.itype == 1 ? dispatch<1>(d, p.mode, true, s) : dispatch<0>(d, p.mode, true, s);
+}
+
+int xp_sticky_error(cudaStream_t s, bool* failed) {
+  unsigned int h = 0;
+  const unsigned int zero = 0;
+  CCFJ_CUDA_TRY(cudaMemcpyFromSymbolAsync(&h, g_xp_error, sizeof(h), 0, cudaMemcpyDeviceToHost, s));
+  CCFJ_CUDA_TRY(cudaStreamSynchronize(s));
+  if (h) CCFJ_CUDA_TRY(cudaMemcpyToSymbol(g_xp_error, &zero, sizeof(zero)));
+  *failed = h != 0;
+  return CCFJ_OK;
 }
 
 int xp_run(const XpProblem& p, const XpWork& w, cudaStream_t s) {

@@ -41,6 +41,9 @@ bool xp_eligible(int mode, int itype, long long total, int nsets, int nf_all, in
 // ok = false (and no error) where the memory cannot be had: the caller then
 // computes every column directly.
 int xp_plan(const XpProblem& p, Scratch& sc, cudaStream_t s, XpWork* w, bool* ok);
+// Waits for `s`, reads the process-wide flag of the product's bounded waits
+// (set when one ran out: that unit's columns are NaN) and clears it.
+int xp_sticky_error(cudaStream_t s, bool* failed);
 // Computes the columns the plan chose, normalised if asked.
 int xp_run(const XpProblem& p, const XpWork& w, cudaStream_t s);
 
