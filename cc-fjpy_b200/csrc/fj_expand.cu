@@ -365,23 +365,62 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
 }
 
 // ------------------------------------------------------------------ basis
-// E: the values of Z0 at the cell's 16 Chebyshev nodes, from the FP64
-// functions (k r reaches 1e4 rad), to coefficients. T_4..T_7 and T_12..T_15
+// J0 and Y0 (END: J1, Y1 and the integrals B too) at x = 2 pi cyc >= 8 to about
+// 1e-9 of the amplitude, in FP64 (k r reaches 1e4 rad, and E is rounded to FP32
+// once): as eval_station_f64, with shorter polynomials and 1 / sqrt(x) by a
+// Newton step from FP32 instead of its divisions and square root (the basis of
+// 1005 cells x 1000 velocities took 164 us with that, 84 us with this).
+template <bool END>
+__device__ __forceinline__ void eval_large(double x, double cyc, ZB<double>& J, ZB<double>& Y) {
+  const double n = rint(cyc);
+  const double a = 4.0 * (cyc - n) - 0.5;
+  const double qf = rint(a);
+  const int q = (int)qf;
+  const double v = a - qf, v2 = v * v;
+  constexpr double csn[] = FJC_M64_SIN;
+  constexpr double ccs[] = FJC_M64_COS;
+  const double s = v * fjs::horner(csn, v2), c = fjs::horner(ccs, v2);
+  double sn = q & 1 ? c : s, cs = q & 1 ? s : c;
+  if (q & 2) sn = -sn;
+  if ((q + 1) & 2) cs = -cs;
+  double y = rsqrtf((float)x);
+  y = y * fma(-0.5 * x * y, y, 1.5);
+  const double s8 = 8.0 * y * y, z = s8 * s8, m = fjs::kSqrt2OverPi * y;
+  constexpr double cp[] = FJC_M64_L_P0;
+  constexpr double cq[] = FJC_M64_L_Q0;
+  const double P = fjs::horner(cp, z) * m, Q = fjs::horner(cq, z) * (s8 * m);
+  J.z0 = P * cs - Q * sn;
+  Y.z0 = P * sn + Q * cs;
+  if (END) {
+    constexpr double cp1[] = FJC_M64_L_P1;
+    constexpr double cq1[] = FJC_M64_L_Q1;
+    constexpr double cr0[] = FJC_M64_L_RHO0;
+    constexpr double cr1[] = FJC_M64_L_RHO1;
+    const double P1 = fjs::horner(cp1, z) * m, Q1 = fjs::horner(cq1, z) * (s8 * m);
+    const double rho0 = fjs::horner(cr0, z), rho1 = fjs::horner(cr1, z) * s8;
+    J.z1 = P1 * sn + Q1 * cs;
+    Y.z1 = Q1 * sn - P1 * cs;
+    J.b = 1.0 + J.z1 * rho0 - J.z0 * rho1;
+    Y.b = Y.z1 * rho0 - Y.z0 * rho1;
+  }
+}
+
+// E: the values of Z0 at the cell's 16 Chebyshev nodes to coefficients. T_4..T_7 and T_12..T_15
 // carry a minus sign here and in the moments, where it saves the negation of
 // the paired recurrence. One thread per (velocity, cell).
 template <int MODE, int ITYPE>
 __global__ void __launch_bounds__(kTileRows) xp_basis_kernel(XpDev d) {
   using MT = ModeTraits<MODE>;
   constexpr bool DY = MT::WY;
-  __shared__ double dct[kNodes][kNodes];  // [node][term]
-  __shared__ double node[kNodes];
+  __shared__ double dct[kNodes / 2][kNodes];  // [node][term]; node 15 - m by the term's parity
+  __shared__ double node[kNodes / 2];         // from the cell's middle
   const int t = threadIdx.x;
-  for (int e = t; e < kNodes * kNodes; e += kTileRows) {
-    const int m = e / kNodes, n = e % kNodes;
+  if (t < kNodes / 2 * kNodes) {
+    const int m = t / kNodes, n = t % kNodes;
     const double v = cospi(n * (m + 0.5) / kNodes) * (n == 0 ? 1.0 : 2.0) / kNodes;
     dct[m][n] = n & 4 ? -v : v;
   }
-  if (t < kNodes) node[t] = kCentre + cospi((t + 0.5) / kNodes) / (double)kPerHalf;
+  if (t < kNodes / 2) node[t] = cospi((t + 0.5) / kNodes) / (double)kPerHalf;
   __syncthreads();
   const int lo = d.plan->lo, hi = d.plan->hi;
   const double hu = d.plan->hu;
@@ -393,16 +432,27 @@ __global__ void __launch_bounds__(kTileRows) xp_basis_kernel(XpDev d) {
     for (int n = 0; n < kNodes; ++n) eJ[n] = eY[n] = 0.0;
     const double x0 = cell_begin<DY>(cell), len = cell_len<DY>(cell);
     if (j < d.nc) {
-#pragma unroll 1
-      for (int m = 0; m < kNodes; ++m) {
-        const double cyc = (x0 + len * node[m]) * per_c;
+      auto values = [&](double at, double& J0, double& Y0) {
+        const double cyc = fma(len, at, x0) * per_c, x = fjs::kTwoPi * cyc;
         ZB<double> J{}, Y{};
-        fjs::eval_station_f64<MT::WJ, MT::WY, false>(fjs::kTwoPi * cyc, cyc, J, Y);
+        if (x >= 8.0)
+          eval_large<false>(x, cyc, J, Y);
+        else
+          fjs::eval_station_f64<MT::WJ, MT::WY, false>(x, cyc, J, Y);
+        J0 = J.z0;
+        Y0 = Y.z0;
+      };
+#pragma unroll 1
+      for (int m = 0; m < kNodes / 2; ++m) {
+        double ja = 0.0, ya = 0.0, jb = 0.0, yb = 0.0;
+        values(kCentre + node[m], ja, ya);
+        values(kCentre - node[m], jb, yb);
+        const double js = ja + jb, jd = ja - jb, ys = ya + yb, yd = ya - yb;
 #pragma unroll
         for (int n = 0; n < kNodes; ++n) {
           const double w = dct[m][n];
-          if (MT::WJ) eJ[n] = fma(w, J.z0, eJ[n]);
-          if (MT::WY) eY[n] = fma(w, Y.z0, eY[n]);
+          if (MT::WJ) eJ[n] = fma(w, n & 1 ? jd : js, eJ[n]);
+          if (MT::WY) eY[n] = fma(w, n & 1 ? yd : ys, eY[n]);
         }
       }
     }
@@ -423,7 +473,10 @@ __global__ void __launch_bounds__(kTileRows) xp_basis_kernel(XpDev d) {
       double r1 = 0.0, r2J = 0.0, r2Y = 0.0, r1Y = 0.0;
       if (j < d.nc) {
         const double x = x0 + len, cyc = x * per_c, ik = 1.0 / (fjs::kTwoPi * per_c);
-        fjs::eval_station_f64<MT::WJ, MT::WY, true>(fjs::kTwoPi * cyc, cyc, J, Y);
+        if (cyc >= 8.0 / fjs::kTwoPi)
+          eval_large<true>(fjs::kTwoPi * cyc, cyc, J, Y);
+        else
+          fjs::eval_station_f64<MT::WJ, MT::WY, true>(fjs::kTwoPi * cyc, cyc, J, Y);
         r1 = x * J.z1 * ik;
         r2J = (x * J.z0 - J.b * ik) * ik * ik;
         r1Y = x * Y.z1 * ik;

@@ -140,6 +140,9 @@ def sample_sincos():
 DEG = {
     'f32': dict(S0=6, MID=10, PQ=2, RHO=5, SIN=4, COS=4),
     'f64': dict(S0=13, MID=22, PQ=11, RHO=20, SIN=7, COS=8),
+    # FP64 arithmetic to about 1e-9, for values that are then rounded to FP32
+    # (the x >= 8 forms alone)
+    'm64': dict(PQ=4, RHO=7, SIN=4, COS=5),
 }
 
 
@@ -154,14 +157,15 @@ def main():
     tS, vS, SN, CS = sample_sincos()
     names6 = ['j0', 'j1', 'bj', 'y0', 'y1', 'by']
     namesL = ['p0', 'q0', 'p1', 'q1', 'rho0', 'rho1']
-    for prec, dt in (('f32', np.float32), ('f64', np.float64)):
+    for prec, dt in (('f32', np.float32), ('f64', np.float64), ('m64', np.float64)):
         D = DEG[prec]
+        mid = prec == 'm64'
         # S0 in w = (t+1)/2
-        for i, nm in enumerate(['a', 'b', 'c', 'd', 'e', 'f']):
+        for i, nm in enumerate([] if mid else ['a', 'b', 'c', 'd', 'e', 'f']):
             cw = to_var(fit_monomial(t0, V0[:, i], D['S0']), -1.0, 2.0)
             out[(prec, 's0_' + nm)] = cw
             report.append((prec, 's0_' + nm, horner_err(cw, w0, V0[:, i], dt)))
-        for tag, tt, VV in (('s1', t1, V1), ('s2', t2, V2)):
+        for tag, tt, VV in () if mid else (('s1', t1, V1), ('s2', t2, V2)):
             for i, nm in enumerate(names6):
                 cu = fit_monomial(tt, VV[:, i], D['MID'])
                 out[(prec, tag + '_' + nm)] = cu
