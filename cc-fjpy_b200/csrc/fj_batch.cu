@@ -68,10 +68,10 @@ __global__ void batch_prep_u_kernel(InDesc in, const long long* __restrict__ off
                                     const float* __restrict__ drs, const float* __restrict__ wtr,
                                     const float4* __restrict__ geo,
                                     const float* __restrict__ thr, int itype,
-                                    void* __restrict__ dst, const unsigned char* __restrict__ use) {
+                                    void* __restrict__ dst, Elsewhere other) {
   // rows on grid x (a CTA takes a run of rows), frequencies on grid y
   const int fi = blockIdx.y * blockDim.x + threadIdx.x;
-  if (fi >= nf) return;
+  if (fi >= nf || other.all()) return;
   const long long col = (long long)fi * in.cs;
   const long long per = (total + gridDim.x - 1) / gridDim.x;
   const long long end = min(total, (blockIdx.x + 1) * per);
@@ -82,7 +82,7 @@ __global__ void batch_prep_u_kernel(InDesc in, const long long* __restrict__ off
       b = set_of(off, nsets, i);
       b_end = off[b + 1];
     }
-    if (use && use[(long long)b * nf + fi]) continue;
+    if (other.at((long long)b * nf + fi)) continue;
     const float g = in.p[(in.perm ? in.perm[i] : i) * in.ld + col];
     if (itype == 1) {
       const bool hl = i > off[b], hr = i + 1 < off[b + 1];
@@ -151,6 +151,7 @@ struct BatchDev {
 template <int MODE, int ITYPE, int CPT>
 __global__ void __launch_bounds__(256, fj_min_blocks<float>()) fj_batch_persistent_kernel(BatchDev bd) {
   __shared__ long long item_s;
+  if (bd.base.other.all()) return;
   for (;;) {
     if (threadIdx.x == 0 && threadIdx.y == 0) item_s = (long long)atomicAdd(bd.counter, 1ULL);
     __syncthreads();
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(256, fj_min_blocks<float>()) fj_batch_persiste
     a.gb[0] = static_cast<const char*>(bd.base.gb[0]) + o * a.nf * esz;
     if (ModeTraits<MODE>::NIN > 1) a.gb[1] = static_cast<const char*>(bd.base.gb[1]) + o * a.nf * esz;
     a.out += (long long)b * a.nc * a.nf;
-    if (a.use) a.use += (long long)b * a.nf;
+    if (a.other.use) a.other.use += (long long)b * a.nf;
     // velocity tiles fastest: the items of one frequency tile run side by
     // side and share its station coefficients in L2
     const int fi = (rem / bd.ctiles) * 32 + threadIdx.x;
@@ -183,15 +184,16 @@ __global__ void __launch_bounds__(256, fj_min_blocks<float>()) fj_batch_persiste
 
 // Per (set, frequency) column normalisation (builtin-max semantics, as
 // fj_normalize_kernel), set = blockIdx.y.
-// Columns marked in `use` [nsets][nf] are finished elsewhere.
+// Columns of `other` [nsets][nf] are finished elsewhere.
 __global__ void batch_normalize_kernel(float* __restrict__ out, int nc, int nf,
-                                       const unsigned char* __restrict__ use) {
+                                       Elsewhere other) {
+  if (other.all()) return;
   __shared__ float red[8][33];
   __shared__ float colmax[32];
   float* o = out + (long long)blockIdx.y * nc * nf;
   int fi = blockIdx.x * 32 + threadIdx.x;
-  if (use) {
-    if (fi < nf && use[(long long)blockIdx.y * nf + fi]) fi = nf;
+  if (other.use) {
+    if (fi < nf && other.at((long long)blockIdx.y * nf + fi)) fi = nf;
     if (!__syncthreads_or(fi < nf)) return;
   }
   // two running maxima and eight loads in flight per thread (the maximum
@@ -353,7 +355,7 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
   XpProblem xp{};
   XpWork xw{};
   bool expanded = false;
-  const unsigned char* use = nullptr;
+  Elsewhere other{};
   if (expand) {
     xp.rs = a.r;
     xp.wtr = wtr;
@@ -374,17 +376,17 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
     xp.total_all = total_all > 0 ? total_all : total;
     const int st = xp_plan(xp, sc, s, &xw, &expanded);
     if (st != CCFJ_OK) return st;
-    if (expanded) use = xw.use;
+    if (expanded) other = Elsewhere{xw.use, xw.left};
   }
   BatchDev bd{};
-  bd.base.use = use;
+  bd.base.other = other;
   const float tau = a.tau > 0 ? a.tau : kDefaultTau32;
   float* kb = nullptr;
   if (a.itype == 1) {
     kb = sc.get_n<float>(a.nf);
     if (!kb) return CCFJ_ERR_ALLOC;
     fj_kbounds_kernel<float><<<div_up(a.nf, 8), dim3(32, 8), 0, s>>>(a.f, a.c, a.nf, a.nc, tau, kb,
-                                                                nullptr);
+                                                                other);
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_kbounds_kernel");
   }
@@ -394,7 +396,7 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
     if (!g) return CCFJ_ERR_ALLOC;
     const unsigned rows = (unsigned)std::min<long long>(1024, div_up(total, 8));
     batch_prep_u_kernel<<<dim3(rows, div_up(a.nf, 32)), dim3(32, 8), 0, s>>>(
-        in[j], a.offsets, a.nsets, total, a.nf, a.r, drs, wtr, geo, kb, a.itype, g, use);
+        in[j], a.offsets, a.nsets, total, a.nf, a.r, drs, wtr, geo, kb, a.itype, g, other);
     count_launch();
     CCFJ_LAUNCH_CHECK("batch_prep_u_kernel");
     bd.base.gb[j] = g;
@@ -430,7 +432,7 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
   CCFJ_LAUNCH_CHECK("fj_batch_persistent_kernel");
   if (a.normalize) {
     batch_normalize_kernel<<<dim3(div_up(a.nf, 32), a.nsets), dim3(32, 8), 0, s>>>(a.out, a.nc,
-                                                                                   a.nf, use);
+                                                                                   a.nf, other);
     count_launch();
     CCFJ_LAUNCH_CHECK("batch_normalize_kernel");
   }
@@ -441,7 +443,7 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
 // asks for a variant of the direct kernel or a switch point of its rule.
 bool batch_expands(const ccfj_batch_args& a, long long total) {
   return a.variant == 0 && !(a.tau > 0) &&
-         xp_eligible(a.mode, a.itype, total, a.nsets, a.nf, a.nc);
+         xp_eligible(total, a.nsets, a.nf, a.nc);
 }
 
 // ---------------------------------------------------------- graph cache
@@ -719,7 +721,7 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
 
 int normalize_sets(float* out, int nsets, int nc, int nf, cudaStream_t s) {
   CCFJ_REQUIRE(nsets <= 65535, "normalisation of %d sets (> 65535)", nsets);
-  batch_normalize_kernel<<<dim3(div_up(nf, 32), nsets), dim3(32, 8), 0, s>>>(out, nc, nf, nullptr);
+  batch_normalize_kernel<<<dim3(div_up(nf, 32), nsets), dim3(32, 8), 0, s>>>(out, nc, nf, Elsewhere{});
   count_launch();
   CCFJ_LAUNCH_CHECK("batch_normalize_kernel");
   return CCFJ_OK;

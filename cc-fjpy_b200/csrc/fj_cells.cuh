@@ -211,6 +211,16 @@ struct Cell<double> {
   }
 };
 
+// Columns that the expansion (fj_expand.cu) computes: a byte per column, and
+// the number of columns that are left to the direct kernels, so that these can
+// leave at once when there are none. NULL pointers: every column is direct.
+struct Elsewhere {
+  const unsigned char* use;
+  const long long* left;
+  __device__ __forceinline__ bool all() const { return left && *left == 0; }
+  __device__ __forceinline__ bool at(long long column) const { return use && use[column] != 0; }
+};
+
 struct FjDev {
   const float* rs;
   const float* drs;  // [nr + 1]: r_i - r_{i-1}, 0 at i = 0 and at i = nr
@@ -232,9 +242,7 @@ struct FjDev {
   int i_lo, i_hi;
   float* part;
   int split_len;  // stations per range when a launch splits the set (grid z)
-  // Columns with a nonzero byte are computed elsewhere (fj_expand.cu): they
-  // are not stored, and a tile of 32 of them is skipped. NULL: none.
-  const unsigned char* use;
+  Elsewhere other;  // not stored, and a tile of 32 of them is skipped
 };
 
 // ------------------------------------------------- folded interval sum
@@ -341,9 +349,9 @@ __device__ __forceinline__ StationCoef<T> station_coef(T g, T gl, T gr, bool has
 template <typename T>
 __global__ void fj_kbounds_kernel(const float* __restrict__ f, const float* __restrict__ c,
                                   int nf, int nc, T tau, T* __restrict__ thr,
-                                  const unsigned char* __restrict__ use) {
+                                  Elsewhere other) {
   const int fi = blockIdx.x * blockDim.y + threadIdx.y;
-  if (fi >= nf || (use && use[fi])) return;
+  if (fi >= nf || other.all()) return;
   const float fl = f[fi];
   T lo = T(INFINITY), hi = T(0);
   for (int j = threadIdx.x; j < nc; j += 32) {
@@ -372,10 +380,10 @@ __device__ __forceinline__ float4 station_geometry(float r, float d_next) {
 template <typename T>
 __global__ void fj_prep_u_kernel(InDesc in, int nr, int nf, const float* __restrict__ wtr,
                                  const float4* __restrict__ geo, T* __restrict__ dst,
-                                 const unsigned char* __restrict__ use) {
+                                 Elsewhere other) {
   // pairs on grid x (as many rows of CTAs as prep_rows gives), frequencies on y
   const int fi = blockIdx.y * blockDim.x + threadIdx.x;
-  if (fi >= nf || (use && use[fi])) return;
+  if (fi >= nf || other.all() || other.at(fi)) return;
   for (int i = blockIdx.x * blockDim.y + threadIdx.y; i < nr; i += gridDim.x * blockDim.y) {
     const long long row = in.perm ? in.perm[i] : i;
     const T g = (T)in.p[row * in.ld + (long long)fi * in.cs];
@@ -399,9 +407,9 @@ __global__ void fj_prep_coef_kernel(InDesc in, int nr, int nf, const float* __re
                                     const float* __restrict__ drs,
                                     const float4* __restrict__ geo, const T* __restrict__ thr,
                                     StationCoef<T>* __restrict__ dst,
-                                    const unsigned char* __restrict__ use) {
+                                    Elsewhere other) {
   const int fi = blockIdx.y * blockDim.x + threadIdx.x;
-  if (fi >= nf || (use && use[fi])) return;
+  if (fi >= nf || other.all() || other.at(fi)) return;
   const long long* perm = in.perm;
   const long long col = (long long)fi * in.cs;
   for (int i = blockIdx.x * blockDim.y + threadIdx.y; i < nr; i += gridDim.x * blockDim.y) {
@@ -658,9 +666,9 @@ __device__ __forceinline__ void fj_cells(const FjDev& a, int fi, int c0) {
   bool f_valid = fi < a.nf;
   const int fbase = fi - (int)(threadIdx.x & 31);  // first frequency of the warp (and CTA)
   fi = f_valid ? fi : a.nf - 1;
-  if (a.use) {
+  if (a.other.use) {
     // the CTA's warps have the same frequencies, so all of them leave
-    const bool elsewhere = a.use[fi] != 0;
+    const bool elsewhere = a.other.at(fi);
     if (__all_sync(0xffffffffu, elsewhere)) return;
     f_valid = f_valid && !elsewhere;
   }

@@ -100,8 +100,11 @@ struct XpTile {
 struct XpPlan {
   double hu, inv_hu;  // cell length in u = r f, and its inverse
   long long units;
+  long long left;     // columns left to the direct kernels
   int lo, hi;         // cells of E
 };
+
+constexpr int kBad = 1 << 30;
 
 struct XpDev {
   const float* rs;
@@ -117,6 +120,7 @@ struct XpDev {
   int normalize;
   int ft;                // column tiles of a set
   int chunk;             // stations of a moments chunk
+  double nf_all;         // frequencies of the whole problem
   int mtiles;            // velocity tiles
   int run;               // cells of a GEMM unit
   int nsrc, nacc;        // products of a result, results of a column
@@ -126,7 +130,10 @@ struct XpDev {
   unsigned char* use;
   XpPlan* plan;
   XpTile* tile;
-  int* bad;              // [nsets * ft] the tile's part of r is out of order
+  // [nsets * ft] columns of the tile that go direct; kBad: the tile's part of
+  // r is out of order, or a velocity is not positive and finite
+  int* direct;
+  int* slot_set;         // [slot] the set of a moments chunk
   float* E;              // [basis][cell][velocity tile][128][16]
   float* Eend;           // [basis][group][velocity tile][128][cell of the group][2]
   float* W;              // [block][input][128][16]
@@ -142,6 +149,15 @@ struct XpDev {
 __device__ __forceinline__ long long set_begin(const XpDev& d, int b) { return d.off ? d.off[b] : 0; }
 __device__ __forceinline__ long long set_end(const XpDev& d, int b) {
   return d.off ? d.off[b + 1] : d.total;
+}
+
+// Slot of a set's first chunk: sets' slots do not overlap, since a set of n
+// pairs has at most n / chunk + 1 chunks.
+__device__ __forceinline__ long long slot_begin(const XpDev& d, int b) {
+  return set_begin(d, b) / d.chunk + b;
+}
+__device__ __forceinline__ int chunks_of(const XpDev& d, long long n) {
+  return max(1, (int)((n - 1 + d.chunk - 1) / d.chunk));
 }
 
 // ------------------------------------------------------------------ cells
@@ -189,6 +205,16 @@ __device__ __forceinline__ float cell_begin(int cell) {
 }
 
 // ------------------------------------------------------------------- plan
+// Whether the expansion is worth its launches for a set of n pairs: they take
+// about 45 us together, and the direct kernels walk the pairs one after the
+// other at 1 to 1.5 us a pair (60 pairs x 40 f x 50 c: 98 us, 58 us here), or
+// are bound by their terms (6e6: 50 us). Decided by the whole problem's sizes,
+// so that frequency windows, blocks and sets of a batch decide alike.
+constexpr double kAnyCost = 4e8;  // issue slots, 20 us
+__host__ __device__ inline bool worth(double n, double per_pair) {
+  return n >= 48.0 || (n >= 2.0 && n * per_pair >= 6e6);
+}
+
 // One CTA of 128 threads per (set, 128 frequencies).
 template <int MODE, int ITYPE>
 __global__ void xp_columns_kernel(XpDev d) {
@@ -223,7 +249,6 @@ __global__ void xp_columns_kernel(XpDev d) {
   }
   const double hu = kCellPhase / fjs::kTwoPi * (double)lo, inv_hu = 1.0 / hu;
   const int tile = b * d.ft + blockIdx.x;
-  if (t == 0) d.bad[tile] = !fine;
   if (tile == 0 && t == 0) {
     d.plan->hu = hu;
     d.plan->inv_hu = inv_hu;
@@ -231,7 +256,7 @@ __global__ void xp_columns_kernel(XpDev d) {
   const int fi = blockIdx.x * kTileCols + t;
   int first = 0, last = 0;
   bool use = false;
-  if (fine && fi < d.nf && n > 0) {
+  if (fine && fi < d.nf && worth((double)n, d.nf_all * d.nc)) {
     const float fl = d.f[fi];
     const float r0 = d.rs[o], r1 = d.rs[o + n - 1];
     if (fl == 0.0f) {
@@ -252,10 +277,18 @@ __global__ void xp_columns_kernel(XpDev d) {
         const double grid =
             (cells + kGroup) * kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0) + 200.0 * n;
         const double direct = (double)n * d.nc * d.nsrc * (cells > n ? 250.0 : 56.0);
-        use = grid < direct;
+        // (a problem whose columns all cost little keeps them together: the
+        // direct kernels' time is the walk over the pairs, for one column too)
+        use = grid < direct || grid * d.nf_all < kAnyCost;
       }
     }
-    d.use[(long long)b * d.nf + fi] = use;
+  }
+  if (fi < d.nf) d.use[(long long)b * d.nf + fi] = use;
+  const int left = __syncthreads_count(fi < d.nf && !use);
+  if (t == 0) d.direct[tile] = fine ? left : kBad;
+  if (blockIdx.x == 0) {  // the set's slots of moments chunks
+    const long long s0 = slot_begin(d, b), s1 = b + 1 < d.nsets ? slot_begin(d, b + 1) : d.slots;
+    for (long long s = s0 + t; s < s1; s += kTileCols) d.slot_set[s] = b;
   }
   const bool has = use && last > first;
   int mn = has ? first : 0x7fffffff, mx = has ? last : 0;
@@ -279,27 +312,37 @@ __global__ void xp_columns_kernel(XpDev d) {
   }
 }
 
+// Runs of cells [lo, hi): they end at multiples of d.run, so that a column's
+// sum does not depend on the tile it is in.
+__device__ __forceinline__ int runs_of(const XpDev& d, int lo, int hi) {
+  return hi > lo ? (hi + d.run - 1) / d.run - lo / d.run : 0;
+}
+
 // One CTA: exclusive sums over the tiles; without the memory for all of them,
 // or with distances out of order anywhere, every column goes direct.
 __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
   __shared__ long long sw[32], su[32];
-  __shared__ int slo[32], shi[32], sbad[32];
+  __shared__ int slo[32], shi[32];
+  __shared__ long long sleft[32];
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
   const int ntile = d.nsets * d.ft;
   long long bw = 0, bu = 0;
-  int lo = 0x7fffffff, hi = 0, bad = 0;
+  int lo = 0x7fffffff, hi = 0;
+  long long left = 0;
+  bool bad = false;
   for (int i0 = 0; i0 < ntile; i0 += 1024) {
     const int i = i0 + t;
     long long w = 0, u = 0;
     if (i < ntile) {
       const int a = d.tile[i].lo, z = d.tile[i].hi;
       w = z - a;
-      u = (long long)d.nacc * d.mtiles * ((z - a + d.run - 1) / d.run);
+      u = (long long)d.nacc * d.mtiles * runs_of(d, a, z);
       if (z > a) {
         lo = min(lo, a);
         hi = max(hi, z);
       }
-      bad |= d.bad[i];
+      left += d.direct[i] & (kBad - 1);
+      bad = bad || (d.direct[i] & kBad) != 0;
     }
     long long iw = w, iu = u;
     for (int s = 1; s < 32; s <<= 1) {
@@ -332,29 +375,32 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
   for (int s = 16; s > 0; s >>= 1) {
     lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, s));
     hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, s));
-    bad |= __shfl_xor_sync(0xffffffffu, bad, s);
+    left += __shfl_xor_sync(0xffffffffu, left, s);
   }
+  bad = __syncthreads_or(bad);
   if (lane == 0) {
     slo[wid] = lo;
     shi[wid] = hi;
-    sbad[wid] = bad;
+    sleft[wid] = left;
   }
   __syncthreads();
+  left = 0;
   for (int k = 0; k < 32; ++k) {
     lo = min(lo, slo[k]);
     hi = max(hi, shi[k]);
-    bad |= sbad[k];
+    left += sleft[k];
   }
   const bool ok = !bad && bw <= d.blocks_cap && bu <= d.units_cap;
   if (t == 0) {
     d.plan->units = ok ? bu : 0;
+    d.plan->left = ok ? left : (long long)d.nsets * d.nf;
     d.plan->lo = ok && hi > lo ? lo : 0;
     d.plan->hi = ok && hi > lo ? hi : 0;
   }
   __syncthreads();
   if (ok) {
     for (int i = t; i < ntile; i += 1024) {
-      const int runs = (d.tile[i].hi - d.tile[i].lo + d.run - 1) / d.run;
+      const int runs = runs_of(d, d.tile[i].lo, d.tile[i].hi);
       int* u = d.unit_tile + d.tile[i].unit;
       for (int k = 0; k < d.nacc * d.mtiles * runs; ++k) u[k] = i;
     }
@@ -547,26 +593,6 @@ __device__ __forceinline__ void piece_point(float2 (&acc)[NIN][kNodes / 2], floa
   add_point<NIN>(acc, fmaf(th, x, tm), a);
 }
 
-// Slot of a set's first chunk: sets' slots do not overlap, since a set of n
-// pairs has at most n / chunk + 1 chunks.
-__device__ __forceinline__ long long slot_begin(const XpDev& d, int b) {
-  return set_begin(d, b) / d.chunk + b;
-}
-__device__ __forceinline__ int chunks_of(const XpDev& d, long long n) {
-  return max(1, (int)((n - 1 + d.chunk - 1) / d.chunk));
-}
-__device__ __forceinline__ int set_of_slot(const XpDev& d, long long slot) {
-  int lo = 0, hi = d.nsets;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (slot_begin(d, mid) <= slot)
-      lo = mid;
-    else
-      hi = mid;
-  }
-  return lo;
-}
-
 // A CTA is one warp; it takes 32 frequencies and a chunk of stations. Chunk q
 // visits the stations after q chunk up to (q + 1) chunk (chunk 0 of itype 0 its
 // first station too), and for itype 1 the intervals that end there. Its lanes
@@ -582,22 +608,24 @@ __device__ __forceinline__ int set_of_slot(const XpDev& d, long long slot) {
 //
 // Bound by issue: 15 paired multiply-adds and about as many other instructions
 // a point, 2 or 3 points for most intervals. The spectra come in by cp.async,
-// 32 stations ahead; unrolling the stations instead (loads into registers)
+// 16 stations ahead; unrolling the stations instead (loads into registers)
 // left the warps waiting for instructions as long as they issued.
+constexpr int kMomStations = 16;
 template <int NIN>
 struct MomStage {
-  float g[NIN][32][32];  // [station][frequency]
-  float4 st[32];         // r, the interval's length, 1 / max(length, 0.1), trapezoid weight
+  float g[NIN][kMomStations][32];  // [station][frequency]
+  float4 st[kMomStations];  // r, the interval's length, 1 / max(length, 0.1), trapezoid weight
 };
 
 template <int NIN, int ITYPE, bool DY>
-__global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
+__global__ void __launch_bounds__(32, NIN == 1 ? 25 : 14) xp_moments_kernel(XpDev d, int ftiles) {
   __shared__ __align__(16) MomStage<NIN> stage[2];
   __shared__ float2 rule[14];
+  __shared__ float2 tot[NIN][kNodes / 2][32];  // sums of earlier stations of the lane's cell
   const int lane = threadIdx.x;
   const long long slot = blockIdx.x / ftiles;
   const int fi = (int)(blockIdx.x % ftiles) * 32 + lane;
-  const int b = set_of_slot(d, slot);
+  const int b = d.slot_set[slot];
   const long long o = set_begin(d, b);
   const int n = (int)(set_end(d, b) - o);
   const int q = (int)(slot - slot_begin(d, b));
@@ -613,11 +641,11 @@ __global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
   const XpTile tile = d.tile[b * d.ft + fc / kTileCols];
   const int s0 = q * d.chunk, s1 = min(s0 + d.chunk, n - 1);
   const float* const rs = d.rs + o;
-  float2 acc[NIN][kNodes / 2], tot[NIN][kNodes / 2];
+  float2 acc[NIN][kNodes / 2];
 #pragma unroll
   for (int k = 0; k < NIN; ++k)
 #pragma unroll
-    for (int m = 0; m < kNodes / 2; ++m) acc[k][m] = tot[k][m] = make_float2(0.f, 0.f);
+    for (int m = 0; m < kNodes / 2; ++m) acc[k][m] = make_float2(0.f, 0.f);
   bool more = false;  // tot holds part of the cell's sums
   float vA;
   int cell = locate<DY>(rs[s0], fx, vA);
@@ -631,10 +659,7 @@ __global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
 #pragma unroll
       for (int k = 0; k < NIN; ++k)
 #pragma unroll
-        for (int m = 0; m < kNodes / 2; ++m) {
-          acc[k][m] = fjs::padd(acc[k][m], tot[k][m]);
-          tot[k][m] = make_float2(0.f, 0.f);
-        }
+        for (int m = 0; m < kNodes / 2; ++m) acc[k][m] = fjs::padd(acc[k][m], tot[k][m][lane]);
       more = false;
     }
 #pragma unroll
@@ -674,17 +699,18 @@ __global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
     const long long* perm = d.in[k].perm;
     return (perm ? __ldg(perm + o + i) : o + i) * d.in[k].ld;
   };
-  // stations base .. base + 31 (each lane one station's numbers, all lanes
+  // stations base .. base + 15 (each lane one station's numbers, all lanes
   // every station's spectrum)
   auto load = [&](int base, int buf) {
-    const int i = min(base + lane, s1);
+    const int i = min(base + (lane & (kMomStations - 1)), s1);
     const float r = rs[i];
     const float D = ITYPE == 1 ? r - rs[i - 1] : 0.0f;
-    stage[buf].st[lane] = make_float4(r, D, 1.0f / fmaxf(D, 0.1f), ITYPE == 0 ? d.wtr[o + i] : 0.0f);
+    if (lane < kMomStations)
+      stage[buf].st[lane] = make_float4(r, D, 1.0f / fmaxf(D, 0.1f), ITYPE == 0 ? d.wtr[o + i] : 0.0f);
     long long row[NIN];
 #pragma unroll
     for (int k = 0; k < NIN; ++k) row[k] = row_of(k, i);
-    const int cnt = min(32, s1 - base + 1);
+    const int cnt = min(kMomStations, s1 - base + 1);
     for (int j = 0; j < cnt; ++j)
 #pragma unroll
       for (int k = 0; k < NIN; ++k)
@@ -702,14 +728,14 @@ __global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
     add_point<NIN>(acc, vA * kPerHalf, a);
   }
   int buf = 0;
-  for (int base = s0 + 1; base <= s1; base += 32, buf ^= 1) {
-    if (base + 32 <= s1)
-      load(base + 32, buf ^ 1);
+  for (int base = s0 + 1; base <= s1; base += kMomStations, buf ^= 1) {
+    if (base + kMomStations <= s1)
+      load(base + kMomStations, buf ^ 1);
     else
       cp_async_commit();  // one group per round keeps the count below
     cp_async_wait<1>();
     __syncwarp();
-    const int cnt = mine ? min(32, s1 - base + 1) : 0;
+    const int cnt = mine ? min(kMomStations, s1 - base + 1) : 0;
     const int mark = cell;
 #pragma unroll 1
     for (int j = 0; j < cnt; ++j) {
@@ -813,13 +839,13 @@ __global__ void __launch_bounds__(32) xp_moments_kernel(XpDev d, int ftiles) {
       for (int k = 0; k < NIN; ++k) gA[k] = gB[k];
       vA = vB;
     }
-    // many stations to a cell (low frequencies): sums of 32 stations, added up
+    // many stations to a cell (low frequencies): sums of 16 stations, added up
     if (cell == mark) {
 #pragma unroll
       for (int k = 0; k < NIN; ++k)
 #pragma unroll
         for (int m = 0; m < kNodes / 2; ++m) {
-          tot[k][m] = fjs::padd(tot[k][m], acc[k][m]);
+          tot[k][m][lane] = more ? fjs::padd(tot[k][m][lane], acc[k][m]) : acc[k][m];
           acc[k][m] = make_float2(0.f, 0.f);
         }
       more = true;
@@ -842,7 +868,7 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
   const int fi = blockIdx.y * 64 + (threadIdx.x >> 2);
   const long long slot = blockIdx.x;
   if (fi >= d.nf) return;
-  const int b = set_of_slot(d, slot);
+  const int b = d.slot_set[slot];
   const int n = (int)(set_end(d, b) - set_begin(d, b));
   const int q = (int)(slot - slot_begin(d, b)), nch = chunks_of(d, n);
   if (q >= nch || !d.use[(long long)b * d.nf + fi]) return;
@@ -982,8 +1008,9 @@ __device__ __forceinline__ Unit unit_at(const XpDev& d, long long unit) {
   const int rest = (int)(unit - u.tile.unit);
   u.mt = rest % d.mtiles;
   u.q = (rest / d.mtiles) % d.nacc;
-  u.c0 = u.tile.lo + rest / (d.mtiles * d.nacc) * d.run;
-  u.c1 = min(u.c0 + d.run, u.tile.hi);
+  const int run = u.tile.lo / d.run + rest / (d.mtiles * d.nacc);
+  u.c0 = max(u.tile.lo, run * d.run);
+  u.c1 = min((run + 1) * d.run, u.tile.hi);
   const int g = u.c0 + (threadIdx.x & 31) * kGroup;
   u.ends = __ballot_sync(0xffffffffu, d.has_ends && g < u.c1 &&
                                           d.ends[(u.tile.w + g - u.tile.lo) / kGroup] != 0);
@@ -1280,18 +1307,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xp_gemm_kernel(XpDev d) {
 // The units of a result added in order, the mode's magnitude, NaN at f = 0
 // (itype 1, as the reference's 1/k), and the normalisation with Python's
 // builtin max (see fj_normalize_kernel). A CTA takes 8 columns (one 32-byte
-// sector of a row) of one set, so that 512 frequencies still make 64 CTAs; a
-// thread keeps its velocities' values in registers up to 2048 velocities.
-constexpr int kFinCols = 8, kFinRows = 128, kFinKeep = 16;
-template <int MODE, int ITYPE>
-__global__ void __launch_bounds__(kFinCols * kFinRows) xp_finish_kernel(XpDev d) {
+// sector of a row) of one set, so that 512 frequencies still make 64 CTAs, or
+// 32 where that leaves enough CTAs (128 subarrays x 512 f x 500 c: 400 us with
+// 8). A thread keeps its velocities' values in registers where they fit (2048
+// or 1024 velocities).
+constexpr int kFinThreads = 1024;
+template <int MODE, int ITYPE, int kFinCols>
+__global__ void __launch_bounds__(kFinThreads) xp_finish_kernel(XpDev d) {
+  constexpr int kFinRows = kFinThreads / kFinCols, kFinKeep = kFinCols == 8 ? 16 : 32;
+  constexpr int kWarpRows = 32 / kFinCols;
   constexpr int NACC = ModeTraits<MODE>::NACC;
-  __shared__ float red[kFinRows / 4][kFinCols];
+  __shared__ float red[kFinRows / kWarpRows][kFinCols];
   const int fi = blockIdx.x * kFinCols + threadIdx.x, b = blockIdx.y;
   const bool mine = fi < d.nf && d.use[(long long)b * d.nf + min(fi, d.nf - 1)] != 0;
   if (!__syncthreads_or(mine)) return;
   const XpTile tile = d.tile[b * d.ft + (blockIdx.x * kFinCols) / kTileCols];
-  const int nrun = (tile.hi - tile.lo + d.run - 1) / d.run;
+  const int nrun = runs_of(d, tile.lo, tile.hi);
   const bool nan_col = ITYPE == 1 && mine && d.f[fi] == 0.0f;
   float* o = d.out + (long long)b * d.nc * d.nf + fi;
   auto value = [&](int c) {
@@ -1329,17 +1360,16 @@ __global__ void __launch_bounds__(kFinCols * kFinRows) xp_finish_kernel(XpDev d)
       }
     }
   }
-  // a warp holds 4 velocities of the 8 columns
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-  if ((threadIdx.y & 3) == 0) red[threadIdx.y >> 2][threadIdx.x] = m;
+#pragma unroll
+  for (int s = kFinCols; s < 32; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+  if (threadIdx.y % kWarpRows == 0) red[threadIdx.y / kWarpRows][threadIdx.x] = m;
   __shared__ float first[kFinCols];
   if (threadIdx.y == 0 && mine) first[threadIdx.x] = fabsf(in_regs ? keep[0] : o[0]);
   __syncthreads();
   if (!mine) return;
   float div = 1.0f;
   if (d.normalize) {
-    for (int y = 0; y < kFinRows / 4; ++y) m = fmaxf(m, red[y][threadIdx.x]);
+    for (int y = 0; y < kFinRows / kWarpRows; ++y) m = fmaxf(m, red[y][threadIdx.x]);
     const float f0 = first[threadIdx.x];
     div = isnan(f0) ? f0 : m;
   }
@@ -1383,6 +1413,7 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   d.nsrc = nsrc_of(p.mode);
   d.nacc = nacc_of(p.mode);
   d.has_ends = p.itype == 1;
+  d.nf_all = p.nf_all;
   const int nin = nin_of(p.mode);
   const bool batch = p.off != nullptr;
   // Stations of a moments chunk: long chunks leave fewer shared cells to
@@ -1390,13 +1421,12 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   if (batch)
     d.chunk = p.total_all >= 100000 ? 128 : 32;
   else
-    d.chunk = p.total <= 1024 ? 8 : p.total <= 2048 ? 16 : p.total <= 4096 ? 32 : p.total <= 8192 ? 64 : 128;
+    d.chunk = p.total <= 128 ? 4 : p.total <= 1024 ? 8 : p.total <= 2048 ? 16 : p.total <= 4096 ? 32 : p.total <= 8192 ? 64 : 128;
   // Shorter runs of cells where the tiles alone leave SMs idle.
   const long long mn = (long long)div_up(p.nf_all, kTileCols) * d.mtiles * d.nacc;
   d.run = batch || mn >= 96 ? 64 : mn >= 32 ? 32 : mn >= 12 ? 16 : 8;
-  // No column that is cheaper here than directly (xp_columns_kernel) has more
-  // cells than this.
-  const double most = (double)p.total * p.nc * d.nsrc * 250.0 /
+  // No column that the plan takes (xp_columns_kernel) has more cells than this.
+  const double most = std::max((double)p.total * p.nc * d.nsrc * 250.0, kAnyCost / p.nf_all) /
                       (kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0));
   d.cells_cap = (int)std::min<double>(kMaxCells, 2 * kGroup + kDyadic + most) & ~(kGroup - 1);
   const long long ntile = (long long)p.nsets * d.ft;
@@ -1408,7 +1438,7 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   }
   cells &= ~(long long)(kGroup - 1);
   d.blocks_cap = cells;
-  d.units_cap = (long long)d.nacc * d.mtiles * (cells / d.run + ntile);
+  d.units_cap = (long long)d.nacc * d.mtiles * (cells / d.run + 2 * ntile);
   d.slots = p.total / d.chunk + p.nsets + 1;
   size_t at = 0;
   auto place = [&](size_t bytes) {
@@ -1419,7 +1449,8 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   d.use = reinterpret_cast<unsigned char*>(place((size_t)p.nsets * p.nf));
   d.plan = reinterpret_cast<XpPlan*>(place(sizeof(XpPlan)));
   d.tile = reinterpret_cast<XpTile*>(place(sizeof(XpTile) * ntile));
-  d.bad = reinterpret_cast<int*>(place(sizeof(int) * ntile));
+  d.direct = reinterpret_cast<int*>(place(sizeof(int) * ntile));
+  d.slot_set = reinterpret_cast<int*>(place(sizeof(int) * (size_t)d.slots));
   const int nbasis = d.nsrc;
   d.E = reinterpret_cast<float*>(place(sizeof(float) * (size_t)nbasis * d.cells_cap * kNodes * d.ncp));
   d.W = reinterpret_cast<float*>(place(sizeof(float) * (size_t)cells * nin * kBlockFloats));
@@ -1483,8 +1514,12 @@ int run_mode(const XpDev& d, cudaStream_t s) {
   count_launch();
   CCFJ_LAUNCH_CHECK("xp_gemm_kernel");
   prof_end(s);
-  xp_finish_kernel<MODE, ITYPE>
-      <<<dim3(div_up(d.nf, kFinCols), d.nsets), dim3(kFinCols, kFinRows), 0, s>>>(d);
+  if ((long long)d.nsets * div_up(d.nf, 32) >= 4 * sms)
+    xp_finish_kernel<MODE, ITYPE, 32>
+        <<<dim3(div_up(d.nf, 32), d.nsets), dim3(32, kFinThreads / 32), 0, s>>>(d);
+  else
+    xp_finish_kernel<MODE, ITYPE, 8>
+        <<<dim3(div_up(d.nf, 8), d.nsets), dim3(8, kFinThreads / 8), 0, s>>>(d);
   count_launch();
   CCFJ_LAUNCH_CHECK("xp_finish_kernel");
   return CCFJ_OK;
@@ -1508,12 +1543,9 @@ int dispatch(const XpDev& d, int mode, bool plan, cudaStream_t s) {
 
 }  // namespace
 
-bool xp_eligible(int mode, int itype, long long total, int nsets, int nf_all, int nc) {
-  (void)mode;
-  (void)itype;
-  // below this the direct kernels finish before the expansion's launches do
-  return total >= 2ll * nsets && nsets <= 65535 && nf_all <= 65535 * 8 &&
-         (double)total * nf_all * nc >= 6e6;
+bool xp_eligible(long long total, int nsets, int nf_all, int nc) {
+  // (a batch's largest set may hold nearly all pairs; the plan decides set by set)
+  return nsets <= 65535 && nf_all <= 65535 * 8 && worth((double)total, (double)nf_all * nc);
 }
 
 int xp_plan(const XpProblem& p, Scratch& sc, cudaStream_t s, XpWork* w, bool* ok) {
@@ -1529,6 +1561,7 @@ int xp_plan(const XpProblem& p, Scratch& sc, cudaStream_t s, XpWork* w, bool* ok
   layout(p, base, &d);
   w->base = base;
   w->use = d.use;
+  w->left = &d.plan->left;
   *ok = true;
   return p.itype == 1 ? dispatch<1>(d, p.mode, true, s) : dispatch<0>(d, p.mode, true, s);
 }

@@ -29,14 +29,15 @@ struct XpProblem {
 
 // What the host sized and where it lies in the call's scratch.
 struct XpWork {
-  unsigned char* use;  // [nsets][nf] 1: the expansion computes the column
+  const unsigned char* use;  // [nsets][nf] 1: the expansion computes the column
+  const long long* left;     // how many columns it leaves
   void* base;
 };
 
 // Whether a problem of these sizes runs the expansion at all. Decided from
 // the sizes of the whole problem alone, so that frequency windows and blocks
 // of one problem decide alike.
-bool xp_eligible(int mode, int itype, long long total, int nsets, int nf_all, int nc);
+bool xp_eligible(long long total, int nsets, int nf_all, int nc);
 // Reserves the scratch and runs the plan (which columns take the expansion).
 // ok = false (and no error) where the memory cannot be had: the caller then
 // computes every column directly.

@@ -62,6 +62,7 @@ __global__ void fj_prep_geom_kernel(const float* __restrict__ rs, int nr, float*
 
 template <int MODE, int ITYPE, typename T, int CPT>
 __global__ void __launch_bounds__(256, fj_min_blocks<T>()) fj_amortized_kernel(FjDev a) {
+  if (a.other.all()) return;
   if (gridDim.z > 1) {
     // split launch: CTA layer z sums stations [z L, (z + 1) L) into its own
     // partial sums (fj_split_finish_kernel adds the layers in order)
@@ -83,10 +84,10 @@ template <int MODE>
 __global__ void fj_split_finish_kernel(const float* __restrict__ part, int nsplit,
                                        const float* __restrict__ f, const float* __restrict__ c,
                                        int nc, int nf, float* __restrict__ out,
-                                       const unsigned char* __restrict__ use) {
+                                       Elsewhere other) {
   const int fi = blockIdx.x * 32 + threadIdx.x;
   const int ci = blockIdx.y * 8 + threadIdx.y;
-  if (fi >= nf || ci >= nc || (use && use[fi])) return;
+  if (fi >= nf || ci >= nc || other.all() || other.at(fi)) return;
   constexpr int NACC = ModeTraits<MODE>::NACC;
   const long long plane = (long long)nc * nf, at = (long long)ci * nf + fi;
   float tot[2] = {0.f, 0.f};
@@ -185,14 +186,15 @@ __global__ void fj_gather_kernel(InDesc in, int nr, int nf, float* __restrict__ 
 // (src/ccfj-gpu.pyx:266-267): the running maximum starts at row 0 and is
 // replaced only by a strictly larger value, so a NaN in row 0 makes the
 // column NaN while NaNs in later rows are skipped.
-// Columns marked in `use` are finished elsewhere.
+// Columns of `other` are finished elsewhere.
 __global__ void fj_normalize_kernel(float* __restrict__ out, int nc, int nf,
-                                    const unsigned char* __restrict__ use) {
+                                    Elsewhere other) {
+  if (other.all()) return;
   __shared__ float red[8][33];
   __shared__ float colmax[32];
   int fi = blockIdx.x * 32 + threadIdx.x;
-  if (use) {
-    if (fi < nf && use[fi]) fi = nf;
+  if (other.use) {
+    if (fi < nf && other.at(fi)) fi = nf;
     if (!__syncthreads_or(fi < nf)) return;
   }
   float m = -INFINITY;
@@ -369,17 +371,17 @@ size_t interval_data_bytes(const ccfj_fj_args& a) {
 // sizes above; d.rs, d.drs, d.geo (itype 1), d.nr, d.nf, d.tau must be set.
 int prep_interval_data(const ccfj_fj_args& a, FjDev& d, const InDesc* in, int nin, void* kb,
                        void* const* gbuf, const float* wtr, cudaStream_t s) {
-  const unsigned char* use = d.use;
+  const Elsewhere other = d.other;
   const bool fp32 = a.precision == CCFJ_PREC_FP32;
   if (a.itype == 1) {
     const dim3 kbb(32, 8);
     if (fp32)
       fj_kbounds_kernel<float><<<div_up(a.nf, 8), kbb, 0, s>>>(a.f, a.c, a.nf, a.nc, d.tau,
-                                                               static_cast<float*>(kb), use);
+                                                               static_cast<float*>(kb), other);
     else
       fj_kbounds_kernel<double><<<div_up(a.nf, 8), kbb, 0, s>>>(a.f, a.c, a.nf, a.nc,
                                                                 (double)d.tau,
-                                                                static_cast<double*>(kb), use);
+                                                                static_cast<double*>(kb), other);
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_kbounds_kernel");
     d.kb = kb;
@@ -391,20 +393,20 @@ int prep_interval_data(const ccfj_fj_args& a, FjDev& d, const InDesc* in, int ni
       if (fp32)
         fj_prep_coef_kernel<float><<<pg, pb, 0, s>>>(in[j], a.nr, a.nf, d.rs, d.drs, d.geo,
                                                      static_cast<const float*>(kb),
-                                                     static_cast<StationCoef<float>*>(g), use);
+                                                     static_cast<StationCoef<float>*>(g), other);
       else
         fj_prep_coef_kernel<double><<<pg, pb, 0, s>>>(in[j], a.nr, a.nf, d.rs, d.drs, d.geo,
                                                       static_cast<const double*>(kb),
-                                                      static_cast<StationCoef<double>*>(g), use);
+                                                      static_cast<StationCoef<double>*>(g), other);
       count_launch();
       CCFJ_LAUNCH_CHECK("fj_prep_coef_kernel");
     } else {
       if (fp32)
         fj_prep_u_kernel<float><<<pg, pb, 0, s>>>(in[j], a.nr, a.nf, wtr, d.geo,
-                                                  static_cast<float*>(g), use);
+                                                  static_cast<float*>(g), other);
       else
         fj_prep_u_kernel<double><<<pg, pb, 0, s>>>(in[j], a.nr, a.nf, wtr, d.geo,
-                                                   static_cast<double*>(g), use);
+                                                   static_cast<double*>(g), other);
       count_launch();
       CCFJ_LAUNCH_CHECK("fj_prep_u_kernel");
     }
@@ -421,7 +423,7 @@ static bool expansion_allowed(const ccfj_fj_args& a) {
   return a.precision == CCFJ_PREC_FP32 && !(a.tau > 0) &&
          g_force_cpt.load(std::memory_order_relaxed) == 0 &&
          g_force_split.load(std::memory_order_relaxed) == 0 &&
-         xp_eligible(a.mode, a.itype, a.nr, 1, a.nf_total > 0 ? a.nf_total : a.nf, a.nc);
+         xp_eligible(a.nr, 1, a.nf_total > 0 ? a.nf_total : a.nf, a.nc);
 }
 
 // Device-resident transform: every pointer in `a` is a device pointer.
@@ -491,7 +493,7 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
     xp.nf_all = choice.nf_all > 0 ? choice.nf_all : a.nf_total > 0 ? a.nf_total : a.nf;
     const int st = xp_plan(xp, sc, s, &xw, &expanded);
     if (st != CCFJ_OK) return st;
-    if (expanded) d.use = xw.use;
+    if (expanded) d.other = Elsewhere{xw.use, xw.left};
   }
 
   const float* plain[2] = {nullptr, nullptr};
@@ -558,22 +560,22 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
     const dim3 fg(div_up(a.nf, 32), div_up(a.nc, 8)), fb(32, 8);
     switch (a.mode) {
       case CCFJ_MODE_J:
-        fj_split_finish_kernel<CCFJ_MODE_J><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out, d.use);
+        fj_split_finish_kernel<CCFJ_MODE_J><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out, d.other);
         break;
       case CCFJ_MODE_Y:
-        fj_split_finish_kernel<CCFJ_MODE_Y><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out, d.use);
+        fj_split_finish_kernel<CCFJ_MODE_Y><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out, d.other);
         break;
       case CCFJ_MODE_J_MINUS_Y:
         fj_split_finish_kernel<CCFJ_MODE_J_MINUS_Y><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc,
-                                                                     a.nf, a.out, d.use);
+                                                                     a.nf, a.out, d.other);
         break;
       case CCFJ_MODE_ABS_J:
         fj_split_finish_kernel<CCFJ_MODE_ABS_J><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf,
-                                                                 a.out, d.use);
+                                                                 a.out, d.other);
         break;
       default:
         fj_split_finish_kernel<CCFJ_MODE_ABS_H><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf,
-                                                                 a.out, d.use);
+                                                                 a.out, d.other);
         break;
     }
     count_launch();
@@ -581,7 +583,7 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
   }
 
   if (a.normalize) {
-    fj_normalize_kernel<<<div_up(a.nf, 32), dim3(32, 8), 0, s>>>(a.out, a.nc, a.nf, d.use);
+    fj_normalize_kernel<<<div_up(a.nf, 32), dim3(32, 8), 0, s>>>(a.out, a.nc, a.nf, d.other);
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_normalize_kernel");
   }
@@ -1217,7 +1219,7 @@ static int fj_noalloc(const ccfj_fj_args& a, cudaStream_t s) {
   count_launch();
   CCFJ_LAUNCH_CHECK("fj transform kernel");
   if (a.normalize) {
-    fj_normalize_kernel<<<div_up(a.nf, 32), dim3(32, 8), 0, s>>>(a.out, a.nc, a.nf, nullptr);
+    fj_normalize_kernel<<<div_up(a.nf, 32), dim3(32, 8), 0, s>>>(a.out, a.nc, a.nf, Elsewhere{});
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_normalize_kernel");
   }
