@@ -100,6 +100,7 @@ struct XpTile {
 struct XpPlan {
   double hu, inv_hu;  // cell length in u = r f, and its inverse
   long long units;
+  long long blocks;   // W blocks of an input
   long long left;     // columns left to the direct kernels
   int lo, hi;         // cells of E
 };
@@ -393,6 +394,7 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
   const bool ok = !bad && bw <= d.blocks_cap && bu <= d.units_cap;
   if (t == 0) {
     d.plan->units = ok ? bu : 0;
+    d.plan->blocks = ok ? bw : 0;
     d.plan->left = ok ? left : (long long)d.nsets * d.nf;
     d.plan->lo = ok && hi > lo ? lo : 0;
     d.plan->hi = ok && hi > lo ? hi : 0;
@@ -415,7 +417,7 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
 // 1e-9 of the amplitude, in FP64 (k r reaches 1e4 rad, and E is rounded to FP32
 // once): as eval_station_f64, with shorter polynomials and 1 / sqrt(x) by a
 // Newton step from FP32 instead of its divisions and square root (the basis of
-// 1005 cells x 1000 velocities took 164 us with that, 84 us with this).
+// 1005 cells x 1000 velocities took 164 us with that, 89 us with this).
 template <bool END>
 __device__ __forceinline__ void eval_large(double x, double cyc, ZB<double>& J, ZB<double>& Y) {
   const double n = rint(cyc);
@@ -468,6 +470,15 @@ __global__ void __launch_bounds__(kTileRows) xp_basis_kernel(XpDev d) {
   }
   if (t < kNodes / 2) node[t] = cospi((t + 0.5) / kNodes) / (double)kPerHalf;
   __syncthreads();
+  if (ITYPE == 1) {
+    // V and its flags, which the moments write only where there are end rows
+    const long long n4 = d.plan->blocks / kGroup * MT::NIN * (kEndFloats / 4);
+    const long long id = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kTileRows + t;
+    const long long all = (long long)gridDim.x * gridDim.y * kTileRows;
+    for (long long i = id; i < n4; i += all)
+      reinterpret_cast<float4*>(d.V)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (long long i = id; i < d.plan->blocks / kGroup; i += all) d.ends[i] = 0;
+  }
   const int lo = d.plan->lo, hi = d.plan->hi;
   const double hu = d.plan->hu;
   const int j = blockIdx.x * kTileRows + t;
@@ -609,7 +620,11 @@ __device__ __forceinline__ void piece_point(float2 (&acc)[NIN][kNodes / 2], floa
 // Bound by issue: 15 paired multiply-adds and about as many other instructions
 // a point, 2 or 3 points for most intervals. The spectra come in by cp.async,
 // 16 stations ahead; unrolling the stations instead (loads into registers)
-// left the warps waiting for instructions as long as they issued.
+// left the warps waiting for instructions as long as they issued. A lane of
+// short intervals follows its cell by one compare with the next one's start
+// (locate() only after a long interval), and the zeros of V come from the basis
+// kernel: 19,900 pairs x 2048 f 472 us with a locate() and V in every step,
+// 435 us so; 20 subarrays 1884 and 1755 us.
 constexpr int kMomStations = 16;
 template <int NIN>
 struct MomStage {
@@ -618,7 +633,7 @@ struct MomStage {
 };
 
 template <int NIN, int ITYPE, bool DY>
-__global__ void __launch_bounds__(32, NIN == 1 ? 25 : 14) xp_moments_kernel(XpDev d, int ftiles) {
+__global__ void __launch_bounds__(32, NIN == 1 ? 24 : 16) xp_moments_kernel(XpDev d, int ftiles) {
   __shared__ __align__(16) MomStage<NIN> stage[2];
   __shared__ float2 rule[14];
   __shared__ float2 tot[NIN][kNodes / 2][32];  // sums of earlier stations of the lane's cell
@@ -652,7 +667,10 @@ __global__ void __launch_bounds__(32, NIN == 1 ? 25 : 14) xp_moments_kernel(XpDe
   const int cell0 = cell;
   float base_x = cell_begin<DY>(cell);
   const long long edge = ((slot * d.nf + fc) * NIN) * kNodes;
-  float* W = d.W + (tile.w + cell - tile.lo) * NIN * kBlockFloats + (fc & (kTileCols - 1)) * kNodes;
+  // where the current cell goes, and the next one
+  float* here = d.head + edge;
+  long long here_step = kNodes;
+  float* next = d.W + (tile.w + cell + 1 - tile.lo) * NIN * kBlockFloats + (fc & (kTileCols - 1)) * kNodes;
   float* const V = d.V + (tile.w / kGroup) * NIN * kEndFloats + (fc & (kTileCols - 1)) * kGroup * kEndRows;
   auto store = [&](float* base, long long step) {
     if (more) {
@@ -673,19 +691,11 @@ __global__ void __launch_bounds__(32, NIN == 1 ? 25 : 14) xp_moments_kernel(XpDe
       }
     }
   };
-  // the cell is finished; vx, vy: the weights of its end
-  auto flush = [&](const float (&vx)[NIN], const float (&vy)[NIN], bool ends) {
-    const bool first = cell == cell0;
-    store(first ? d.head + edge : W, first ? kNodes : kBlockFloats);
-    if (ITYPE == 1) {
-      const int at = cell - tile.lo;
-      float* v = V + (long long)(at / kGroup) * (NIN * kEndFloats) + (at & (kGroup - 1)) * kEndRows;
-#pragma unroll
-      for (int k = 0; k < NIN; ++k)
-        *reinterpret_cast<float2*>(v + k * kEndFloats) = make_float2(vx[k], vy[k]);
-      if (ends) d.ends[(tile.w + at) / kGroup] = 1;
-    }
-    W += NIN * kBlockFloats;
+  auto flush = [&]() {  // the cell is finished
+    store(here, here_step);
+    here = next;
+    here_step = kBlockFloats;
+    next += NIN * kBlockFloats;
     ++cell;
     if (DY)
       base_x = cell_begin<DY>(cell);
@@ -741,35 +751,32 @@ __global__ void __launch_bounds__(32, NIN == 1 ? 25 : 14) xp_moments_kernel(XpDe
     for (int j = 0; j < cnt; ++j) {
       const float4 st = stage[buf].st[j];
       const float rB = st.x, D = st.y;
-      // the station's cell and place, as locate() finds them, from the cell
-      // that the lane is in
-      const float p = __fmul_rn(rB, fx.hi);
-      const float l = fmaf(rB, fx.lo, fmaf(rB, fx.hi, -p));
-      int cB = cell;
-      float vB;
-      if (DY && cell < kDyadic) {
-        cB = locate<DY>(rB, fx, vB);
-      } else {
-        if ((p - (base_x + 1.0f)) + l >= 0.0f) cB = locate<DY>(rB, fx, vB);
-        vB = (p - (base_x + (float)(cB - cell) + kCentre)) + l;
-      }
-      float gB[NIN], gm[NIN], gh[NIN];
+      float gB[NIN], gm[NIN], gh[NIN], vB;
 #pragma unroll
       for (int k = 0; k < NIN; ++k) gB[k] = stage[buf].g[k][j][lane];
       // itype 1: a short interval whole, in the cell of its far end; a long one
       // from its beginning to the first cell end, from the last cell end on,
       // and between the two in closed form. (Lanes that end a cell do so before
       // all lanes' points.)
-      const float dB = D * fx.hi * (DY ? 1.0f / cell_len<DY>(cB) : 1.0f);
+      float dB = D * fx.hi;
+      int cB = 0;
+      const bool dyadic = DY && cell < kDyadic;
+      if (dyadic) {
+        cB = locate<DY>(rB, fx, vB);
+        dB /= cell_len<DY>(cB);
+      }
       if (ITYPE == 0 || dB <= kShort) {
-        if (cell < cB) {
-          float none[NIN];
-#pragma unroll
-          for (int k = 0; k < NIN; ++k) none[k] = 0.0f;
+        if (dyadic) {
 #pragma unroll 1
-          do
-            flush(none, none, false);
-          while (cell < cB);
+          while (cell < cB) flush();
+        } else {
+          // the station's cell and place, as locate() finds them, from the cell
+          // that the lane is in
+          const float p = __fmul_rn(rB, fx.hi);
+          const float l = fmaf(rB, fx.lo, fmaf(rB, fx.hi, -p));
+#pragma unroll 1
+          while ((p - (base_x + 1.0f)) + l >= 0.0f) flush();
+          vB = (p - (base_x + kCentre)) + l;
         }
         if (ITYPE == 0) {
 #pragma unroll
@@ -794,6 +801,7 @@ __global__ void __launch_bounds__(32, NIN == 1 ? 25 : 14) xp_moments_kernel(XpDe
           }
         }
       } else {
+        if (!dyadic) cB = locate<DY>(rB, fx, vB);
         const int span = cB - cell;
 #pragma unroll 1
         for (int step = 0;; ++step) {
@@ -818,21 +826,22 @@ __global__ void __launch_bounds__(32, NIN == 1 ? 25 : 14) xp_moments_kernel(XpDe
               piece_point<NIN>(acc, rule[i].x, rule[i].y, tm, th, rm, hr, gm, gh);
           }
           if (!cross) break;
-          float vx[NIN], vy[NIN];
-          const bool ends = span > 1 && (step == 0 || step == span - 1);
+          if (span > 1 && (step == 0 || step == span - 1)) {
+            // the cell end's weights: the spectrum's line there, from A, or from B
+            // back, and its slope
+            const int at = cell - tile.lo;
+            float* v = V + (long long)(at / kGroup) * (NIN * kEndFloats) + (at & (kGroup - 1)) * kEndRows;
+            const float back = (vB + kCentre) * cell_len<DY>(cB) * huf;
+            const float h2 = step == 0 ? -huf * huf : huf * huf;
 #pragma unroll
-          for (int k = 0; k < NIN; ++k) {
-            vx[k] = vy[k] = 0.0f;
-            if (ends) {
-              // the spectrum's line at the cell end: from A, or from B back
+            for (int k = 0; k < NIN; ++k) {
               const float sl = (gB[k] - gA[k]) * st.z;
-              const float back = (vB + kCentre) * cell_len<DY>(cB) * huf;
-              const float h2 = step == 0 ? -huf * huf : huf * huf;
-              vx[k] = h2 * fmaf(sl, step == 0 ? 2.0f * hr : D - back, gA[k]);
-              vy[k] = h2 * huf * sl;
+              *reinterpret_cast<float2*>(v + k * kEndFloats) =
+                  make_float2(h2 * fmaf(sl, step == 0 ? 2.0f * hr : D - back, gA[k]), h2 * huf * sl);
             }
+            d.ends[(tile.w + at) / kGroup] = 1;
           }
-          flush(vx, vy, ends);
+          flush();
         }
       }
 #pragma unroll
@@ -889,19 +898,10 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
     v = make_float4(v.x + a.x, v.y + a.y, v.z + a.z, v.w + a.w);
   };
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto clear_end = [&](int cell) {
-    if (ITYPE == 0 || n4 != 0) return;
-    const long long blk = tile.w + cell - tile.lo;
-    float* p = d.V + (blk / kGroup) * NIN * kEndFloats +
-               ((fi & (kTileCols - 1)) * kGroup + (blk & (kGroup - 1))) * kEndRows;
-#pragma unroll
-    for (int k = 0; k < NIN; ++k) *reinterpret_cast<float2*>(p + k * kEndFloats) = make_float2(0.f, 0.f);
-  };
   if (q == 0)
     for (int c = tile.lo; c < me.x; ++c) {
 #pragma unroll
       for (int k = 0; k < NIN; ++k) put(c, k, zero);
-      clear_end(c);
     }
   if (before != me.x) {
 #pragma unroll
@@ -936,11 +936,9 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
         put(me.y, k, v);
       }
     }
-    clear_end(me.y);
     for (int c = me.y + 1; c < tile.hi; ++c) {
 #pragma unroll
       for (int k = 0; k < NIN; ++k) put(c, k, zero);
-      clear_end(c);
     }
   }
 }
@@ -1491,8 +1489,6 @@ int run_mode(const XpDev& d, cudaStream_t s) {
   int dev = 0, sms = 148;
   CCFJ_CUDA_TRY(cudaGetDevice(&dev));
   CCFJ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (ITYPE == 1)
-    CCFJ_CUDA_TRY(cudaMemsetAsync(d.ends, 0, (size_t)(d.blocks_cap / kGroup), s));
   prof_begin(s);
   const int by = std::max(1, std::min(d.cells_cap, 16 * sms / d.mtiles));
   xp_basis_kernel<MODE, ITYPE><<<dim3(d.mtiles, by), kTileRows, 0, s>>>(d);
