@@ -18,6 +18,10 @@
 // * whiten: X / max(|X|, 1e-8) in float32, as the reference;
 // * gram_step: one thread's share of a 16 x 16 station tile of
 //   conj(X_a) X_b for one frequency lane.
+//
+// The device kernel transforms a folded window where it can: with g the
+// common divisor of the bins' stride and M, the bins of x at multiples of g
+// are all the bins of the 2M/g samples sum_t x[n + 2M t/g].
 #pragma once
 
 #include <math.h>
@@ -134,45 +138,69 @@ CC_HD void dft<5>(Cpx* v) {
 // After the last pass (Ns R = M) dst holds the DFT in natural order. The
 // load and the rest are separate so that a caller can run the pass in place
 // (every load before any store).
-template <int R>
-CC_HD void bf_load(const Cpx* src, int M, int t, Cpx* v) {
+// src and dst are pointers or anything that indexes like one (the device
+// kernel's skewed shared array).
+template <int R, class Src>
+CC_HD void bf_load(Src src, int M, int t, Cpx* v) {
   const int stride = M / R;
 #pragma unroll
   for (int r = 0; r < R; ++r) v[r] = src[t + r * stride];
 }
 
-// w[r] = tw[r step] for 0 < r < R: the table entries of step, 2 step and
-// (radix 8) 4 step, the other powers as products of those (one or two
-// products deep). The twiddle indices of neighbouring butterflies lie far
-// apart in the table, so fewer reads mean fewer cache wavefronts.
+// The twiddles w[r] = w[1]^r of a butterfly, 0 < r < R, from the powers that a
+// table holds: 1, 2 and (radix 8) 4; the others as products of those (one or
+// two products deep).
 template <int R>
-CC_HD void twiddle_powers(const Cpx* tw, int step, Cpx* w) {
-  w[1] = tw[step];
-  if (R >= 3) w[2 % R] = tw[2 * step];
+CC_HD void twiddle_powers(Cpx* w) {
   if (R >= 4) w[3 % R] = cmul(w[1], w[2 % R]);
   if (R == 5) w[4 % R] = cmul(w[2 % R], w[2 % R]);
   if (R == 8) {
-    w[4 % R] = tw[4 * step];
     w[5 % R] = cmul(w[4 % R], w[1]);
     w[6 % R] = cmul(w[4 % R], w[2 % R]);
     w[7 % R] = cmul(w[4 % R], w[3 % R]);
   }
 }
 
-template <int R>
-CC_HD void bf_finish(Cpx* dst, int M, int Ns, const Cpx* tw, int t, Cpx* v) {
-  const int jn = t % Ns;
+// Powers that the table of a pass holds
+CC_HD constexpr int twiddle_rows(int R) { return R == 8 ? 3 : R >= 3 ? 2 : 1; }
+
+// Butterfly t = tq Ns + jn with its twiddles (unread for jn = 0)
+template <int R, class Dst>
+CC_HD void bf_twiddled(Dst dst, int Ns, int tq, int jn, const Cpx* w, Cpx* v) {
   if (jn != 0) {
-    const int step = (M / (Ns * R)) * jn;
-    Cpx w[R];
-    twiddle_powers<R>(tw, step, w);
 #pragma unroll
     for (int r = 1; r < R; ++r) v[r] = cmul(v[r], w[r]);
   }
   dft<R>(v);
-  const int base = (t / Ns) * Ns * R + jn;
+  const int base = tq * Ns * R + jn;
 #pragma unroll
   for (int r = 0; r < R; ++r) dst[base + r * Ns] = v[r];
+}
+
+// From the pass's own table, whose row i holds the powers 2^i of its Ns
+// twiddles: neighbouring butterflies read neighbouring entries.
+template <int R, class Dst>
+CC_HD void bf_rows(Dst dst, int Ns, int tq, int jn, const Cpx* rows, Cpx* v) {
+  Cpx w[R];
+  if (jn != 0) {
+#pragma unroll
+    for (int i = 0; i < twiddle_rows(R); ++i) w[1 << i] = rows[i * Ns + jn];
+    twiddle_powers<R>(w);
+  }
+  bf_twiddled<R>(dst, Ns, tq, jn, w, v);
+}
+
+// The same from the one table tw[u] = exp(-2 pi i u / M) of every pass
+template <int R>
+CC_HD void bf_finish(Cpx* dst, int M, int Ns, const Cpx* tw, int t, Cpx* v) {
+  const int jn = t % Ns;
+  const int step = (M / (Ns * R)) * jn;
+  Cpx w[R];
+  if (jn != 0) {
+    for (int i = 0; i < twiddle_rows(R); ++i) w[1 << i] = tw[step << i];
+    twiddle_powers<R>(w);
+  }
+  bf_twiddled<R>(dst, Ns, t / Ns, jn, w, v);
 }
 
 // Radices of a self-sorting plan for M points: 8s, then a 4 or 2, then 3s
@@ -207,7 +235,8 @@ CC_HD int fft_plan(int M, int* radix) {
 
 // Bin k (0 <= k <= M) of the real FFT of 2M samples from the complex FFT Z
 // of z[m] = x[2m] + i x[2m+1]; wk = exp(-i pi k / M).
-CC_HD Cpx real_bin(const Cpx* Z, int M, int k, Cpx wk) {
+template <class Src>
+CC_HD Cpx real_bin(Src Z, int M, int k, Cpx wk) {
   const Cpx a = Z[k == M ? 0 : k];
   const Cpx b = cconj(Z[k == 0 ? 0 : M - k]);
   const Cpx s = cscale(cadd(a, b), 0.5f);
@@ -259,34 +288,75 @@ CC_HD int pair_count(int lo_a, int hi_a, int lo_b, int hi_b) {
 
 // --------------------------------------------------------- pair products
 // Station tiles of kTile x kTile and kLanes frequencies; a CTA of
-// kGramThreads threads: warp w owns tile rows 2w and 2w+1, lane j frequency
-// j of the tile, and every column b.
+// kGramThreads threads: warp w owns tile rows 4w .. 4w+3, lane j frequency
+// j of the tile, and every column b. Four rows by sixteen columns read 20
+// values of shared memory for 64 products (two rows read 18 for 32).
 constexpr int kTile = 16;
 constexpr int kLanes = 32;
-constexpr int kGramThreads = 256;
-constexpr int kRowsPerWarp = kTile / (kGramThreads / 32);  // 2
+constexpr int kGramThreads = 128;
+constexpr int kRowsPerWarp = kTile / (kGramThreads / 32);  // 4
 
-// One shift: xa = the tile's a rows [kTile][kLanes], xb its b rows.
+// acc += conj(a) x, the two halves of each step as a pair: (re, im) gains
+// a.re (x.re, x.im), then a.im (x.im, -x.re). On the device a pair is one packed
+// instruction of two fused multiply-adds, and the operands are built once for
+// the products that share them.
+#if defined(__CUDA_ARCH__)
+typedef unsigned long long Two;
+__device__ __forceinline__ Two two(float lo, float hi) {
+  Two v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void fma_two(Cpx& acc, Two p, Two q) {
+  Two c = two(acc.re, acc.im);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(p), "l"(q));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(acc.re), "=f"(acc.im) : "l"(c));
+}
+#else
+typedef Cpx Two;
+CC_HD Two two(float lo, float hi) { return cpx(lo, hi); }
+CC_HD void fma_two(Cpx& acc, Two p, Two q) {
+  acc.re += p.re * q.re;
+  acc.im += p.im * q.im;
+}
+#endif
+
+// One shift: xa = the tile's a rows [kTile][kLanes], xb its b rows. halves:
+// bit h = columns 8h .. 8h+7 are wanted.
 CC_HD void gram_step(const Cpx* xa, const Cpx* xb, int warp, int lane,
-                     Cpx (&acc)[kRowsPerWarp][kTile]) {
+                     Cpx (&acc)[kRowsPerWarp][kTile], unsigned halves = 3u) {
+  Two re[kRowsPerWarp], im[kRowsPerWarp];
 #pragma unroll
   for (int ra = 0; ra < kRowsPerWarp; ++ra) {
     const Cpx a = xa[(warp * kRowsPerWarp + ra) * kLanes + lane];
+    re[ra] = two(a.re, a.re);
+    im[ra] = two(a.im, a.im);
+  }
 #pragma unroll
-    for (int b = 0; b < kTile; ++b) {
+  for (int h = 0; h < 2; ++h) {
+    if (!(halves >> h & 1u)) continue;
+#pragma unroll
+    for (int b = h * kTile / 2; b < (h + 1) * kTile / 2; ++b) {
       const Cpx x = xb[b * kLanes + lane];
-      // conj(a) * x
-      acc[ra][b].re += a.re * x.re + a.im * x.im;
-      acc[ra][b].im += a.re * x.im - a.im * x.re;
+      const Two q = two(x.re, x.im), turned = two(x.im, -x.re);
+#pragma unroll
+      for (int ra = 0; ra < kRowsPerWarp; ++ra) fma_two(acc[ra][b], re[ra], q);
+#pragma unroll
+      for (int ra = 0; ra < kRowsPerWarp; ++ra) fma_two(acc[ra][b], im[ra], turned);
     }
   }
 }
 
 // The stored value of a pair: (initial + sum) / count, the reference's
 // in-place accumulation followed by its division (src/CrossCorr.cpp:122-144).
+// The FP32 quotient as an FP64 product with inv = 1 / count, rounded once more:
+// a quotient of two 24-bit numbers lies at least 2^-49 of itself from the middle
+// between two floats, so the rounding is that of the division.
+CC_HD Cpx pair_value(Cpx init, Cpx sum, double inv) {
+  return cpx((float)((double)(init.re + sum.re) * inv), (float)((double)(init.im + sum.im) * inv));
+}
 CC_HD Cpx pair_value(Cpx init, Cpx sum, int count) {
-  const float n = (float)count;
-  return cpx((init.re + sum.re) / n, (init.im + sum.im) / n);
+  return pair_value(init, sum, 1.0 / (double)count);
 }
 
 }  // namespace xc

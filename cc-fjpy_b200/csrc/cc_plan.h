@@ -24,13 +24,13 @@ namespace ccfj {
 namespace xc {
 
 // Largest half length the shared-memory FFT handles (M complex points in
-// one CTA: 64 KiB, with each thread holding at most M / 512 points of a
-// pass in registers); longer or odd windows, or lengths with a prime factor
+// one CTA, with each of its 128, 256 or 512 threads holding at most 16
+// points of a pass in registers); longer or odd windows, or lengths with a prime factor
 // above 5, take the direct transform of the requested bins.
 constexpr int kMaxM = 8192;
-constexpr int kFftThreads = 512;
+constexpr int kFftPoints = 16;  // most points of a thread in a pass
 // Shifts staged per step of the pair-product kernel
-constexpr int kShiftChunk = 4;
+constexpr int kShiftChunk = 2;
 // Largest station count (the pair lookup is nsta x nsta)
 constexpr int kMaxStations = 16384;
 
@@ -49,6 +49,7 @@ struct Plan {
   long long nshifts = 0;   // windows per station
   bool stockham = false;   // shared-memory FFT (else direct transform)
   int M = 0;               // F / 2 for the shared-memory FFT
+  bool every_pair = true;  // every pair shares a window
   int npass = 0;
   int radix[kMaxPasses] = {};
   int ldj = 0;             // row length of the spectra (nf rounded up to 32)
@@ -129,6 +130,7 @@ inline int make_plan(const ccfj_cc_args& a, Plan* p, std::string* err) {
     p->pnext[q] = p->pmap[key];
     p->pmap[key] = q;
     used[(size_t)(s0 / kTile) * ntile + s1 / kTile] = 1;
+    if (pair_count(p->lo[s0], p->hi[s0], p->lo[s1], p->hi[s1]) == 0) p->every_pair = false;
   }
   p->tiles.clear();
   for (int ta = 0; ta < ntile; ++ta)
