@@ -133,12 +133,23 @@ __device__ __forceinline__ void spec_pass(Skew s, int M, int& Ns, const Cpx*& tw
   Ns *= R;
 }
 
+// sum += v, what the rounding loses into low.
+__device__ __forceinline__ void add_exact(float& sum, float& low, float v) {
+  const float t = sum + v, b = t - sum;
+  low += (sum - (t - b)) + (v - b);
+  sum = t;
+}
+__device__ __forceinline__ void add_exact(Cpx& sum, Cpx& low, Cpx v) {
+  add_exact(sum.re, low.re, v.re);
+  add_exact(sum.im, low.im, v.im);
+}
+
 // What bounds it: issue, about half of it the passes (index arithmetic, twiddles
 // and transforms), then the reads of the overlapping windows (each sample once
 // per window that holds it, from L2). Both shrink when the wanted bins lie
 // fstride apart: the window is folded to 2M samples on load (SpecJob::fold parts
-// added, more than four in FP64 so that a long sum rounds no worse than the
-// passes that it replaces), which leaves the transform of the wanted bins
+// added, with the roundings carried along or, more than four, in FP64, so that
+// the sum rounds once), which leaves the transform of the wanted bins
 // alone. 100 stations x 51 windows of 14400 samples, every third bin: 317 us
 // without the fold, 135 with it, 119 with each pass's twiddles in their own rows
 // (one table of all had a line per lane), 105 with samples loaded in pairs.
@@ -173,7 +184,11 @@ __global__ void __launch_bounds__(T, 1024 / T) xc_spectra_kernel(SpecJob j) {
       Cpx a[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) a[u] = u < j.fold ? samples(at + u * F2) : cpx(0.f, 0.f);
-      s[m] = cadd(cadd(a[0], a[1]), cadd(a[2], a[3]));
+      Cpx sum = a[0], low = cpx(0.f, 0.f);
+      if (j.fold > 1) add_exact(sum, low, a[1]);
+      if (j.fold > 2) add_exact(sum, low, a[2]);
+      if (j.fold > 3) add_exact(sum, low, a[3]);
+      s[m] = cadd(sum, low);
     }
   } else {
     for (int m = threadIdx.x; m < j.M; m += T) {
