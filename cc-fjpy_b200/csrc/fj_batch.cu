@@ -533,20 +533,32 @@ int batch_device_graph(const ccfj_batch_args& a, long long total, cudaStream_t s
         CCFJ_CUDA_TRY(cudaStreamCreateWithFlags(&g_capture_stream[dev], cudaStreamNonBlocking));
       cap = g_capture_stream[dev];
     }
-    cudaGraph_t graph = nullptr;
-    CCFJ_CUDA_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-    const int st = batch_device(a, total, batch_expands(a, total), cap);
-    const cudaError_t e = cudaStreamEndCapture(cap, &graph);
-    if (st != CCFJ_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      return st;
-    }
-    if (e != cudaSuccess)
-      return set_error(CCFJ_ERR_CUDA, "ccfj_fj_batch_v1: graph capture failed: %s",
-                       cudaGetErrorString(e));
     GraphEntry ge;
-    const cudaError_t ei = cudaGraphInstantiate(&ge.exec, graph, 0);
-    cudaGraphDestroy(graph);
+    cudaError_t ei = cudaSuccess;
+    // A graph's scratch gets its memory at the upload: where that is not to be
+    // had with the expansion's workspace (up to twice the direct kernels'
+    // interval data), the graph is made again without it.
+    for (bool expand = batch_expands(a, total);; expand = false) {
+      cudaGraph_t graph = nullptr;
+      CCFJ_CUDA_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
+      const int st = batch_device(a, total, expand, cap);
+      const cudaError_t e = cudaStreamEndCapture(cap, &graph);
+      if (st != CCFJ_OK) {
+        if (graph) cudaGraphDestroy(graph);
+        return st;
+      }
+      if (e != cudaSuccess)
+        return set_error(CCFJ_ERR_CUDA, "ccfj_fj_batch_v1: graph capture failed: %s",
+                         cudaGetErrorString(e));
+      ei = cudaGraphInstantiate(&ge.exec, graph, 0);
+      cudaGraphDestroy(graph);
+      if (ei == cudaSuccess && expand) {
+        ei = cudaGraphUpload(ge.exec, cap);
+        if (ei != cudaSuccess) cudaGraphExecDestroy(ge.exec);
+      }
+      if (ei != cudaErrorMemoryAllocation || !expand) break;
+      cudaGetLastError();
+    }
     if (ei != cudaSuccess)
       return set_error(CCFJ_ERR_CUDA, "ccfj_fj_batch_v1: graph instantiation failed: %s",
                        cudaGetErrorString(ei));

@@ -1426,7 +1426,14 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   // No column that the plan takes (xp_columns_kernel) has more cells than this.
   const double most = std::max((double)p.total * p.nc * d.nsrc * 250.0, kAnyCost / p.nf_all) /
                       (kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0));
-  d.cells_cap = (int)std::min<double>(kMaxCells, 2 * kGroup + kDyadic + most) & ~(kGroup - 1);
+  // Nor does W get more than the direct kernels' interval data and 512 MiB (all
+  // cells of 4096 frequencies): of more frequencies, those with many cells go
+  // direct. By the whole problem's sizes, for its windows to decide alike.
+  const double fit = ((double)p.total * p.nf_all * 16 + (512 << 20)) / (kBlockFloats * 4) /
+                     div_up(p.nf_all, kTileCols);
+  d.cells_cap = (int)std::min({(double)kMaxCells, 2 * kGroup + kDyadic + most,
+                               batch ? (double)kMaxCells : std::max(64.0, fit)}) &
+                ~(kGroup - 1);
   const long long ntile = (long long)p.nsets * d.ft;
   long long cells = ntile * d.cells_cap;
   if (batch) {

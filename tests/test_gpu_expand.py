@@ -213,3 +213,13 @@ def test_batch_of_uneven_sets(lib, func, itype):
             top = np.abs(z).max(axis=0)
             assert np.abs(y - z / top).max() <= TOL
     assert not all(np.array_equal(y, d, equal_nan=True) for y, d in zip(ys, direct))
+
+
+def test_many_frequencies():
+    """More frequencies than W has room for all cells of: those with many cells
+    go direct, in a window of the frequencies as in the whole call."""
+    case = _case(400, 9001, 257, seed=17, rmax=1.2e5, fmax=14.0)
+    full = _run(case)
+    _check(full, _run(case, precision=1))
+    for a, b in ((0, 64), (8000, 9001)):
+        assert np.array_equal(_run(case, cols=(a, b)), full[:, a:b])
