@@ -139,6 +139,13 @@ __global__ void __launch_bounds__(tc::kThreads, 2) fj_mw_tc_kernel(MwTcDev a) {
   const int fi = blockIdx.y;
   const int c0 = blockIdx.x * tc::kThreads;
   const int ci = min(c0 + tid, a.nc - 1);
+  // Warps of the last tile whose rows all lie past the last velocity generate
+  // nothing: a row of A enters its own row of the accumulators alone, and that
+  // is not read. 400 records x 32 windows x 512 f x 800 c (25 of 32 warps live):
+  // 1072 -> 1044 us; a tile of one warp still takes most of a full one's time,
+  // which is the chain of its intervals.
+  const bool live = c0 + (tid & ~31) < a.nc;
+  const int halves = c0 + 128 < a.nc ? 2 : 1;  // accumulators with a velocity
   unsigned char* sA = smem;
   unsigned char* sB = smem + 2 * TcSmem::kABytesStage;
   const int bstage = TcSmem::b_bytes_stage(a.N);
@@ -238,7 +245,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2) fj_mw_tc_kernel(MwTcDev a) {
       }
     };
 #pragma unroll 1
-    for (int j4 = 0; j4 < tc::kChunkI; j4 += 4) {
+    for (int j4 = live ? 0 : tc::kChunkI; j4 < tc::kChunkI; j4 += 4) {
       __half2 hi[4], lo[4];
 #pragma unroll
       for (int jj = 0; jj < 4; jj += 2) {
@@ -309,7 +316,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2) fj_mw_tc_kernel(MwTcDev a) {
       } else {
         unsigned char* bHi = sB + s * bstage;
         unsigned char* bLo = bHi + tc::kSlices * a.N * 32;
-        for (int m = 0; m < 2; ++m) {
+        for (int m = 0; m < halves; ++m) {
           unsigned char* ah = sA + s * TcSmem::kABytesStage + m * (2 * tc::kSlices * tc::kSliceBytes128);
           unsigned char* al = ah + tc::kSlices * tc::kSliceBytes128;
           const uint32_t d = tmem + (uint32_t)(m * a.N);  // accumulator m: columns [m N, (m+1) N)
@@ -358,7 +365,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2) fj_mw_tc_kernel(MwTcDev a) {
     const uint32_t tbase = tmem + ((uint32_t)(tid & 96) << 16) + (uint32_t)(mh * a.N);
     const int c = c0 + tid;
     const float inv_sa = 1.0f / sa;  // exact: a power of two
-    for (int col = 0; col < a.N; col += 16) {
+    for (int col = live ? 0 : a.N; col < a.N; col += 16) {
       float v[16];
       tc::tmem_ld16(tbase + (uint32_t)col, v);
       if (c < a.nc) {
