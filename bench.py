@@ -9,8 +9,8 @@ complex64 spectra from the c(f) law with a first overtone and sigma = 0.2
 noise (tests/cases.py). Metric: F-J terms per second, terms = nf * nc * npairs.
 
   value   inputs resident in HBM; one step = the full device transform
-          (gather by the sort permutation, interval preparation, the FP32
-          station-amortised kernel, per-frequency normalisation)
+          (gather by the sort permutation, the wave-cell expansion's moments,
+          basis and product, per-frequency normalisation)
   e2e     the same metric through the public API ccfj.fj_noise on host
           numpy arrays (host->device copy of the spectra and device->host copy
           of the result inside the timed region)
@@ -26,7 +26,7 @@ FP64 oracle and the reference's own FJcpu.cpp output (sampled columns):
   4  MWFJ, 1000 traces x 16384 samples, 64 windows, nf 1024, nc 2000
      (tensor cores)
   5  ragged batch, 512 subarrays (50-20,000 pairs each), nf 1024, nc 500, one
-     persistent graph-replayed launch
+     graph-replayed call
 
   --impl reference   times the reference's own CPU implementation
           (src/ccfj.pyx over src/FJcpu.cpp with OpenMP, built into
@@ -62,13 +62,12 @@ for _p in (os.path.join(REPO, "oracle"), os.path.join(REPO, "tests"),
 
 METRIC = "F-J terms/s (nf·nc·npairs), FP32/batched vs FP64 GPU form at ≤1e-4 rel err"
 NPAIRS, NF, NC = 19900, 2048, 1000
-# Algorithmic FLOPs per (f, c, pair) term, FMA = 2, special-function unit
-# operations not counted: a station evaluation E (J0 and J1 with a shared
-# phase, the Struve remainder, the B(x) combine) and an interval combine A
-# per real input.
-FLOPS_E1, FLOPS_A1 = 104, 24     # itype 1
-FLOPS_PER_TERM_ITYPE1 = FLOPS_E1 + FLOPS_A1
+# Algorithmic FLOPs of a station evaluation (itype 1: J0 and J1 with a shared
+# phase, the Struve remainder, the B(x) combine), FMA = 2, special-function
+# unit operations not counted.
+FLOPS_E1 = 104
 FALLBACK_BF16_TFLOPS = 1590.0
+FALLBACK_HBM_GBS = 6650.0
 
 
 # ------------------------------------------------------------- workloads
@@ -89,7 +88,7 @@ def config_dict():
     return {"workload": "fj_noise large array: %d pairs (200 stations, 300x300 km), nf=%d over "
                         "0.005-2 Hz, nc=%d over 500-5000 m/s, itype=1, func=0" % (NPAIRS, NF, NC),
             "npairs": NPAIRS, "nf": NF, "nc": NC, "itype": 1, "func": 0,
-            "l2": "inputs larger than L2 (326 MB complex64 spectra + 326 MB interval data)",
+            "l2": "inputs larger than L2 (326 MB complex64 spectra)",
             "parallelism": "one GPU per rank, independent workloads"}
 
 
@@ -424,6 +423,28 @@ def _fp32_roofline(flops, kernel_s, peak, kernel, flops_per_term, traffic=None):
             "peak_source": "FP32 FMA probe at bench time (ccfj_fp32_peak_probe), measured"}
 
 
+def hbm_peak():
+    """Measured copy bandwidth in GB/s (read + write), else the pool's fallback."""
+    try:
+        with open(os.path.join(REPO, "MEASURED_PEAKS.json")) as fh:
+            return float(json.load(fh)["hbm_gbs"]), "MEASURED_PEAKS.json hbm_gbs (measured)"
+    except (OSError, ValueError, KeyError, TypeError):
+        return FALLBACK_HBM_GBS, "fallback 6650 GB/s (MEASURED_PEAKS.json absent)"
+
+
+def _expansion_roofline(nbytes, call_s, kernel_s=None):
+    """The expansion evaluates the special functions once per cell and
+    velocity, not once per term, so a rate of terms says nothing about the
+    FP32 pipe. What a call cannot do without is the inputs read once and the
+    result written once: its share of the measured copy bandwidth."""
+    peak, source = hbm_peak()
+    ach = nbytes / call_s / 1e9
+    return {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
+            "bytes": int(nbytes), "kernel": "wave-cell expansion (basis, moments, join, tf32 "
+            "product); the call is bound by the moments' issue and the product, not by memory",
+            "kernel_ms": None if kernel_s is None else kernel_s * 1e3, "peak_source": source}
+
+
 def profile_traffic(name):
     """DRAM bytes per launch of a kernel from a committed ncu summary under
     profiles/ (the line 'traffic_bytes_per_launch: <bytes>'), or None."""
@@ -437,10 +458,6 @@ def profile_traffic(name):
             except ValueError:
                 return None
     return None
-
-
-def traffic_per_launch():
-    return profile_traffic("fj_amortized_config2.md")
 
 
 # ------------------------------------------------------------ the configs
@@ -512,16 +529,14 @@ def measure_small(lib, torch, dev, sp, peak, args):
                     "300 c (1000-5000 m/s), sigma 0.1", "unit": "terms/s",
         "value": terms / s, "ms_per_call": s * 1e3, "gpu_launches_per_call": launches,
         "clocks": clocks,
-        "tile_choice": {"velocities_per_thread": cpt.value, "station_ranges": nsplit.value,
+        "tile_choice": {"of": "the direct kernels, for columns the expansion leaves",
+                        "velocities_per_thread": cpt.value, "station_ranges": nsplit.value,
                         "source": "ccfj_autotune_fj_v1 (best of 1/2/4 velocities per thread x "
                                   "1-8 station ranges, %.3f ms)" % best_ms.value},
         "e2e": {"value": terms / te, "unit": "terms/s", "ms_per_call": te * 1e3,
                 "h2d_bytes_per_step": int(uf.nbytes + r.nbytes + 8 * nr + 4 * (nf + nc)),
                 "d2h_bytes_per_step": int(ye.nbytes)},
-        "roofline": _fp32_roofline(FLOPS_PER_TERM_ITYPE1 * terms, ks, peak,
-                                   "fj_amortized_kernel<MODE_J, 1, float, %d>" % cpt.value,
-                                   FLOPS_PER_TERM_ITYPE1,
-                                   traffic=profile_traffic("fj_split_small_array.md")),
+        "roofline": _expansion_roofline(uf.nbytes + 4 * nc * nf, s, ks),
         "accuracy": {"max_abs_err_vs_fp64_normalised": _err(y32, y64),
                      "nan_positions_equal_fp64": _nan_equal(y32, y64),
                      "fp64_sample": "all 300 x 512 cells", "e2e_equals_device": bool(
@@ -578,7 +593,6 @@ def measure_eq(lib, torch, dev, sp, peak, args):
     y64 = out.cpu().numpy()
     terms = ntr * nf * nc
     te, ye = _time_host_calls(lambda: _quiet(ccfj.fj_earthquake, u, r, c, f), 5, 2)
-    fpt = FLOPS_E1 + 2 * FLOPS_A1
     run.res = {
         "workload": "fj_earthquake itype=1 func=0 with the device rFFT: 500 traces x 8192 "
                     "samples at 20 Hz (r 10-2000 km), bins 0-1023, nc=800 (2000-5000 m/s)",
@@ -587,9 +601,7 @@ def measure_eq(lib, torch, dev, sp, peak, args):
         "e2e": {"value": terms / te, "unit": "terms/s", "ms_per_call": te * 1e3,
                 "h2d_bytes_per_step": int(u.nbytes + 4 * ntr + 8 * ntr + 4 * (nf + nc)),
                 "d2h_bytes_per_step": int(ye.nbytes)},
-        "roofline": _fp32_roofline(fpt * terms, ks, peak,
-                                   "fj_amortized_kernel<MODE_ABS_J, 1, float, 2> (Re and Im "
-                                   "share each station evaluation)", fpt),
+        "roofline": _expansion_roofline(u.nbytes + 4 * nc * nf, s, ks),
         "accuracy": {"max_abs_err_vs_fp64_normalised": _err(y32, y64),
                      "nan_positions_equal_fp64": _nan_equal(y32, y64),
                      "fp64_sample": "all 800 x 1024 cells (the f = 0 column is NaN in every "
@@ -744,7 +756,7 @@ def cpu_mwfj(run, ref, threads):
 
 
 def measure_batch(lib, torch, dev, sp, peak, args):
-    """Configuration 5 (ragged batch, one persistent graph-replayed launch)."""
+    """Configuration 5 (ragged batch, one graph-replayed call)."""
     import ccfj
     from ccfj import _lib, _batch
     run = ConfigRun(5)
@@ -840,7 +852,7 @@ def measure_batch(lib, torch, dev, sp, peak, args):
     run.res = {
         "workload": "%d subarrays, %d pairs in total (log-uniform 50-20000 each, r 0.5-300 km), "
                     "nf=1024 (0.01-1 Hz), nc=500 (1000-5000 m/s), itype=1 func=0; one "
-                    "persistent graph-replayed launch" % (nsets, total),
+                    "graph-replayed call" % (nsets, total),
         "unit": "terms/s", "value": terms / s, "ms_per_call": s * 1e3,
         "gpu_launches_per_call": launches, "clocks": clocks,
         "separate_launches_ms": t_sep * 1e3, "speedup_vs_separate_launches": t_sep / s,
@@ -849,9 +861,7 @@ def measure_batch(lib, torch, dev, sp, peak, args):
                                           + 4 * (nf + nc)),
                 "d2h_bytes_per_step": int(4 * nsets * nc * nf),
                 "note": "spectra in pinned host memory, one view per subarray"},
-        "roofline": _fp32_roofline(FLOPS_PER_TERM_ITYPE1 * terms, s, peak,
-                                   "fj_batch_persistent_kernel<MODE_J, 1, 2> (time of the whole "
-                                   "graph replay)", FLOPS_PER_TERM_ITYPE1),
+        "roofline": _expansion_roofline(8 * total * nf + 4 * nsets * nc * nf, s),
         "accuracy": {"max_abs_err_vs_fp64_normalised": float(max(errs)),
                      "nan_positions_equal_fp64": bool(nan_ok),
                      "fp64_sample": "all %d subarrays, every cell (FP64 form: %.1f s)" % (nsets,
@@ -1047,7 +1057,7 @@ def run_ours(args, rank, world):
     peak = ctypes.c_double(0)
     _lib.check(lib.ccfj_fp32_peak_probe(sp, ctypes.byref(peak)))
     peak = peak.value
-    achieved = FLOPS_PER_TERM_ITYPE1 * terms / (kern_ms / 1e3) / 1e12
+    roofline = _expansion_roofline(uf.nbytes + 4 * NC * NF, t / args.steps, kern_ms / 1e3)
     bf16 = bf16_peak()
 
     runs = []
@@ -1060,10 +1070,7 @@ def run_ours(args, rank, world):
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic (seeded; spectra from the c(f) dispersion law)",
             "config": config_dict(), "e2e": e2e, "clocks": clocks, "gpu_launches": int(launches),
-            "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                         "frac": achieved / peak, "traffic": traffic_per_launch(),
-                         "kernel": "fj_amortized_kernel<MODE_J, itype 1, float>",
-                         "kernel_ms": kern_ms, "flops_per_term": FLOPS_PER_TERM_ITYPE1},
+            "roofline": roofline,
             "accuracy": {"max_abs_err_vs_fp64_normalised": err}}))
         return 0
     if not args.headline_only:
@@ -1136,14 +1143,7 @@ def run_ours(args, rank, world):
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic (seeded; spectra from the c(f) dispersion law)",
         "config": config_dict(), "e2e": e2e,
-        "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak,
-                     "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic_per_launch(),
-                     "kernel": "fj_amortized_kernel<MODE_J, itype 1, float>",
-                     "kernel_ms": kern_ms,
-                     "flops_per_term": FLOPS_PER_TERM_ITYPE1,
-                     "peak_source": "measured at bench time: FP32 FMA probe "
-                                    "(ccfj_fp32_peak_probe); MEASURED_PEAKS.json has no FP32 "
-                                    "figure"},
+        "roofline": roofline,
         "cpu_baseline": cpu,
         "clocks": clocks,
         "gpu_launches": int(launches),
