@@ -152,7 +152,8 @@ __device__ __forceinline__ void add_exact(Cpx& sum, Cpx& low, Cpx v) {
 // the sum rounds once), which leaves the transform of the wanted bins
 // alone. 100 stations x 51 windows of 14400 samples, every third bin: 317 us
 // without the fold, 135 with it, 119 with each pass's twiddles in their own rows
-// (one table of all had a line per lane), 105 with samples loaded in pairs.
+// (one table of all had a line per lane), 105 with samples loaded in pairs; the
+// carried roundings add 8.
 template <int T>
 __global__ void __launch_bounds__(T, 1024 / T) xc_spectra_kernel(SpecJob j) {
   extern __shared__ Cpx smem[];  // [skewed(M)]
