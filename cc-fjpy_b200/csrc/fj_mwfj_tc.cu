@@ -20,8 +20,8 @@
 // slope column uses I1 / (k s) against the spectrum difference g2 - g1
 // (s = max(r2 - r1, 0.1), so that (I1 / k) b = (I1 / (k s)) (g2 - g1)).
 //
-// CTA: 256 threads = 256 velocities (two M = 128 accumulators), one
-// frequency, all windows (N = 2 nwin padded to a multiple of 16, <= 256).
+// CTA: 256 threads = 256 velocities (two M = 128 accumulators; or one of 128
+// where that pads the velocities less), one frequency, all windows (N = 2 nwin padded to a multiple of 16, <= 256).
 // Per chunk of 16 intervals (K = 32): every thread writes its 32 A values
 // (hi and lo) into shared memory in the K-major, no-swizzle canonical
 // layout; one thread waits for the chunk's B (a 1-D bulk copy, issued two
@@ -31,6 +31,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "fj_cells.cuh"
 #include "fj_fft.cuh"
 #include "fj_tcgen05.cuh"
@@ -39,7 +41,7 @@ namespace ccfj {
 
 namespace tc {
 
-constexpr int kThreads = 256;       // velocities per CTA (2 x M = 128)
+constexpr int kThreads = 256;       // velocities per CTA (2 x M = 128), or half of it
 constexpr int kChunkI = 16;         // intervals per chunk
 constexpr int kChunkK = 2 * kChunkI;  // K per chunk (I0 and I1/k per interval)
 constexpr int kSlices = kChunkK / 16;  // MMA K = 16 for 16-bit operands
@@ -110,14 +112,16 @@ struct MwTcDev {
 };
 
 // Shared-memory layout of one CTA (dynamic):
-//   A[stage][half m][hi/lo][slice] 128 rows x 16 K fp16   2*2*2*2*4096 = 64 KB
+//   A[stage][half m][hi/lo][slice] 128 rows x 16 K fp16   2*(T/128)*2*2*4096: 64 or 32 KB
 //   B[stage][hi/lo][slice]         N rows x 16 K fp16     2*2*2*(N*32) B
 //   barriers, tmem address
 struct TcSmem {
-  static constexpr int kABytesStage = 2 * 2 * tc::kSlices * tc::kSliceBytes128;
+  __host__ __device__ static constexpr int a_bytes_stage(int T) {
+    return T / 128 * 2 * tc::kSlices * tc::kSliceBytes128;
+  }
   __host__ __device__ static int b_bytes_stage(int N) { return 2 * tc::kSlices * N * 32; }
-  __host__ __device__ static int total(int N) {
-    return 2 * kABytesStage + 2 * b_bytes_stage(N) + 64;
+  __host__ __device__ static int total(int N, int T) {
+    return 2 * a_bytes_stage(T) + 2 * b_bytes_stage(N) + 64;
   }
 };
 
@@ -132,12 +136,13 @@ __device__ __forceinline__ int tile_off(int row, int k, int rows) {
 // two stations are evaluated, and the two intervals' moments formed, with
 // paired FP32 instructions (one lane per station); elsewhere, and without
 // PAIRED, one interval at a time.
-template <bool PAIRED>
-__global__ void __launch_bounds__(tc::kThreads, 2) fj_mw_tc_kernel(MwTcDev a) {
+template <bool PAIRED, int T>
+__global__ void __launch_bounds__(T, 512 / T) fj_mw_tc_kernel(MwTcDev a) {
+  constexpr int kAStage = TcSmem::a_bytes_stage(T);
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x;
   const int fi = blockIdx.y;
-  const int c0 = blockIdx.x * tc::kThreads;
+  const int c0 = blockIdx.x * T;
   const int ci = min(c0 + tid, a.nc - 1);
   // Warps of the last tile whose rows all lie past the last velocity generate
   // nothing: a row of A enters its own row of the accumulators alone, and that
@@ -145,9 +150,9 @@ __global__ void __launch_bounds__(tc::kThreads, 2) fj_mw_tc_kernel(MwTcDev a) {
   // 1072 -> 1044 us; a tile of one warp still takes most of a full one's time,
   // which is the chain of its intervals.
   const bool live = c0 + (tid & ~31) < a.nc;
-  const int halves = c0 + 128 < a.nc ? 2 : 1;  // accumulators with a velocity
+  const int halves = T == 256 && c0 + 128 < a.nc ? 2 : 1;  // accumulators with a velocity
   unsigned char* sA = smem;
-  unsigned char* sB = smem + 2 * TcSmem::kABytesStage;
+  unsigned char* sB = smem + 2 * kAStage;
   const int bstage = TcSmem::b_bytes_stage(a.N);
   uint64_t* bar = reinterpret_cast<uint64_t*>(sB + 2 * bstage);  // [0,1] B full, [2,3] MMA done
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 4);
@@ -219,7 +224,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2) fj_mw_tc_kernel(MwTcDev a) {
       }
     }
     // A of this chunk: I0 and I1/k of intervals 1 + 16 kc + j
-    unsigned char* aHi = sA + s * TcSmem::kABytesStage + mh * (2 * tc::kSlices * tc::kSliceBytes128);
+    unsigned char* aHi = sA + s * kAStage + mh * (2 * tc::kSlices * tc::kSliceBytes128);
     unsigned char* aLo = aHi + tc::kSlices * tc::kSliceBytes128;
     // interval i (stations i - 1, i): I0 and I1 / (k s), scaled
     auto one_interval = [&](int i, float& I0, float& I1k) {
@@ -317,7 +322,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2) fj_mw_tc_kernel(MwTcDev a) {
         unsigned char* bHi = sB + s * bstage;
         unsigned char* bLo = bHi + tc::kSlices * a.N * 32;
         for (int m = 0; m < halves; ++m) {
-          unsigned char* ah = sA + s * TcSmem::kABytesStage + m * (2 * tc::kSlices * tc::kSliceBytes128);
+          unsigned char* ah = sA + s * kAStage + m * (2 * tc::kSlices * tc::kSliceBytes128);
           unsigned char* al = ah + tc::kSlices * tc::kSliceBytes128;
           const uint32_t d = tmem + (uint32_t)(m * a.N);  // accumulator m: columns [m N, (m+1) N)
           for (int sl = 0; sl < tc::kSlices; ++sl) {
@@ -595,11 +600,20 @@ int mwfj_tensor(const ccfj_eq_args& a, const float2* spec, cudaStream_t s, Scrat
   d.tau = a.tau > 0 ? a.tau : kDefaultTau32;
   d.wait_cycles = tc::kWaitCycles;
   d.self_test_no_copy = 0;
-  const int smem = TcSmem::total(N);
-  auto* kern = paired ? fj_mw_tc_kernel<true> : fj_mw_tc_kernel<false>;
+  // 128 velocities a CTA where the velocities fill an odd number of such halves
+  // and four CTAs fit an SM's shared memory (N <= 80: 53 KB each), so that as
+  // many warps run as with two CTAs of 256; else 256, which bring B in half as
+  // often. 400 records x 32 windows x 512 f x 800 c: the call 1402 us with 256,
+  // 1279 with 128.
+  const bool narrow = (a.nc - 1) % tc::kThreads < 128 && N <= 80;
+  const int threads = narrow ? 128 : tc::kThreads;
+  d.tmem_cols = narrow ? std::max(32, cols / 2) : cols;
+  const int smem = TcSmem::total(N, threads);
+  auto* kern = narrow ? (paired ? fj_mw_tc_kernel<true, 128> : fj_mw_tc_kernel<false, 128>)
+                      : (paired ? fj_mw_tc_kernel<true, 256> : fj_mw_tc_kernel<false, 256>);
   CCFJ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   prof_begin(s);
-  kern<<<dim3(div_up(a.nc, tc::kThreads), nf), tc::kThreads, smem, s>>>(d);
+  kern<<<dim3(div_up(a.nc, threads), nf), threads, smem, s>>>(d);
   prof_end(s);
   count_launch();
   CCFJ_LAUNCH_CHECK("fj_mw_tc_kernel");
@@ -658,10 +672,10 @@ int mw_tc_self_test(cudaStream_t s, int* status) {
   d.tau = kDefaultTau32;
   d.wait_cycles = 2000000;  // ~1 ms
   d.self_test_no_copy = 1;
-  const int smem = TcSmem::total(N);
-  CCFJ_CUDA_TRY(cudaFuncSetAttribute(fj_mw_tc_kernel<true>,
+  const int smem = TcSmem::total(N, tc::kThreads);
+  CCFJ_CUDA_TRY(cudaFuncSetAttribute(fj_mw_tc_kernel<true, tc::kThreads>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  fj_mw_tc_kernel<true><<<1, tc::kThreads, smem, s>>>(d);
+  fj_mw_tc_kernel<true, tc::kThreads><<<1, tc::kThreads, smem, s>>>(d);
   count_launch();
   CCFJ_LAUNCH_CHECK("fj_mw_tc_kernel (self-test)");
   bool failed = false;
