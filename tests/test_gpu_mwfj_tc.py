@@ -67,6 +67,17 @@ def test_paired_generator_agrees_with_one_interval_at_a_time(ntr, nwin, nc):
         assert O.rel_error(y2[w], y3[w]) <= 1e-5
 
 
+@pytest.mark.parametrize("nwin,nc", [(40, 384), (40, 385), (41, 384), (2, 100), (16, 128)])
+def test_velocity_tiles_of_128_and_256(nwin, nc):
+    """Velocities that end a tile of 128 or begin the next one, windows on both
+    sides of what tiles of 128 take; tolerance as for the paths above."""
+    case = _case(63, 21, nwin, nc=nc)
+    y_tc, y_cc = _run(2, case), _run(1, case)
+    assert np.array_equal(np.isnan(y_tc), np.isnan(y_cc))
+    for w in range(nwin):
+        assert O.rel_error(y_tc[w], y_cc[w]) <= TOL
+
+
 def test_tensor_path_f0_column_is_nan():
     case = _case(77, 20, 16)
     y = _run(2, case)
