@@ -64,6 +64,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "fj_cell.h"
 #include "fj_cells.cuh"
 #include "fj_expand.cuh"
 #include "fj_tcgen05.cuh"
@@ -72,24 +73,18 @@ namespace ccfj {
 
 namespace {
 
+using namespace xp;
+
 constexpr int kNodes = 16;          // Chebyshev terms of a cell
-constexpr double kCellPhase = 9.8;  // radians of a cell at the slowest velocity
 // Cells of one frequency: 2048 are 3190 wavelengths of the slowest velocity.
 // Columns with more go to the direct kernels.
 constexpr int kMaxCells = 2048;
-constexpr int kDyadic = 24;         // halved cells below the first (Y basis)
 constexpr int kTileCols = 128;      // frequencies of a W tile and GEMM column tile
 constexpr int kTileRows = 128;      // velocities of a GEMM tile
 constexpr int kGroup = 4;           // tiles begin and end with groups of cells
 constexpr int kEndRows = 2;         // rows of a cell's end
 constexpr int kEndFloats = kTileCols * kGroup * kEndRows;  // one (tile, group, input) of V
 constexpr int kBlockFloats = kTileCols * kNodes;  // one (tile, cell, input) of W
-// Intervals up to this share of a cell are short: whole in the cell of their
-// far end. A cell's polynomials live on [-kShort, 1] of it; the middle of that
-// is kCentre, and t = (x - middle) kPerHalf.
-constexpr float kShort = 0.0625f;
-constexpr float kCentre = 0.46875f;
-constexpr float kPerHalf = 1.8823529f;
 
 struct XpTile {
   int lo, hi;    // cells [lo, hi) of the tile's columns, whole groups
@@ -159,50 +154,6 @@ __device__ __forceinline__ long long slot_begin(const XpDev& d, int b) {
 }
 __device__ __forceinline__ int chunks_of(const XpDev& d, long long n) {
   return max(1, (int)((n - 1 + d.chunk - 1) / d.chunk));
-}
-
-// ------------------------------------------------------------------ cells
-// x = r f / hu as a double-float product of r and fx = f / hu.
-struct Fx {
-  float hi, lo;
-};
-__device__ __forceinline__ Fx make_fx(float f, double inv_hu) {
-  const double v = __dmul_rn((double)f, inv_hu);  // (not fused: every kernel forms the same fx)
-  Fx x;
-  x.hi = (float)v;
-  x.lo = (float)(v - (double)x.hi);
-  return x;
-}
-
-// The cell that holds x = r f / hu, and x's place in it from kCentre (so that
-// its rounding is smallest, -kCentre .. 1 - kCentre). The cell never decreases
-// with r. DY: the cells below 1 are [2^(i-24), 2^(i-23)).
-template <bool DY>
-__device__ __forceinline__ int locate(float r, Fx fx, float& v) {
-  const float p = __fmul_rn(r, fx.hi);  // (not fused into p - c: l holds its rounding)
-  const float l = fmaf(r, fx.lo, fmaf(r, fx.hi, -p));
-  float c = floorf(p);
-  if ((p - c) + l < 0.0f) c -= 1.0f;
-  if (!DY || c >= 1.0f) {
-    v = (p - (c + kCentre)) + l;
-    return (int)c + (DY ? kDyadic - 1 : 0);
-  }
-  // x < 1: [len, 2 len) with len the power of two at or below x
-  float len = __int_as_float(__float_as_int(p) & 0x7f800000);
-  if (p >= 1.0f) len = 0.5f;  // x just below 1
-  if ((p - len) + l < 0.0f) len *= 0.5f;
-  v = ((p - len * (1.0f + kCentre)) + l) / len;
-  const int e = (__float_as_int(len) >> 23) - 127;  // -24 .. -1
-  return max(e + kDyadic, 0);
-}
-template <bool DY>
-__device__ __forceinline__ float cell_len(int cell) {
-  return DY && cell < kDyadic ? __int_as_float((cell - kDyadic + 127) << 23) : 1.0f;
-}
-template <bool DY>
-__device__ __forceinline__ float cell_begin(int cell) {
-  if (!DY) return (float)cell;
-  return cell < kDyadic ? cell_len<DY>(cell) : (float)(cell - kDyadic + 1);
 }
 
 // ------------------------------------------------------------------- plan
@@ -772,11 +723,10 @@ __global__ void __launch_bounds__(32, NIN == 1 ? 24 : 16) xp_moments_kernel(XpDe
         } else {
           // the station's cell and place, as locate() finds them, from the cell
           // that the lane is in
-          const float p = __fmul_rn(rB, fx.hi);
-          const float l = fmaf(rB, fx.lo, fmaf(rB, fx.hi, -p));
+          const Place x = place_of(rB, fx);
 #pragma unroll 1
-          while ((p - (base_x + 1.0f)) + l >= 0.0f) flush();
-          vB = (p - (base_x + kCentre)) + l;
+          while (reached(x, base_x + 1.0f)) flush();
+          vB = (x.p - (base_x + kCentre)) + x.l;
         }
         if (ITYPE == 0) {
 #pragma unroll
