@@ -355,6 +355,16 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
     if (st != CCFJ_OK) return st;
     in[1] = InDesc{hb, a.nf, 1, nullptr};
   }
+  // The direct kernel's buffers before the expansion's workspace: where there
+  // is no memory for both, the workspace is refused and every column is direct.
+  const size_t esz = a.itype == 1 ? sizeof(StationCoef<float>) : 4;
+  float* kb = a.itype == 1 ? sc.get_n<float>(a.nf) : nullptr;
+  if (a.itype == 1 && !kb) return CCFJ_ERR_ALLOC;
+  void* gbuf[2] = {nullptr, nullptr};
+  for (int j = 0; j < nin; ++j) {
+    gbuf[j] = sc.get((size_t)total * a.nf * esz);
+    if (!gbuf[j]) return CCFJ_ERR_ALLOC;
+  }
   XpProblem xp{};
   XpWork xw{};
   bool expanded = false;
@@ -384,19 +394,14 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
   BatchDev bd{};
   bd.base.other = other;
   const float tau = a.tau > 0 ? a.tau : kDefaultTau32;
-  float* kb = nullptr;
   if (a.itype == 1) {
-    kb = sc.get_n<float>(a.nf);
-    if (!kb) return CCFJ_ERR_ALLOC;
     fj_kbounds_kernel<float><<<div_up(a.nf, 8), dim3(32, 8), 0, s>>>(a.f, a.c, a.nf, a.nc, tau, kb,
                                                                 other);
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_kbounds_kernel");
   }
-  const size_t esz = a.itype == 1 ? sizeof(StationCoef<float>) : 4;
   for (int j = 0; j < nin; ++j) {
-    void* g = sc.get((size_t)total * a.nf * esz);
-    if (!g) return CCFJ_ERR_ALLOC;
+    void* g = gbuf[j];
     const unsigned rows = (unsigned)std::min<long long>(1024, div_up(total, 8));
     batch_prep_u_kernel<<<dim3(rows, div_up(a.nf, 32)), dim3(32, 8), 0, s>>>(
         in[j], a.offsets, a.nsets, total, a.nf, a.r, drs, wtr, geo, kb, a.itype, g, other);

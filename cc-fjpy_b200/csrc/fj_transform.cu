@@ -470,6 +470,33 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
     in[1] = InDesc{hb, a.nf, 1, nullptr};
   }
 
+  // The direct kernels' buffers before the expansion's workspace: where there
+  // is no memory for both, the workspace is refused and every column is direct.
+  void* kb = nullptr;
+  void* gbuf[2] = {nullptr, nullptr};
+  if (amortized) {
+    if (a.itype == 1) {
+      kb = sc.get(kbounds_bytes(a));
+      if (!kb) return CCFJ_ERR_ALLOC;
+    }
+    for (int j = 0; j < nin; ++j) {
+      gbuf[j] = sc.get(interval_data_bytes(a));
+      if (!gbuf[j]) return CCFJ_ERR_ALLOC;
+    }
+  }
+  const int cpt = variant_for(a, cpt_choice);
+  if (a.precision == CCFJ_PREC_FP32) {
+    const int nsplit = split_for(a, cpt, split_choice);
+    if (nsplit > 1) {
+      d.split_len = (int)div_up(div_up(a.nr, nsplit), kSplitAlign) * kSplitAlign;
+      const int n = (int)div_up(a.nr, d.split_len);
+      if (n > 1) {
+        d.part = sc.get_n<float>((size_t)n * nin_of(a.mode) * a.nc * a.nf);
+        if (!d.part) return CCFJ_ERR_ALLOC;
+      }
+    }
+  }
+
   // the expansion plans which columns it takes; the direct kernels below
   // compute the others
   XpProblem xp{};
@@ -508,31 +535,8 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
       plain[j] = g;
     }
   } else {
-    void* kb = nullptr;
-    if (a.itype == 1) {
-      kb = sc.get(kbounds_bytes(a));
-      if (!kb) return CCFJ_ERR_ALLOC;
-    }
-    void* gbuf[2] = {nullptr, nullptr};
-    for (int j = 0; j < nin; ++j) {
-      gbuf[j] = sc.get(interval_data_bytes(a));
-      if (!gbuf[j]) return CCFJ_ERR_ALLOC;
-    }
     const int st = prep_interval_data(a, d, in, nin, kb, gbuf, wtr, s);
     if (st != CCFJ_OK) return st;
-  }
-
-  const int cpt = variant_for(a, cpt_choice);
-  if (a.precision == CCFJ_PREC_FP32) {
-    const int nsplit = split_for(a, cpt, split_choice);
-    if (nsplit > 1) {
-      d.split_len = (int)div_up(div_up(a.nr, nsplit), kSplitAlign) * kSplitAlign;
-      const int n = (int)div_up(a.nr, d.split_len);
-      if (n > 1) {
-        d.part = sc.get_n<float>((size_t)n * nin_of(a.mode) * a.nc * a.nf);
-        if (!d.part) return CCFJ_ERR_ALLOC;
-      }
-    }
   }
   if (!expanded) prof_begin(s);
   switch (a.mode) {
