@@ -199,7 +199,10 @@ void* Scratch::get(size_t bytes) {
     return nullptr;
   }
   void* p = dev_alloc((bytes + 255) & ~size_t(255), s_);
-  if (p) ptrs_[n_++] = p;
+  if (p) {
+    ptrs_[n_++] = p;
+    bytes_ += bytes;
+  }
   return p;
 }
 

@@ -42,11 +42,13 @@ class Scratch {
   T* get_n(size_t n) {
     return static_cast<T*>(get(n * sizeof(T)));
   }
+  size_t bytes() const { return bytes_; }  // got so far
 
  private:
   cudaStream_t s_;
   void* ptrs_[32] = {};
   int n_ = 0;
+  size_t bytes_ = 0;
 };
 
 #define CCFJ_CUDA_TRY(expr)                                                                  \

@@ -1501,11 +1501,30 @@ bool xp_eligible(long long total, int nsets, int nf_all, int nc) {
   return nsets <= 65535 && nf_all <= 65535 * 8 && worth((double)total, (double)nf_all * nc);
 }
 
+// A call that is being captured gets its memory when the graph is launched, too
+// late to do without the workspace. So the workspace has to fit, with what the
+// call has already asked for, into what the device has free now. (What earlier
+// graphs hold and don't use counts as taken: the device still reports it as used
+// after they have run.)
+static bool captured_without_memory(size_t bytes, cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (!s || allocator_hooked() || cudaStreamIsCapturing(s, &cs) != cudaSuccess ||
+      cs == cudaStreamCaptureStatusNone)
+    return false;
+  size_t free_bytes = 0, all = 0;
+  if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return bytes > free_bytes;
+}
+
 int xp_plan(const XpProblem& p, Scratch& sc, cudaStream_t s, XpWork* w, bool* ok) {
   XpDev d;
   *ok = false;
   const size_t bytes = layout(p, nullptr, &d);
   if (d.slots > 0x7fffffffll || d.slots * div_up(p.nf, 32) > 0x7fffffffll) return CCFJ_OK;
+  if (captured_without_memory(bytes + sc.bytes(), s)) return CCFJ_OK;
   void* base = sc.get(bytes);
   if (!base) {
     clear_error();

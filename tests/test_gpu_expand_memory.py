@@ -96,3 +96,55 @@ def test_memory_that_ends_between_the_two_needs(lib, name):
             with Budget(lib, int(limit)):
                 y = call()
             assert np.array_equal(y, full if limit == top else plain), limit
+
+
+def test_captured_call_near_the_device_s_limit(lib):
+    """A caller's graph takes its memory at its launch: a call captured while
+    the device has room for the direct kernels alone still runs."""
+    import torch
+    from ccfj import _lib
+    nr, nf, nc = 400, 4000, 300
+    rng = np.random.default_rng(23)
+    r = np.sort(rng.uniform(500.0, 1e5, nr)).astype(np.float32)
+    f, c = np.linspace(0.02, 1.5, nf, dtype=np.float32), np.linspace(800, 4500, nc, dtype=np.float32)
+    u = rng.standard_normal((nr, nf)).astype(np.float32)
+    T = [torch.from_numpy(x).cuda() for x in (r, f, c, u)]
+    out = torch.empty((nc, nf), device="cuda")
+    a = _lib.FjArgs()
+    a.struct_size = ctypes.sizeof(a)
+    a.nr, a.nf, a.nc, a.itype, a.mode, a.normalize, a.device_ptrs = nr, nf, nc, 1, 0, 1, 1
+    a.r, a.f, a.c, a.out = T[0].data_ptr(), T[1].data_ptr(), T[2].data_ptr(), out.data_ptr()
+    a.u[0], a.u_ld, a.u_rows, a.u_es, a.u_ncols, a.fstride = T[3].data_ptr(), nf, nr, 1, nf, 1
+
+    def captured():
+        s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            _lib.check(lib.ccfj_fj_v1(ctypes.byref(a), ctypes.c_void_p(s.cuda_stream)))
+        out.fill_(float("nan"))
+        g.replay()
+        torch.cuda.synchronize()
+        return out.cpu().numpy()
+
+    def eager():
+        out.fill_(float("nan"))
+        _lib.check(lib.ccfj_fj_v1(ctypes.byref(a), None))
+        torch.cuda.synchronize()
+        return out.cpu().numpy()
+
+    full = eager()
+    try:
+        assert lib.ccfj_set_fj_variant(2) == 0
+        direct = eager()
+    finally:
+        lib.ccfj_set_fj_variant(0)
+    # the direct kernels take 26 MB of interval data, the workspace 895 MB
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    rest = torch.empty(free - (450 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        y = captured()
+    finally:
+        del rest
+        torch.cuda.empty_cache()
+    assert np.array_equal(y, direct)
+    assert np.array_equal(captured(), full)
