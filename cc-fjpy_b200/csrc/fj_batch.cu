@@ -320,10 +320,10 @@ int batch_variant(const ccfj_batch_args& a, long long total) {
 
 // The device sequence of one batch (all pointers device pointers;
 // `total` = offsets[nsets], known to the caller).
-// `expand`: the wave-cell expansion may take columns; total_all: the pairs of
-// the whole batch that these sets are a group of.
+// `expand`: the wave-cell expansion may take columns; total_all, nsets_all: the
+// pairs and sets of the whole batch that these sets are a group of.
 int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStream_t s,
-                 long long total_all = 0) {
+                 long long total_all = 0, int nsets_all = 0) {
   Scratch sc(s);
   const int nin = nin_of_mode(a.mode);
   float* drs = sc.get_n<float>(total + 1);
@@ -387,6 +387,7 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
     xp.normalize = a.normalize;
     xp.nf_all = a.nf;
     xp.total_all = total_all > 0 ? total_all : total;
+    xp.nsets_all = nsets_all > 0 ? nsets_all : a.nsets;
     const int st = xp_plan(xp, sc, s, &xw, &expanded);
     if (st != CCFJ_OK) return st;
     if (expanded) other = Elsewhere{xw.use, xw.left};
@@ -730,7 +731,7 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
     dg.out = dout + (size_t)G.b0 * a.nc * a.nf;
     dg.variant = variant;
     CCFJ_CUDA_TRY(cudaStreamWaitEvent(s, lane.ev[g], 0));
-    st = batch_device(dg, dg.total_pairs, expand, s, total);
+    st = batch_device(dg, dg.total_pairs, expand, s, total, a.nsets);
     if (st != CCFJ_OK) return st;
     if (g + 1 < ng && (st = copy_group(g + 1)) != CCFJ_OK) return st;
   }

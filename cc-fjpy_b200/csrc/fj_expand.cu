@@ -122,6 +122,7 @@ struct XpDev {
   int nsrc, nacc;        // products of a result, results of a column
   int has_ends;          // itype 1: V and Eend are in use
   int cells_cap;
+  int tile_cells;        // a tile of a set of n pairs has at most n / 4 + this many
   long long blocks_cap, units_cap, slots;
   unsigned char* use;
   XpPlan* plan;
@@ -129,6 +130,7 @@ struct XpDev {
   // [nsets * ft] columns of the tile that go direct; kBad: the tile's part of
   // r is out of order, or a velocity is not positive and finite
   int* direct;
+  int* set_bad;          // [nsets] some tile of the set is bad: all its columns go direct
   int* slot_set;         // [slot] the set of a moments chunk
   float* E;              // [basis][cell][velocity tile][128][16]
   float* Eend;           // [basis][group][velocity tile][128][cell of the group][2]
@@ -235,9 +237,6 @@ __global__ void xp_columns_kernel(XpDev d) {
       }
     }
   }
-  if (fi < d.nf) d.use[(long long)b * d.nf + fi] = use;
-  const int left = __syncthreads_count(fi < d.nf && !use);
-  if (t == 0) d.direct[tile] = fine ? left : kBad;
   if (blockIdx.x == 0) {  // the set's slots of moments chunks
     const long long s0 = slot_begin(d, b), s1 = b + 1 < d.nsets ? slot_begin(d, b + 1) : d.slots;
     for (long long s = s0 + t; s < s1; s += kTileCols) d.slot_set[s] = b;
@@ -253,14 +252,24 @@ __global__ void xp_columns_kernel(XpDev d) {
     ired[t >> 5][1] = mx;
   }
   __syncthreads();
+  for (int w = 0; w < kWarps; ++w) {
+    mn = min(mn, ired[w][0]);
+    mx = max(mx, ired[w][1]);
+  }
+  if (mx <= mn) mn = mx = 0;
+  mn &= ~(kGroup - 1);
+  mx = (mx + kGroup - 1) & ~(kGroup - 1);
+  // a tile with more cells than its share of W goes direct (see layout())
+  if (mx - mn > n / 4 + d.tile_cells) {
+    use = false;
+    mn = mx = 0;
+  }
+  if (fi < d.nf) d.use[(long long)b * d.nf + fi] = use;
+  const int left = __syncthreads_count(fi < d.nf && !use);
   if (t == 0) {
-    for (int w = 0; w < kWarps; ++w) {
-      mn = min(mn, ired[w][0]);
-      mx = max(mx, ired[w][1]);
-    }
-    if (mx <= mn) mn = mx = 0;
-    d.tile[tile].lo = mn & ~(kGroup - 1);
-    d.tile[tile].hi = (mx + kGroup - 1) & ~(kGroup - 1);
+    d.direct[tile] = fine ? left : kBad;
+    d.tile[tile].lo = mn;
+    d.tile[tile].hi = mx;
   }
 }
 
@@ -270,8 +279,8 @@ __device__ __forceinline__ int runs_of(const XpDev& d, int lo, int hi) {
   return hi > lo ? (hi + d.run - 1) / d.run - lo / d.run : 0;
 }
 
-// One CTA: exclusive sums over the tiles; without the memory for all of them,
-// or with distances out of order anywhere, every column goes direct.
+// One CTA: exclusive sums over the tiles. The columns of a set with distances
+// out of order go direct, those of the other sets don't depend on it.
 __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
   __shared__ long long sw[32], su[32];
   __shared__ int slo[32], shi[32];
@@ -281,11 +290,23 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
   long long bw = 0, bu = 0;
   int lo = 0x7fffffff, hi = 0;
   long long left = 0;
+  for (int b = t; b < d.nsets; b += 1024) d.set_bad[b] = 0;
+  __syncthreads();
   bool bad = false;
+  for (int i = t; i < ntile; i += 1024)
+    if (d.direct[i] & kBad) {
+      d.set_bad[i / d.ft] = 1;
+      bad = true;
+    }
+  bad = __syncthreads_or(bad);
   for (int i0 = 0; i0 < ntile; i0 += 1024) {
     const int i = i0 + t;
     long long w = 0, u = 0;
     if (i < ntile) {
+      if (bad && d.set_bad[i / d.ft]) {
+        d.tile[i].lo = d.tile[i].hi = 0;
+        d.direct[i] = min(kTileCols, d.nf - i % d.ft * kTileCols);
+      }
       const int a = d.tile[i].lo, z = d.tile[i].hi;
       w = z - a;
       u = (long long)d.nacc * d.mtiles * runs_of(d, a, z);
@@ -293,8 +314,7 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
         lo = min(lo, a);
         hi = max(hi, z);
       }
-      left += d.direct[i] & (kBad - 1);
-      bad = bad || (d.direct[i] & kBad) != 0;
+      left += d.direct[i];
     }
     long long iw = w, iu = u;
     for (int s = 1; s < 32; s <<= 1) {
@@ -329,7 +349,6 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
     hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, s));
     left += __shfl_xor_sync(0xffffffffu, left, s);
   }
-  bad = __syncthreads_or(bad);
   if (lane == 0) {
     slo[wid] = lo;
     shi[wid] = hi;
@@ -342,7 +361,8 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
     hi = max(hi, shi[k]);
     left += sleft[k];
   }
-  const bool ok = !bad && bw <= d.blocks_cap && bu <= d.units_cap;
+  // (always so: the tiles' shares add up to less)
+  const bool ok = bw <= d.blocks_cap && bu <= d.units_cap;
   if (t == 0) {
     d.plan->units = ok ? bu : 0;
     d.plan->blocks = ok ? bw : 0;
@@ -357,9 +377,11 @@ __global__ void __launch_bounds__(1024) xp_scan_kernel(XpDev d) {
       int* u = d.unit_tile + d.tile[i].unit;
       for (int k = 0; k < d.nacc * d.mtiles * runs; ++k) u[k] = i;
     }
-  } else {
+  }
+  if (!ok || bad) {
     const long long ncol = (long long)d.nsets * d.nf;
-    for (long long i = t; i < ncol; i += 1024) d.use[i] = 0;
+    for (long long i = t; i < ncol; i += 1024)
+      if (!ok || d.set_bad[i / d.nf]) d.use[i] = 0;
   }
 }
 
@@ -1374,7 +1396,7 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   const long long mn = (long long)div_up(p.nf_all, kTileCols) * d.mtiles * d.nacc;
   d.run = batch || mn >= 96 ? 64 : mn >= 32 ? 32 : mn >= 12 ? 16 : 8;
   // No column that the plan takes (xp_columns_kernel) has more cells than this.
-  const double most = std::max((double)p.total * p.nc * d.nsrc * 250.0, kAnyCost / p.nf_all) /
+  const double most = std::max((double)p.total_all * p.nc * d.nsrc * 250.0, kAnyCost / p.nf_all) /
                       (kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0));
   // Nor does W get more than the direct kernels' interval data and 512 MiB (all
   // cells of 4096 frequencies): of more frequencies, those with many cells go
@@ -1386,10 +1408,23 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
                 ~(kGroup - 1);
   const long long ntile = (long long)p.nsets * d.ft;
   long long cells = ntile * d.cells_cap;
+  d.tile_cells = d.cells_cap;
   if (batch) {
-    // as much as the direct kernels' interval data, and 64 MiB
-    const long long direct = (long long)p.total * p.nf * 16 / ((long long)kBlockFloats * 4);
-    cells = std::min(cells, direct + (64ll << 20) / (kBlockFloats * 4));
+    // W of a tile of n pairs: as much as the direct kernels' interval data (n / 4
+    // blocks) and tile_cells more. Its own share, and not what other sets leave,
+    // so that a set's columns go the same way whatever sets it shares a call or
+    // a group of a host batch with. tile_cells: 384, as long as that comes to
+    // less than 4 GiB and a quarter of the interval data together, or 64 MiB in
+    // all. (Of 400 batches of 4 to 64 sets of 20-4000 pairs, drawn at random,
+    // 320 left no tile out that 64 MiB beside the interval data had held for all
+    // tiles together, 256 left out tiles of three; 500 sets of 50-200 pairs x
+    // 512 f, r to 300 km at 1 Hz: at most 192.)
+    const long long block = (long long)kBlockFloats * 4;
+    const long long ntile_all = (long long)p.nsets_all * d.ft;
+    const long long more = (4ll << 30) / block / nin + (long long)p.total_all * p.nf * 4 / block;
+    d.tile_cells = (int)std::min<long long>(
+        kMaxCells, std::max(std::min(384ll, more / ntile_all), (64ll << 20) / block / ntile_all));
+    cells = std::min(cells, (p.total / 4 + (long long)p.nsets * d.tile_cells) * d.ft);
   }
   cells &= ~(long long)(kGroup - 1);
   d.blocks_cap = cells;
@@ -1405,6 +1440,7 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   d.plan = reinterpret_cast<XpPlan*>(place(sizeof(XpPlan)));
   d.tile = reinterpret_cast<XpTile*>(place(sizeof(XpTile) * ntile));
   d.direct = reinterpret_cast<int*>(place(sizeof(int) * ntile));
+  d.set_bad = reinterpret_cast<int*>(place(sizeof(int) * (size_t)p.nsets));
   d.slot_set = reinterpret_cast<int*>(place(sizeof(int) * (size_t)d.slots));
   const int nbasis = d.nsrc;
   d.E = reinterpret_cast<float*>(place(sizeof(float) * (size_t)nbasis * d.cells_cap * kNodes * d.ncp));

@@ -21,10 +21,11 @@ struct XpProblem {
   InDesc in[2];
   float* out;  // [nsets][nc][nf]
   int normalize;
-  // frequencies and pairs of the whole problem that this one is a window or
-  // a group of sets of
+  // frequencies, pairs and sets of the whole problem that this one is a window
+  // or a group of sets of
   int nf_all;
   long long total_all;
+  int nsets_all;
 };
 
 // What the host sized and where it lies in the call's scratch.

@@ -505,7 +505,7 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
   if (expand) {
     xp.rs = a.r;
     xp.wtr = wtr;
-    xp.nsets = 1;
+    xp.nsets = xp.nsets_all = 1;
     xp.total = xp.total_all = a.nr;
     xp.nf = a.nf;
     xp.nc = a.nc;
