@@ -5,6 +5,7 @@
 #include <map>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 #include "ccfj_core.cuh"
 #include "tune_cache.h"
@@ -204,6 +205,46 @@ void* Scratch::get(size_t bytes) {
     bytes_ += bytes;
   }
   return p;
+}
+
+namespace {
+std::mutex g_flag_mu;
+std::vector<unsigned int*> g_flags;  // free words
+constexpr int kFlagsPerPage = 64;
+}  // namespace
+
+unsigned int* CallFlag::word() {
+  if (word_) return word_;
+  std::lock_guard<std::mutex> lk(g_flag_mu);
+  if (g_flags.empty()) {
+    unsigned int* page = nullptr;
+    const cudaError_t e = cudaHostAlloc((void**)&page, kFlagsPerPage * sizeof(unsigned int),
+                                        cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      set_error(CCFJ_ERR_ALLOC, "cudaHostAlloc failed: %s", cudaGetErrorString(e));
+      return nullptr;
+    }
+    for (int i = 0; i < kFlagsPerPage; ++i) g_flags.push_back(page + i);
+  }
+  word_ = g_flags.back();
+  g_flags.pop_back();
+  *word_ = 0;
+  return word_;
+}
+
+int CallFlag::status(const char* call) {
+  waited_ = true;
+  if (word_ && *static_cast<volatile unsigned int*>(word_) != 0)
+    return set_error(CCFJ_ERR_TIMEOUT, "%s: a bounded device wait ran out", call);
+  return CCFJ_OK;
+}
+
+CallFlag::~CallFlag() {
+  if (!word_) return;
+  if (!waited_) cudaStreamSynchronize(s_);
+  std::lock_guard<std::mutex> lk(g_flag_mu);
+  g_flags.push_back(word_);
 }
 
 }  // namespace ccfj

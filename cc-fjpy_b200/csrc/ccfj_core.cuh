@@ -51,6 +51,28 @@ class Scratch {
   size_t bytes_ = 0;
 };
 
+// The word that the kernels of one host-memory call set when a bounded wait of
+// theirs runs out. It lies in pinned host memory, which a kernel writes only in
+// that case, so that reading it costs no copy. Words are taken from a pool that
+// grows with the calls that run at the same time; a call that leaves early
+// waits for its stream before it gives its word back.
+class CallFlag {
+ public:
+  explicit CallFlag(cudaStream_t s) : s_(s) {}
+  ~CallFlag();
+  // nullptr (and an error recorded) without memory for it
+  unsigned int* word();
+  // Once the call's stream has been waited for: CCFJ_OK or CCFJ_ERR_TIMEOUT
+  int status(const char* call);
+
+ private:
+  CallFlag(const CallFlag&) = delete;
+  CallFlag& operator=(const CallFlag&) = delete;
+  cudaStream_t s_;
+  unsigned int* word_ = nullptr;
+  bool waited_ = false;
+};
+
 #define CCFJ_CUDA_TRY(expr)                                                                  \
   do {                                                                                       \
     cudaError_t e__ = (expr);                                                                \

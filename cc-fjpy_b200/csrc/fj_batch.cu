@@ -321,9 +321,10 @@ int batch_variant(const ccfj_batch_args& a, long long total) {
 // The device sequence of one batch (all pointers device pointers;
 // `total` = offsets[nsets], known to the caller).
 // `expand`: the wave-cell expansion may take columns; total_all, nsets_all: the
-// pairs and sets of the whole batch that these sets are a group of.
+// pairs and sets of the whole batch that these sets are a group of; err: as
+// XpProblem::err.
 int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStream_t s,
-                 long long total_all = 0, int nsets_all = 0) {
+                 long long total_all = 0, int nsets_all = 0, unsigned int* err = nullptr) {
   Scratch sc(s);
   const int nin = nin_of_mode(a.mode);
   float* drs = sc.get_n<float>(total + 1);
@@ -385,6 +386,7 @@ int batch_device(const ccfj_batch_args& a, long long total, bool expand, cudaStr
     xp.in[1] = in[1];
     xp.out = a.out;
     xp.normalize = a.normalize;
+    xp.err = err;
     xp.nf_all = a.nf;
     xp.total_all = total_all > 0 ? total_all : total;
     xp.nsets_all = nsets_all > 0 ? nsets_all : a.nsets;
@@ -655,6 +657,9 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
   const std::vector<SetGroup> groups = plan_groups(a, total, nin, ubytes);
   const int ng = (int)groups.size();
   Scratch sc(s);
+  CallFlag flag(s);
+  unsigned int* err = flag.word();
+  if (!err) return CCFJ_ERR_ALLOC;
   float* du = sc.get_n<float>(hi - lo);
   // the batch's offsets, then (pipelined) each group's rebased offsets
   long long* doff = sc.get_n<long long>(a.nsets + 1 + (ng > 0 ? a.nsets + ng : 0));
@@ -685,9 +690,10 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
   d.perm = dp;
   const size_t out_bytes = sizeof(float) * a.nsets * a.nc * a.nf;
   if (ng == 0) {
-    const int st = batch_device(d, total, batch_expands(a, total), s);
+    int st = batch_device(d, total, batch_expands(a, total), s, total, a.nsets, err);
     if (st != CCFJ_OK) return st;
-    return copy_to_host(a.out, dout, out_bytes, 0, s);
+    st = copy_to_host(a.out, dout, out_bytes, 0, s);
+    return st != CCFJ_OK ? st : flag.status("ccfj_fj_batch_v1");
   }
 
   // Pipelined: each group's offsets rebased to its first pair (one copy for
@@ -731,11 +737,12 @@ int batch_host(const ccfj_batch_args& a, cudaStream_t s) {
     dg.out = dout + (size_t)G.b0 * a.nc * a.nf;
     dg.variant = variant;
     CCFJ_CUDA_TRY(cudaStreamWaitEvent(s, lane.ev[g], 0));
-    st = batch_device(dg, dg.total_pairs, expand, s, total, a.nsets);
+    st = batch_device(dg, dg.total_pairs, expand, s, total, a.nsets, err);
     if (st != CCFJ_OK) return st;
     if (g + 1 < ng && (st = copy_group(g + 1)) != CCFJ_OK) return st;
   }
-  return copy_to_host(a.out, dout, out_bytes, 0, s);
+  st = copy_to_host(a.out, dout, out_bytes, 0, s);
+  return st != CCFJ_OK ? st : flag.status("ccfj_fj_batch_v1");
 }
 
 }  // namespace

@@ -64,8 +64,10 @@ static int eq_validate(const ccfj_eq_args* a) {
 }
 
 // All pointers device pointers. call_err: a device word that receives this
-// call's timeout flag of the tensor-core path (NULL: scratch of the call).
-static int eq_device(const ccfj_eq_args& a, cudaStream_t s, unsigned int* call_err = nullptr) {
+// call's timeout flag of the tensor-core path (NULL: scratch of the call);
+// xp_err: as FjChoice::err.
+static int eq_device(const ccfj_eq_args& a, cudaStream_t s, unsigned int* call_err = nullptr,
+                     unsigned int* xp_err = nullptr) {
   Scratch sc(s);
   const int nw = a.nwin > 0 ? a.nwin : 1;
   const long long rows_out = (long long)nw * a.ntr;
@@ -130,7 +132,9 @@ static int eq_device(const ccfj_eq_args& a, cudaStream_t s, unsigned int* call_e
     d.c = a.c;
     d.out = a.out + (size_t)w * a.nc * a.nf;
     d.tau = a.tau;
-    st = fj_device(d, s);
+    FjChoice choice;
+    choice.err = xp_err;
+    st = fj_device(d, s, choice);
     if (st != CCFJ_OK) return st;
   }
   return CCFJ_OK;
@@ -142,6 +146,8 @@ static int eq_host(const ccfj_eq_args& a, cudaStream_t s) {
       CCFJ_REQUIRE(a.perm[i] >= 0 && a.perm[i] < a.u_rows,
                    "ccfj_fj_earthquake_v1: perm[%d]=%lld out of range", i, a.perm[i]);
   Scratch sc(s);
+  CallFlag flag(s);
+  if (!flag.word()) return CCFJ_ERR_ALLOC;
   ccfj_eq_args d = a;
   d.device_ptrs = 1;
   d.out_f64 = 0;
@@ -184,7 +190,7 @@ static int eq_host(const ccfj_eq_args& a, cudaStream_t s) {
   d.f = df;
   d.c = dc;
   d.out = dout;
-  int st = eq_device(d, s, derr);
+  int st = eq_device(d, s, derr, flag.word());
   if (st != CCFJ_OK) return st;
   const size_t nout = (size_t)nw * a.nc * a.nf;
   st = a.out_f64 ? copy_to_host(a.out, dout, nout, 1, s)
@@ -195,7 +201,7 @@ static int eq_host(const ccfj_eq_args& a, cudaStream_t s) {
   if (st != CCFJ_OK) return st;
   if (failed)
     return set_error(CCFJ_ERR_TIMEOUT, "ccfj_fj_earthquake_v1: a bounded device wait ran out");
-  return CCFJ_OK;
+  return flag.status("ccfj_fj_earthquake_v1");
 }
 
 std::atomic<int> g_mwfj_path{0};

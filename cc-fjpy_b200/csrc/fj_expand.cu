@@ -142,6 +142,9 @@ struct XpDev {
   float* head;           // [slot][nf][input][16]
   float* tail;
   int2* span;            // [slot][nf] first and last cell of a chunk
+  unsigned int* err;     // the call's flag of the product's waits, or NULL
+  long long wait_cycles;
+  int no_load;           // self-test: the product's operands never come
 };
 
 __device__ __forceinline__ long long set_begin(const XpDev& d, int b) { return d.off ? d.off[b] : 0; }
@@ -934,7 +937,8 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
 // FP32 multiply-adds (128 x 64 tiles, 8 x 8 a thread, paired).
 //
 // Every wait is bounded. One that runs out sets `abort`, the other roles then
-// run out or see it, the unit's sums become NaN and g_xp_error is set.
+// run out or see it, the unit's sums become NaN, and g_xp_error and the call's
+// own flag are set.
 __device__ unsigned int g_xp_error = 0;
 constexpr int kDrainWarps = 8, kLoadWarps = 8;
 constexpr int kGemmThreads = 32 * (kDrainWarps + kLoadWarps + 1);
@@ -1054,7 +1058,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xp_gemm_kernel(XpDev d) {
     if (!tc::mbar_try_wait(bar, parity)) {
       const long long t0 = clock64();
       while (ok && !tc::mbar_try_wait(bar, parity))
-        if (abort_flag || clock64() - t0 > tc::kWaitCycles) ok = false;
+        if (abort_flag || clock64() - t0 > d.wait_cycles) ok = false;
     }
     ok = __all_sync(0xffffffffu, ok);
     if (!ok) abort_flag = 1;
@@ -1111,7 +1115,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xp_gemm_kernel(XpDev d) {
     const long long plane = (long long)d.cells_cap * kNodes * d.ncp;
     uint32_t it = 0;
     bool ok = true;
-    for (long long unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
+    for (long long unit = d.no_load ? units : blockIdx.x; ok && unit < units; unit += gridDim.x) {
       const Unit u = unit_at(d, unit);
       struct Raw {
         float4 a[2], b[2];
@@ -1214,7 +1218,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xp_gemm_kernel(XpDev d) {
       if (tc::mbar_try_wait(bar, parity)) return true;
       const long long t0 = clock64();
       while (!tc::mbar_try_wait(bar, parity))
-        if (abort_flag || clock64() - t0 > tc::kWaitCycles) {
+        if (abort_flag || clock64() - t0 > d.wait_cycles) {
           abort_flag = 1;
           return false;
         }
@@ -1268,7 +1272,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xp_gemm_kernel(XpDev d) {
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (tid == 0 && abort_flag) atomicOr(&g_xp_error, 1u);
+  if (tid == 0 && abort_flag) {
+    if (!d.no_load) atomicOr(&g_xp_error, 1u);
+    if (d.err) *static_cast<volatile unsigned int*>(d.err) = 1u;  // host memory
+  }
   if (warp == kMmaWarp)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
@@ -1377,6 +1384,8 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   d.in[1] = p.in[1];
   d.out = p.out;
   d.normalize = p.normalize;
+  d.err = p.err;
+  d.wait_cycles = tc::kWaitCycles;
   d.ft = (int)div_up(p.nf, kTileCols);
   d.mtiles = (int)div_up(p.nc, kTileRows);
   d.ncp = d.mtiles * kTileRows;
@@ -1584,6 +1593,44 @@ int xp_sticky_error(cudaStream_t s, bool* failed) {
   return CCFJ_OK;
 }
 
+int xp_self_test(cudaStream_t s, int* status) {
+  Scratch sc(s);
+  CallFlag flag(s);
+  XpDev d{};
+  d.plan = sc.get_n<XpPlan>(1);
+  d.tile = sc.get_n<XpTile>(1);
+  d.unit_tile = sc.get_n<int>(1);
+  d.part = sc.get_n<float>(kTileRows * kTileCols);
+  d.err = flag.word();
+  if (!d.plan || !d.tile || !d.unit_tile || !d.part || !d.err) return CCFJ_ERR_ALLOC;
+  // one unit of one group of cells
+  XpPlan plan{};
+  plan.units = 1;
+  XpTile tile{};
+  tile.hi = kGroup;
+  const int unit_tile = 0;
+  CCFJ_CUDA_TRY(cudaMemcpyAsync(d.plan, &plan, sizeof(plan), cudaMemcpyHostToDevice, s));
+  CCFJ_CUDA_TRY(cudaMemcpyAsync(d.tile, &tile, sizeof(tile), cudaMemcpyHostToDevice, s));
+  CCFJ_CUDA_TRY(cudaMemcpyAsync(d.unit_tile, &unit_tile, sizeof(int), cudaMemcpyHostToDevice, s));
+  CCFJ_CUDA_TRY(cudaMemsetAsync(d.part, 0, sizeof(float) * kTileRows * kTileCols, s));
+  d.mtiles = d.nacc = d.nsrc = 1;
+  d.run = kGroup;
+  d.wait_cycles = 2000000;  // ~1 ms
+  d.no_load = 1;
+  CCFJ_CUDA_TRY(cudaFuncSetAttribute(xp_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kGemmSmem));
+  xp_gemm_kernel<1><<<1, kGemmThreads, kGemmSmem, s>>>(d);
+  count_launch();
+  CCFJ_LAUNCH_CHECK("xp_gemm_kernel (self-test)");
+  float sum = 0.0f;
+  CCFJ_CUDA_TRY(cudaMemcpyAsync(&sum, d.part, sizeof(sum), cudaMemcpyDeviceToHost, s));
+  CCFJ_CUDA_TRY(cudaStreamSynchronize(s));
+  *status = flag.status("self-test");
+  if (sum == sum)
+    return set_error(CCFJ_ERR_CUDA, "self-test: the product gave a number without its operands");
+  return CCFJ_OK;
+}
+
 int xp_run(const XpProblem& p, const XpWork& w, cudaStream_t s) {
   XpDev d;
   layout(p, w.base, &d);
@@ -1591,3 +1638,14 @@ int xp_run(const XpProblem& p, const XpWork& w, cudaStream_t s) {
 }
 
 }  // namespace ccfj
+
+CCFJ_API int ccfj_self_test_product_timeout(void* stream) {
+  ccfj::clear_error();
+  int status = CCFJ_OK;
+  const int st = ccfj::xp_self_test((cudaStream_t)stream, &status);
+  if (st != CCFJ_OK) return st;
+  if (status != CCFJ_ERR_TIMEOUT)
+    return ccfj::set_error(CCFJ_ERR_CUDA, "self-test: the product did not report its timeout");
+  ccfj::clear_error();
+  return CCFJ_OK;
+}

@@ -26,6 +26,7 @@ struct XpProblem {
   int nf_all;
   long long total_all;
   int nsets_all;
+  unsigned int* err;  // set when a bounded wait of the product runs out, or NULL
 };
 
 // What the host sized and where it lies in the call's scratch.
@@ -46,6 +47,10 @@ int xp_plan(const XpProblem& p, Scratch& sc, cudaStream_t s, XpWork* w, bool* ok
 // Waits for `s`, reads the process-wide flag of the product's bounded waits
 // (set when one ran out: that unit's columns are NaN) and clears it.
 int xp_sticky_error(cudaStream_t s, bool* failed);
+// Self-test of those waits: one CTA of the product whose operands never come,
+// with a ~1 ms limit, as a host-memory call reads it: *status becomes
+// CCFJ_ERR_TIMEOUT where the kernel gave up and set the call's flag.
+int xp_self_test(cudaStream_t s, int* status);
 // Computes the columns the plan chose, normalised if asked.
 int xp_run(const XpProblem& p, const XpWork& w, cudaStream_t s);
 

@@ -29,11 +29,13 @@ int hilbert_rows_fft(const InDesc& in, int n, int es, int nr, int nf, int fstrid
 // launch, fixed-order sum). path: -1 decides by sizes and settings whether
 // the wave-cell expansion may take columns (fj_expand.cu), 0 keeps it off, 1
 // allows it, with nf_all the frequencies of the whole problem that this one
-// is a block of.
+// is a block of. err: the word of a host-memory call that a bounded wait which
+// runs out sets (CallFlag), or NULL.
 struct FjChoice {
   int cpt = 0, nsplit = 0;
   int path = -1;
   int nf_all = 0;
+  unsigned int* err = nullptr;
 };
 // Device-resident transform (all pointers in args are device pointers).
 int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice = FjChoice());

@@ -517,6 +517,7 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
     xp.in[1] = in[1];
     xp.out = a.out;
     xp.normalize = a.normalize;
+    xp.err = choice.err;
     xp.nf_all = choice.nf_all > 0 ? choice.nf_all : a.nf_total > 0 ? a.nf_total : a.nf;
     const int st = xp_plan(xp, sc, s, &xw, &expanded);
     if (st != CCFJ_OK) return st;
@@ -725,6 +726,9 @@ static int fj_host_blocks(const ccfj_fj_args& a, cudaStream_t s, int nblk, int n
   block.nsplit = full_split;
   block.path = expansion_allowed(a) ? 1 : 0;
   block.nf_all = a.nf_total > 0 ? a.nf_total : a.nf;
+  CallFlag flag(s);
+  block.err = flag.word();
+  if (!block.err) return CCFJ_ERR_ALLOC;
   Scratch sc(s);
   float* dr = sc.get_n<float>(a.nr);
   float* df = sc.get_n<float>(a.nf);
@@ -886,7 +890,7 @@ static int fj_host_blocks(const ccfj_fj_args& a, cudaStream_t s, int nblk, int n
   destroy();
   if (e != cudaSuccess)
     return set_error(CCFJ_ERR_CUDA, "ccfj_fj_v1: %s", cudaGetErrorString(e));
-  return CCFJ_OK;
+  return flag.status("ccfj_fj_v1");
 }
 
 // Host-memory variant: copies the inputs in, runs the device path, copies
@@ -916,6 +920,10 @@ static int fj_host(const ccfj_fj_args& a, cudaStream_t s) {
   const int nblk = host_block_count(a, merged ? (long long)(hi - lo) : nin * span);
   if (nblk > 1) return fj_host_blocks(a, s, nblk, nin, merged);
   Scratch sc(s);
+  CallFlag flag(s);
+  FjChoice choice;
+  choice.err = flag.word();
+  if (!choice.err) return CCFJ_ERR_ALLOC;
   ccfj_fj_args d = a;
   d.device_ptrs = 1;
   float* dr = sc.get_n<float>(a.nr);
@@ -951,9 +959,10 @@ static int fj_host(const ccfj_fj_args& a, cudaStream_t s) {
   d.f = df;
   d.c = dc;
   d.out = dout;
-  int st = fj_device(d, s);
+  int st = fj_device(d, s, choice);
   if (st != CCFJ_OK) return st;
-  return copy_to_host(a.out, dout, sizeof(float) * a.nc * a.nf, 0, s);
+  st = copy_to_host(a.out, dout, sizeof(float) * a.nc * a.nf, 0, s);
+  return st != CCFJ_OK ? st : flag.status("ccfj_fj_v1");
 }
 
 int fj_entry(const ccfj_fj_args* a, cudaStream_t s) {

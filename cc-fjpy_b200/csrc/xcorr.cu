@@ -634,6 +634,9 @@ static int cc_fj_noise(const ccfj_cc_args& cc, const ccfj_fj_args& fj, cudaStrea
   CCFJ_REQUIRE(cc.npairs >= 1 && cc.nf >= 1, "ccfj_cc_fj_noise_v1: npairs=%d nf=%d", cc.npairs,
                cc.nf);
   Scratch sc(s);
+  CallFlag flag(s);
+  FjChoice choice;
+  if (!cc.device_ptrs && !(choice.err = flag.word())) return CCFJ_ERR_ALLOC;
   float* spec = sc.get_n<float>(2 * (size_t)cc.npairs * cc.nf);
   if (!spec) return CCFJ_ERR_ALLOC;
   ccfj_cc_args c = cc;
@@ -690,10 +693,10 @@ static int cc_fj_noise(const ccfj_cc_args& cc, const ccfj_fj_args& fj, cudaStrea
   }
   st = run(c, s);
   if (st != CCFJ_OK) return st;
-  st = fj_device(f, s);
-  if (st != CCFJ_OK) return st;
-  if (!fj.device_ptrs) return copy_to_host(fj.out, f.out, sizeof(float) * fj.nc * fj.nf, 0, s);
-  return CCFJ_OK;
+  st = fj_device(f, s, choice);
+  if (st != CCFJ_OK || fj.device_ptrs) return st;
+  st = copy_to_host(fj.out, f.out, sizeof(float) * fj.nc * fj.nf, 0, s);
+  return st != CCFJ_OK ? st : flag.status("ccfj_cc_fj_noise_v1");
 }
 
 }  // namespace xc

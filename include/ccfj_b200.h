@@ -252,6 +252,10 @@ CCFJ_API int ccfj_device_status(void *stream);
  * returns CCFJ_OK if the kernel gave up, reported the timeout and left the
  * device usable (CCFJ_ERR_CUDA otherwise). No counterpart in the reference. */
 CCFJ_API int ccfj_self_test_wait_timeout(void *stream);
+/* The same for the transform's tensor-core product: one CTA whose operands
+ * never come gives up, its sums are NaN, and the flag that host-memory calls
+ * return as CCFJ_ERR_TIMEOUT is set. */
+CCFJ_API int ccfj_self_test_product_timeout(void *stream);
 
 /* ---------------------------------------- ambient-noise cross-correlation
  * The reference's CrossCorrelation (src/CrossCorr.cpp:33-159, called by CC
