@@ -101,7 +101,6 @@ struct XpPlan {
 };
 
 constexpr int kBad = 1 << 30;
-
 struct XpDev {
   const float* rs;
   const float* wtr;
@@ -117,6 +116,7 @@ struct XpDev {
   int ft;                // column tiles of a set
   int chunk;             // stations of a moments chunk
   double nf_all;         // frequencies of the whole problem
+  double cells_in_time;  // a column with fewer takes the expansion (worth_cells)
   int mtiles;            // velocity tiles
   int run;               // cells of a GEMM unit
   int nsrc, nacc;        // products of a result, results of a column
@@ -170,6 +170,45 @@ __device__ __forceinline__ int chunks_of(const XpDev& d, long long n) {
 constexpr double kAnyCost = 4e8;  // issue slots, 20 us
 __host__ __device__ inline bool worth(double n, double per_pair) {
   return n >= 48.0 || (n >= 2.0 && n * per_pair >= 6e6);
+}
+
+// Whether a column with this many cells takes the expansion. Two estimates:
+//
+// Throughput, for a chip that is full: multiply-adds of the expansion against
+// those of the direct kernel (56 issue slots a term measured on short
+// intervals, 250 where most are long against the wavelength; itype 0 has no
+// intervals, and its sparse columns count 250 in batches and below 48 pairs
+// alone). A problem whose columns all cost little keeps them together: the
+// direct kernels' time is the walk over the pairs, for one column too.
+//
+// Latency, for one transform: both ways are chains, of launches here, of pairs
+// there, and a problem with columns on both sides of the line pays for both. A
+// column takes the expansion if a problem that had this one as its highest
+// frequency would be computed in less time (cells_in_time()), or up to 1.3 times as
+// long. Not where a column has many more cells than pairs (earthquake records
+// over thousands of km): such problems have columns beyond any line, and more
+// of them on this side made them slower.
+//
+// Of 1683 transforms drawn at random (2-19,900 pairs, half of them of up to 600
+// pairs, where the line lies), 135 took more than 15% longer than the direct
+// kernels alone with the first estimate only (an itype 0 case 2.7 times as
+// long), 94 with both; 58 became more than 15% faster and 2 slower (66 pairs x
+// 906 f x 38 c 164 -> 88 us, 95 by the direct kernels; 182 pairs x 208 f x 23 c,
+// itype 0, 118 -> 91 us, 101 directly). Still slower than directly: problems
+// whose upper frequencies go direct while the lower ones do not (156 records x
+// 320 f x 43 c 329 us, 187 directly).
+constexpr double kMargin = 1.3;
+constexpr double kDense = 6.5;
+__device__ __forceinline__ bool worth_cells(const XpDev& d, int itype, int cells_of_column,
+                                            double n) {
+  const double cells = cells_of_column;
+  const double grid =
+      (cells + kGroup) * kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0) + 200.0 * n;
+  const bool sparse = cells > n;
+  const double direct =
+      n * d.nc * d.nsrc * (sparse && (itype == 1 || n < 48.0 || d.off) ? 250.0 : 56.0);
+  if (grid < direct || grid * d.nf_all < kAnyCost) return true;
+  return cells < d.cells_in_time && cells * d.nacc <= kDense * n;
 }
 
 // One CTA of 128 threads per (set, 128 frequencies).
@@ -227,16 +266,7 @@ __global__ void xp_columns_kernel(XpDev d) {
         float rel;
         first = locate<DY>(r0, fx, rel);
         last = locate<DY>(r1, fx, rel) + 1;
-        // multiply-adds of the expansion against those of the direct kernel
-        // (56 issue slots a term measured on short intervals, 250 where most
-        // are long against the wavelength)
-        const double cells = last - first;
-        const double grid =
-            (cells + kGroup) * kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0) + 200.0 * n;
-        const double direct = (double)n * d.nc * d.nsrc * (cells > n ? 250.0 : 56.0);
-        // (a problem whose columns all cost little keeps them together: the
-        // direct kernels' time is the walk over the pairs, for one column too)
-        use = grid < direct || grid * d.nf_all < kAnyCost;
+        use = worth_cells(d, ITYPE, last - first, (double)n);
       }
     }
   }
@@ -1366,6 +1396,37 @@ int nin_of(int mode) { return mode == CCFJ_MODE_J || mode == CCFJ_MODE_Y ? 1 : 2
 int nsrc_of(int mode) { return mode == CCFJ_MODE_J_MINUS_Y || mode == CCFJ_MODE_ABS_H ? 2 : 1; }
 int nacc_of(int mode) { return mode == CCFJ_MODE_ABS_J || mode == CCFJ_MODE_ABS_H ? 2 : 1; }
 
+// The cells of the highest frequency of one transform at which the expansion
+// takes kMargin times the direct kernels' time; none for a batch, whose sets run
+// side by side. The constants (microseconds) are a fit to one B200's times of
+// the transforms that worth_cells() names: half of the predictions are within
+// 12% of the direct kernels' time and 8% of the expansion's, nine in ten within
+// 50% and 25%.
+double cells_in_time(const XpProblem& p, const XpDev& d) {
+  if (p.off) return 0.0;
+  const int nin = nin_of(p.mode);
+  const bool trapezoid = p.itype == 0, two = d.nsrc == 2;
+  const double n = (double)p.total, nf = p.nf_all;
+  const double launches = 60.0 + (trapezoid ? 0.0 : 8.0) + 20.0 * (nin - 1) +
+                          2.0 * std::min(d.chunk, 32) * nin;
+  // half the cells of the highest frequency in the product and the moments (a
+  // linear grid's mean), all of them in the basis
+  const double per_cell =
+      0.5 * (4.9e-3 * div_up(p.nf_all, kTileCols) * d.mtiles * d.nacc * d.nsrc + 5.5e-5 * nf * nin) +
+      1.7e-4 * d.ncp + (trapezoid ? 0.0 : 0.035);
+  // The direct kernels: a walk over the pairs (in as many station ranges as their
+  // untuned choice, split_for()) or their terms, whichever is longer.
+  const double ctas = (double)div_up(p.nc, trapezoid ? 32 : 16) * div_up(p.nf_all, 32);
+  double ranges = 1.0;
+  for (int k = 2; k <= 4; ++k)
+    if (k * ctas <= 444.0 && n >= 64.0 * k) ranges = k;
+  const double walk = n / ranges * (trapezoid ? (two ? 0.95 : 0.85) : (two ? 1.5 : 1.0));
+  const double terms =
+      n * nf * p.nc * 1e-8 * (trapezoid ? (two ? 350.0 : 126.0) : (two ? 1100.0 : 500.0));
+  const double direct = 34.0 + 20.0 * (nin - 1) + std::pow(std::pow(walk, 4) + std::pow(terms, 4), 0.25);
+  return (kMargin * direct - launches) / per_cell;
+}
+
 size_t round256(size_t v) { return (v + 255) & ~size_t(255); }
 
 // Sizes, and places relative to `base`; returns the bytes needed.
@@ -1405,8 +1466,11 @@ size_t layout(const XpProblem& p, void* base, XpDev* out) {
   const long long mn = (long long)div_up(p.nf_all, kTileCols) * d.mtiles * d.nacc;
   d.run = batch || mn >= 96 ? 64 : mn >= 32 ? 32 : mn >= 12 ? 16 : 8;
   // No column that the plan takes (xp_columns_kernel) has more cells than this.
-  const double most = std::max((double)p.total_all * p.nc * d.nsrc * 250.0, kAnyCost / p.nf_all) /
-                      (kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0));
+  d.cells_in_time = cells_in_time(p, d);
+  const double most =
+      std::max(std::max((double)p.total_all * p.nc * d.nsrc * 250.0, kAnyCost / p.nf_all) /
+                   (kNodes * ((double)d.ncp * d.nsrc * d.nacc + 200.0)),
+               d.cells_in_time);
   // Nor does W get more than the direct kernels' interval data and 512 MiB (all
   // cells of 4096 frequencies): of more frequencies, those with many cells go
   // direct. By the whole problem's sizes, for its windows to decide alike.

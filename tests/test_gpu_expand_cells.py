@@ -91,3 +91,21 @@ def test_distances_on_cell_ends_of_many_frequencies(mode, itype):
     r = np.sort(np.concatenate([ends, np.nextafter(ends, np.float32(0)),
                                 np.nextafter(ends, np.float32(1e9))]))
     _check(_case(rng, r, f), mode, itype)
+
+
+# sizes near the line between the two ways, where a problem's upper frequencies
+# go direct: few pairs and many cells, few velocities, both rules, both bases
+@pytest.mark.parametrize("nr,nf,nc,mode,itype", [(62, 289, 53, "J", 1), (40, 658, 260, "J", 1),
+                                                 (257, 700, 23, "J-Y", 0), (57, 900, 508, "J", 0),
+                                                 (117, 745, 288, "|J|", 1), (83, 500, 77, "|H|", 1)])
+def test_windows_decide_as_the_whole_problem(nr, nf, nc, mode, itype):
+    rng = np.random.default_rng(nr)
+    r = np.sort(rng.uniform(500.0, RMAX, nr))
+    f = np.linspace(0.01, 1.8, nf)
+    u = cases.noise_spectra(rng, r, f, sigma=0.3)
+    case = ([np.ascontiguousarray(u.real), np.ascontiguousarray(u.imag)], r,
+            np.linspace(700.0, 4500.0, nc), f)
+    full = _run(case, MODES[mode], itype, normalize=True)
+    for a, b in ((0, 1), (1, 130), (130, 131), (131, nf)):
+        assert np.array_equal(_run(case, MODES[mode], itype, normalize=True, cols=(a, b)),
+                              full[:, a:b])
