@@ -445,21 +445,6 @@ def _expansion_roofline(nbytes, call_s, kernel_s=None):
             "kernel_ms": None if kernel_s is None else kernel_s * 1e3, "peak_source": source}
 
 
-def profile_traffic(name):
-    """DRAM bytes per launch of a kernel from a committed ncu summary under
-    profiles/ (the line 'traffic_bytes_per_launch: <bytes>'), or None."""
-    p = os.path.join(REPO, "profiles", name)
-    if not os.path.exists(p):
-        return None
-    for ln in open(p):
-        if ln.strip().startswith("traffic_bytes_per_launch:"):
-            try:
-                return float(ln.split(":", 1)[1].strip().split()[0])
-            except ValueError:
-                return None
-    return None
-
-
 # ------------------------------------------------------------ the configs
 class ConfigRun:
     """One configuration: device measurements first (GPU), then the

@@ -190,7 +190,8 @@ CC_HD void bf_rows(Dst dst, int Ns, int tq, int jn, const Cpx* rows, Cpx* v) {
   bf_twiddled<R>(dst, Ns, tq, jn, w, v);
 }
 
-// The same from the one table tw[u] = exp(-2 pi i u / M) of every pass
+// The same from the one table tw[u] = exp(-2 pi i u / M) of every pass (the host
+// replay's form)
 template <int R>
 CC_HD void bf_finish(Cpx* dst, int M, int Ns, const Cpx* tw, int t, Cpx* v) {
   const int jn = t % Ns;

@@ -55,8 +55,8 @@
 //   xp_finish_kernel   adds a column's units in order, |.| and normalisation
 //
 // Measured against the direct kernels on one B200 (device-resident call):
-// 19,900 pairs x 2048 f x 1000 c 61.3 -> 1.07 ms, 200 x 512 x 300 0.215 ->
-// 0.089 ms, 128 subarrays of 50-20,000 pairs (512 f x 500 c) 196 -> 4.3 ms; the
+// 19,900 pairs x 2048 f x 1000 c 61.3 -> 0.98 ms, 200 x 512 x 300 0.215 ->
+// 0.091 ms, 128 subarrays of 50-20,000 pairs (512 f x 500 c) 196 -> 3.6 ms; the
 // error against 64-bit quadrature 1.1e-6 -> 2e-7 of the spectrum (2-norm).
 //
 // Every sum is in an order fixed by the sizes, so results do not depend on
@@ -623,8 +623,9 @@ __device__ __forceinline__ void piece_point(float2 (&acc)[NIN][kNodes / 2], floa
 // short interval is not cut at a cell's end: since the lanes' cells end at
 // different stations, cutting each one ran two pieces in nearly every step.
 //
-// Bound by issue: 15 paired multiply-adds and about as many other instructions
-// a point, 2 or 3 points for most intervals. The spectra come in by cp.async,
+// Bound by issue (66% of the slots at 19,900 pairs x 2048 f, with 17 warps an SM)
+// and the FMA pipe's throttle: 15 paired multiply-adds and about as many other
+// instructions a point, 2 or 3 points for most intervals. The spectra come in by cp.async,
 // 16 stations ahead; unrolling the stations instead (loads into registers)
 // left the warps waiting for instructions as long as they issued. A lane of
 // short intervals follows its cell by one compare with the next one's start
@@ -962,9 +963,11 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
 // rows x 64 columns of the totals), 8 that bring the operands in (global to
 // registers, split, to shared memory as 8 x 16 byte core matrices), one that
 // issues the MMAs. Four stages of one step each: a cell (K = 16) or a group's
-// end rows (K = 8). Bound by shared memory: a step's MMAs read 48 KB of it and
-// the loaders store 32 KB. 19,900 pairs x 2048 f x 1000 c: 322 us, 884 us with
-// FP32 multiply-adds (128 x 64 tiles, 8 x 8 a thread, paired).
+// end rows (K = 8). No unit is full: at 19,900 pairs x 2048 f x 1000 c (335 us; 884
+// us with FP32 multiply-adds, 128 x 64 tiles, 8 x 8 a thread, paired) the tensor
+// pipe is active 36% of the time, the loaders' stores (32 KB a step) and the
+// drains take 39% of the shared memory's wavefronts beside the 48 KB a step that
+// the MMAs read, and the largest stall is the loaders' wait for L2.
 //
 // Every wait is bounded. One that runs out sets `abort`, the other roles then
 // run out or see it, the unit's sums become NaN, and g_xp_error and the call's

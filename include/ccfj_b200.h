@@ -153,12 +153,14 @@ CCFJ_API int ccfj_fj_batch_v1(const ccfj_batch_args *args, void *stream);
 /* Destroys the cached batch graphs (call before freeing buffers that a
  * cached graph refers to, if their addresses may be reused). */
 CCFJ_API int ccfj_batch_graph_cache_clear(void);
-/* Runs the batch (device pointers; out is overwritten) with 1, 2 and 4
- * velocities per thread, records the fastest for the batch's class (mode,
- * itype and the powers of two of total pairs, nsets, nf and nc) on this
- * device for later calls that pass variant 0 -- in this process, and in
- * later ones through the persistent table of ccfj_set_tune_cache -- and
- * returns it and its time. */
+/* Runs the batch (device pointers; out is overwritten) by the direct kernel
+ * alone, with 1, 2 and 4 velocities per thread, records the fastest for the
+ * batch's class (mode, itype and the powers of two of total pairs, nsets, nf
+ * and nc) on this device for later calls that pass variant 0 -- in this
+ * process, and in later ones through the persistent table of
+ * ccfj_set_tune_cache -- and returns it and its time. Such calls use it for
+ * the columns that the wave-cell expansion leaves to the direct kernel; a call
+ * that passes the variant runs without the expansion, in about that time. */
 CCFJ_API int ccfj_autotune_batch_v1(const ccfj_batch_args *args, void *stream,
                                     int *best_variant, float *best_ms);
 
@@ -362,19 +364,21 @@ CCFJ_API int ccfj_pick_v1(const float *spec, int nc, int nf, const float *c, con
                           void *stream);
 
 /* ------------------------------------------------------------- tuning
- * Tile choices of the FP32 transform: 1, 2 or 4 velocities per thread, and
+ * Tile choices of the direct kernels of the FP32 transform, which compute the
+ * columns that the wave-cell expansion leaves to them (all of them where a
+ * variant, a split or tau is given): 1, 2 or 4 velocities per thread, and
  * the number of station ranges (split launch: ranges of whole 32-station
  * chunks summed in a fixed order by a second kernel, so a given choice
- * gives the same result on every run). ccfj_autotune_fj_v1 times every
- * velocities-per-thread variant with 1 range and, where the unsplit grid
+ * gives the same result on every run). ccfj_autotune_fj_v1 times the direct
+ * kernels alone, every velocities-per-thread variant with 1 range and, where the unsplit grid
  * leaves resident slots idle, with 2-8 ranges, on the given problem (device
  * pointers; out is overwritten), records the fastest for the problem's
  * class (mode, itype and the powers of two of nr, nf, nc) on this device,
  * and returns its velocities per thread and time. Untuned classes use 2
  * (itype 1) or 4 (itype 0) velocities per thread and as many ranges (at
  * most 4) as fill the SMs' resident slots without starting another wave.
- * ccfj_set_fj_variant(cpt) forces a velocities-per-thread variant (0
- * restores the tuned or default choice).
+ * ccfj_set_fj_variant(cpt) forces a velocities-per-thread variant, and keeps
+ * the expansion off (0 restores the tuned or default choice and the expansion).
  *
  * Persistence: ccfj_set_tune_cache(path) names a text table that both
  * autotuners write every result to and that later calls (in this or any
@@ -386,8 +390,9 @@ CCFJ_API int ccfj_pick_v1(const float *spec, int nc, int nf, const float *c, con
 CCFJ_API int ccfj_autotune_fj_v1(const ccfj_fj_args *args, void *stream, int *best_cpt,
                                  float *best_ms);
 CCFJ_API int ccfj_set_fj_variant(int cpt);
-/* Forces the number of station ranges of FP32 transforms (1 = unsplit;
- * 0 restores the tuned or default choice). */
+/* Forces the number of station ranges of FP32 transforms (1 = unsplit), and
+ * keeps the expansion off (0 restores the tuned or default choice and the
+ * expansion). */
 CCFJ_API int ccfj_set_fj_split(int nsplit);
 CCFJ_API int ccfj_set_tune_cache(const char *path);
 CCFJ_API int ccfj_tuned_choice_fj(const ccfj_fj_args *args, int *cpt, int *nsplit);
