@@ -54,7 +54,8 @@ struct Plan {
   int radix[kMaxPasses] = {};
   int ldj = 0;             // row length of the spectra (nf rounded up to 32)
   std::vector<int> lo, hi; // [nsta] kept shifts lo..hi
-  std::vector<Window> windows;  // kept (shift, station) windows, station-major
+  long long nwindows = 0;       // kept (shift, station) windows
+  std::vector<Window> windows;  // the same, station-major (list_windows)
   std::vector<Tile> tiles;      // station tiles holding at least one pair
   std::vector<int> pmap;        // [nsta * nsta]: first pair (a, b), or -1
   std::vector<int> pnext;       // [npairs]: next pair with the same (a, b), or -1
@@ -66,7 +67,9 @@ inline int plan_fail(std::string* err, const std::string& msg) {
 }
 
 // Fills *p for the arguments (host pointers for pairs and startend).
-inline int make_plan(const ccfj_cc_args& a, Plan* p, std::string* err) {
+// list_windows: Plan::windows too, which the host replay walks (the kernels find
+// a window by the station's lo and hi, and the list grows with both).
+inline int make_plan(const ccfj_cc_args& a, Plan* p, std::string* err, bool list_windows = true) {
   if (a.nsta < 1 || a.nsta > kMaxStations)
     return plan_fail(err, "nsta=" + std::to_string(a.nsta) + " must be in 1.." +
                               std::to_string(kMaxStations));
@@ -105,6 +108,7 @@ inline int make_plan(const ccfj_cc_args& a, Plan* p, std::string* err) {
   const int nsta = a.nsta;
   p->lo.assign(nsta, 0);
   p->hi.assign(nsta, -1);
+  p->nwindows = 0;
   p->windows.clear();
   for (int i = 0; i < nsta; ++i) {
     long long lo, hi;
@@ -112,7 +116,9 @@ inline int make_plan(const ccfj_cc_args& a, Plan* p, std::string* err) {
     if (hi >= lo) {
       p->lo[i] = (int)lo;
       p->hi[i] = (int)hi;
-      for (long long k = lo; k <= hi; ++k) p->windows.push_back(Window{(int)k, i});
+      p->nwindows += hi - lo + 1;
+      if (list_windows)
+        for (long long k = lo; k <= hi; ++k) p->windows.push_back(Window{(int)k, i});
     }
   }
 

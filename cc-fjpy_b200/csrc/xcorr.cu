@@ -439,13 +439,13 @@ static int run(const ccfj_cc_args& a, cudaStream_t s) {
   CCFJ_REQUIRE(a.data != nullptr, "ccfj_cc_v1: data is NULL");
   Plan p;
   std::string err;
-  const int pst = make_plan(a, &p, &err);
+  const int pst = make_plan(a, &p, &err, false);
   if (pst != CCFJ_OK) return set_error(pst, "ccfj_cc_v1: %s", err.c_str());
   const long long nout = (long long)a.npairs * a.nf;
   CCFJ_REQUIRE(nout == 0 || (a.out_re && (a.out_layout == 1 || a.out_im)),
                "ccfj_cc_v1: output pointer is NULL");
   CCFJ_REQUIRE(a.nf <= 65535LL * kLanes, "ccfj_cc_v1: nf=%d too large", a.nf);
-  CCFJ_REQUIRE(p.windows.size() <= (size_t)0x7fffffff, "ccfj_cc_v1: too many windows");
+  CCFJ_REQUIRE(p.nwindows <= 0x7fffffff, "ccfj_cc_v1: too many windows");
   const long long nrec = (long long)a.nsta * a.npts;
   if (!a.device_ptrs && a.onebit)  // the reference rewrites the caller's samples
     for (long long n = 0; n < nrec; ++n) a.data[n] = onebit(a.data[n]);
