@@ -33,6 +33,7 @@ def load_rule(folder):
     lib.cell_disagreements.argtypes = [ctypes.c_longlong, ctypes.c_ulonglong, F]
     lib.cell_disagreements.restype = ctypes.c_longlong
     lib.cell_carries.argtypes = [F, F, F, F, I, ctypes.c_void_p]
+    lib.cell_hu.argtypes, lib.cell_hu.restype = [F], ctypes.c_double
     lib.cell_locate.argtypes = [F, F, F, I]
     lib.cell_walk.argtypes = [F, F, F, I, I]
     return lib

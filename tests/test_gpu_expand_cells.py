@@ -17,7 +17,6 @@ from test_gpu_expand import MODES, TOL, _run
 
 pytestmark = pytest.mark.gpu
 CMIN, RMAX = 500.0, 3e5
-HU = 9.8 / (2 * np.pi) * CMIN  # a cell: 9.8 radians at the slowest velocity
 
 
 @pytest.fixture(scope="module")
@@ -81,12 +80,12 @@ def test_last_station_on_the_plan_s_last_cell_end(rule, mode, itype):
 
 
 @pytest.mark.parametrize("mode,itype", [("J", 1), ("J", 0), ("|J|", 1)])
-def test_distances_on_cell_ends_of_many_frequencies(mode, itype):
+def test_distances_on_cell_ends_of_many_frequencies(rule, mode, itype):
     """Stations on, just below and just above the cell ends of 40 frequencies of
     the call's 600, and each of those frequencies among its neighbours."""
     rng = np.random.default_rng(6)
     f = np.linspace(0.3, 1.4, 600).astype(np.float32)
-    ends = np.concatenate([(HU * rng.choice(np.arange(1, 90), 12, replace=False)) / fk
+    ends = np.concatenate([(rule.cell_hu(CMIN) * rng.choice(np.arange(1, 90), 12, replace=False)) / fk
                            for fk in f[::15].astype(np.float64)]).astype(np.float32)
     r = np.sort(np.concatenate([ends, np.nextafter(ends, np.float32(0)),
                                 np.nextafter(ends, np.float32(1e9))]))
