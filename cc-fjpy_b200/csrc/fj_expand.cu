@@ -873,12 +873,17 @@ __global__ void __launch_bounds__(32, NIN == 1 ? 24 : 16) xp_moments_kernel(XpDe
 }
 
 // Adds the parts of the cells that lie across chunk boundaries, in chunk
-// order, and clears the cells of the tile that a column does not reach. Four
-// threads per (slot, frequency). The first chunk that begins in a cell adds
-// all that the cell got: the tail of the chunk before it, its own head, and
-// the heads of the chunks after it that begin in the same cell.
+// order, and clears the cells of the tile that a column does not reach. That is
+// shared by a chunk for 32 cells, up to kClear chunks: by the first and the last
+// one alone it was a chain of stores as long as the tile (279 records x 105 f
+// over 1116 cells: 71 us, 20 us so). Bound by latency, so six CTAs an SM: with the
+// registers for four, 128 subarrays took 50 us longer. Four threads per (slot,
+// frequency). The first chunk that begins in a cell adds all that the cell got:
+// the tail of the chunk before it, its own head, and the heads of the chunks
+// after it that begin in the same cell.
+constexpr int kClear = 32;
 template <int NIN, int ITYPE, bool DY>
-__global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
+__global__ void __launch_bounds__(256, 6) xp_join_kernel(XpDev d) {
   const int n4 = threadIdx.x & 3;
   const int fi = blockIdx.y * 64 + (threadIdx.x >> 2);
   const long long slot = blockIdx.x;
@@ -891,7 +896,7 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
   const int2* span = d.span + slot * d.nf + fi;  // of chunk q + i: span[i nf]
   const int2 me = span[0];
   const int before = q > 0 ? span[-(long long)d.nf].x : -1;
-  if (before == me.x && q != nch - 1) return;
+  if (before == me.x && q != nch - 1 && q >= kClear) return;
   const XpTile tile = d.tile[b * d.ft + fi / kTileCols];
   float* const col = d.W + (fi & (kTileCols - 1)) * kNodes + n4 * 4;
   auto put = [&](int cell, int k, float4 v) {
@@ -904,11 +909,16 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
     v = make_float4(v.x + a.x, v.y + a.y, v.z + a.z, v.w + a.w);
   };
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (q == 0)
-    for (int c = tile.lo; c < me.x; ++c) {
+  const int share = min(nch, max(1, min(kClear, (tile.hi - tile.lo) / 32)));
+  if (q < share) {
+    const int first = span[-(long long)q * d.nf].x, last = span[(long long)(nch - 1 - q) * d.nf].y;
+    for (int c = tile.lo + q; c < tile.hi; c += share)
+      if (c < first || c > last) {
 #pragma unroll
-      for (int k = 0; k < NIN; ++k) put(c, k, zero);
-    }
+        for (int k = 0; k < NIN; ++k) put(c, k, zero);
+      }
+  }
+  if (before == me.x && q != nch - 1) return;
   if (before != me.x) {
 #pragma unroll
     for (int k = 0; k < NIN; ++k) {
@@ -941,10 +951,6 @@ __global__ void __launch_bounds__(256) xp_join_kernel(XpDev d) {
         add(v, d.tail + at + k * kNodes);
         put(me.y, k, v);
       }
-    }
-    for (int c = me.y + 1; c < tile.hi; ++c) {
-#pragma unroll
-      for (int k = 0; k < NIN; ++k) put(c, k, zero);
     }
   }
 }
