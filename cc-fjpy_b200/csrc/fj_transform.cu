@@ -78,12 +78,12 @@ __global__ void __launch_bounds__(256, fj_min_blocks<T>()) fj_amortized_kernel(F
 
 // Sum of the station ranges of a split launch, in range order (the result
 // does not depend on how the ranges were scheduled), then the amplitude
-// gamma(k), the mode's combination and NaN at k = 0, as fj_cells finishes
-// an unsplit sum.
+// gamma(k), the mode's combination and (itype 1) NaN at k = 0, as fj_cells
+// finishes an unsplit sum.
 template <int MODE>
 __global__ void fj_split_finish_kernel(const float* __restrict__ part, int nsplit,
                                        const float* __restrict__ f, const float* __restrict__ c,
-                                       int nc, int nf, float* __restrict__ out,
+                                       int nc, int nf, int itype, float* __restrict__ out,
                                        Elsewhere other) {
   const int fi = blockIdx.x * 32 + threadIdx.x;
   const int ci = blockIdx.y * 8 + threadIdx.y;
@@ -98,7 +98,7 @@ __global__ void fj_split_finish_kernel(const float* __restrict__ part, int nspli
   cell.init(f[fi], c[ci]);
   const float gam = cell.gamma();
   float res[2] = {gam * tot[0], gam * tot[1]};
-  out[at] = cell.k == 0.0f ? __int_as_float(0x7fffffff) : finish<MODE, float>(res, 1.0f);
+  out[at] = itype == 1 && cell.k == 0.0f ? __int_as_float(0x7fffffff) : finish<MODE, float>(res, 1.0f);
 }
 
 // ------------------------------------------ FP64 comparator (plain form)
@@ -564,24 +564,17 @@ int fj_device(const ccfj_fj_args& a, cudaStream_t s, const FjChoice& choice) {
     const int n = (int)div_up(a.nr, d.split_len);
     const dim3 fg(div_up(a.nf, 32), div_up(a.nc, 8)), fb(32, 8);
     switch (a.mode) {
-      case CCFJ_MODE_J:
-        fj_split_finish_kernel<CCFJ_MODE_J><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out, d.other);
-        break;
-      case CCFJ_MODE_Y:
-        fj_split_finish_kernel<CCFJ_MODE_Y><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.out, d.other);
-        break;
-      case CCFJ_MODE_J_MINUS_Y:
-        fj_split_finish_kernel<CCFJ_MODE_J_MINUS_Y><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc,
-                                                                     a.nf, a.out, d.other);
-        break;
-      case CCFJ_MODE_ABS_J:
-        fj_split_finish_kernel<CCFJ_MODE_ABS_J><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf,
-                                                                 a.out, d.other);
-        break;
-      default:
-        fj_split_finish_kernel<CCFJ_MODE_ABS_H><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf,
-                                                                 a.out, d.other);
-        break;
+#define CCFJ_FINISH(M)                                                                    \
+  case M:                                                                                 \
+    fj_split_finish_kernel<M><<<fg, fb, 0, s>>>(d.part, n, a.f, a.c, a.nc, a.nf, a.itype, \
+                                                a.out, d.other);                          \
+    break
+      CCFJ_FINISH(CCFJ_MODE_J);
+      CCFJ_FINISH(CCFJ_MODE_Y);
+      CCFJ_FINISH(CCFJ_MODE_J_MINUS_Y);
+      CCFJ_FINISH(CCFJ_MODE_ABS_J);
+      CCFJ_FINISH(CCFJ_MODE_ABS_H);
+#undef CCFJ_FINISH
     }
     count_launch();
     CCFJ_LAUNCH_CHECK("fj_split_finish_kernel");
