@@ -192,11 +192,11 @@ __host__ __device__ inline bool worth(double n, double per_pair) {
 // Of 1683 transforms drawn at random (2-19,900 pairs, half of them of up to 600
 // pairs, where the line lies), 135 took more than 15% longer than the direct
 // kernels alone with the first estimate only (an itype 0 case 2.7 times as
-// long), 94 with both; 58 became more than 15% faster and 2 slower (66 pairs x
-// 906 f x 38 c 164 -> 88 us, 95 by the direct kernels; 182 pairs x 208 f x 23 c,
-// itype 0, 118 -> 91 us, 101 directly). Still slower than directly: problems
+// long), 85 with both; 77 became more than 15% faster and 1 slower (66 pairs x
+// 906 f x 38 c 164 -> 89 us, 95 by the direct kernels; 182 pairs x 208 f x 23 c,
+// itype 0, 118 -> 79 us, 101 directly). Still slower than directly: problems
 // whose upper frequencies go direct while the lower ones do not (156 records x
-// 320 f x 43 c 329 us, 187 directly).
+// 320 f x 43 c 306 us, 187 directly).
 constexpr double kMargin = 1.3;
 constexpr double kDense = 6.5;
 __device__ __forceinline__ bool worth_cells(const XpDev& d, int itype, int cells_of_column,
@@ -1326,12 +1326,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xp_gemm_kernel(XpDev d) {
 // sector of a row) of one set, so that 512 frequencies still make 64 CTAs, or
 // 32 where that leaves enough CTAs (128 subarrays x 512 f x 500 c: 400 us with
 // 8). A thread keeps its velocities' values in registers where they fit (2048
-// or 1024 velocities).
+// or 1024 velocities). Bound by the latency of the units' loads: 16 in flight
+// where few columns leave few CTAs and short runs make many units (140 f x 197 c
+// over 1436 cells: 57 us with 4, 34 with 16).
 constexpr int kFinThreads = 1024;
 template <int MODE, int ITYPE, int kFinCols>
 __global__ void __launch_bounds__(kFinThreads) xp_finish_kernel(XpDev d) {
   constexpr int kFinRows = kFinThreads / kFinCols, kFinKeep = kFinCols == 8 ? 16 : 32;
-  constexpr int kWarpRows = 32 / kFinCols;
+  constexpr int kWarpRows = 32 / kFinCols, kAhead = 16;
   constexpr int NACC = ModeTraits<MODE>::NACC;
   __shared__ float red[kFinRows / kWarpRows][kFinCols];
   const int fi = blockIdx.x * kFinCols + threadIdx.x, b = blockIdx.y;
@@ -1349,8 +1351,17 @@ __global__ void __launch_bounds__(kFinThreads) xp_finish_kernel(XpDev d) {
                        (tile.unit + q * d.mtiles + c / kTileRows) * (kTileRows * kTileCols) +
                        (c % kTileRows) * kTileCols + (fi & (kTileCols - 1));
       const long long step = (long long)d.mtiles * NACC * kTileRows * kTileCols;
+      int s = 0;
+      if (kFinCols == 8)
+        for (; s + kAhead <= nrun; s += kAhead) {
+          float t[kAhead];
+#pragma unroll
+          for (int i = 0; i < kAhead; ++i) t[i] = p[(s + i) * step];
+#pragma unroll
+          for (int i = 0; i < kAhead; ++i) v[q] += t[i];
+        }
 #pragma unroll 4
-      for (int s = 0; s < nrun; ++s) v[q] += p[s * step];
+      for (; s < nrun; ++s) v[q] += p[s * step];
     }
     if (nan_col) return __int_as_float(0x7fffffff);
     return NACC == 1 ? v[0] : sqrtf(v[0] * v[0] + v[1] * v[1]);
